@@ -37,15 +37,19 @@ void note_launch(unsigned long long k = 1);
 
 // ---------------------------------------------------------------- geometry
 // M_a is the padded FFT length of axis a: 2 n_a as in the reference, or, for
-// a library-built Green tensor with IPBC = 0, the next length >= 2 n_a that the
-// register-FFT pipeline runs (the circulant embedding of the lags -(n-1)..n-1
-// is exact for any M >= 2n - 1; the spectrum is still even per axis, so the
+// a library-built Green tensor, the next length >= 2 n_a that the register-FFT
+// pipeline runs (the circulant embedding of the lags -(n-1)..n-1 is exact for
+// any M >= 2n - 1; with IPBC = 0 the spectrum is still even per axis, so the
 // octant k_a = 0..M_a/2 holds it).
 struct Geometry {
   int nx = 0, ny = 0, nz = 0, Mx = 0, My = 0, Mz = 0;
   int nat = 0, nat0 = 0, ipbc = 0;
   size_t ngrid() const { return (size_t)Mx * My * Mz; }
   size_t octant() const { return (size_t)(Mx / 2 + 1) * (My / 2 + 1) * (Mz / 2 + 1); }
+  // row lengths of the x-first pipeline's A (rows of n_y) and B (rows of n_z):
+  // even, so that rows of complex floats start on 16 bytes for odd n too
+  int ldy() const { return (ny + 1) & ~1; }
+  int ldz() const { return (nz + 1) & ~1; }
   bool padded() const { return Mx != 2 * nx || My != 2 * ny || Mz != 2 * nz; }
   size_t green_count() const { return ipbc == 0 ? 6 * octant() : 6 * ngrid(); }
 };
@@ -99,7 +103,7 @@ template <typename T> struct Engine {
   int slab_nr = 0, slab_B = 0;  // slab = slab_nr RHS x slab_B planes
   size_t slab_budget_elems = 0;
   int slices_layout = 0;
-  int xpipe = 0;           // 1: x-first transposed pipeline (power-of-two grids)
+  int xpipe = 0;           // 1: x-first transposed pipeline (register-FFT axis lengths)
   // launch shapes of the z-first pipeline (set from the environment at
   // prepare, changed by the autotuner): register-pass block sizes, y-pass
   // columns per block, complex elements per generic-pass tile (0: default)
@@ -109,8 +113,10 @@ template <typename T> struct Engine {
   int tune_zg = 0;
   // elements per RHS of the first-pass grid: the z-transformed grid (z-first)
   // or the x-transformed grid A (x-first)
+  // one middle-stage plane of one RHS: a kz plane (z-first) or a kx column plane (x-first)
+  size_t plane_per_rhs() const { return xpipe ? (size_t)3 * g.My * g.ldz() : (size_t)3 * g.ny * g.Mx; }
   size_t zhat_per_rhs() const {
-    return xpipe ? (size_t)3 * g.nz * g.Mx * g.ny : (size_t)3 * g.Mz * g.ny * g.nx;
+    return xpipe ? (size_t)3 * g.nz * g.Mx * g.ldy() : (size_t)3 * g.Mz * g.ny * g.nx;
   }
   cudaStream_t stream = 0;
   size_t bytes_allocated = 0;

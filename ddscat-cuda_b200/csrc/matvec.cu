@@ -577,19 +577,36 @@ template <typename T> static cplx<T>* upload_twiddles(int n, size_t& bytes) {
   return d;
 }
 
+// Largest ratio of padded to 2n grid points at which the register pipeline is
+// the faster one.  The generic passes cost 0.10-0.13 ns per point when 2n has
+// the factors 2, 3, 5 only and 0.27 ns and more with larger ones (their
+// butterflies grow with the factor), the register passes 0.02-0.03 ns.
+// Measured at 8 RHS per call, ms per RHS padded / on 2n: factors 2, 3, 5:
+// 135x135x40 (4.3 times the points) 0.52 / 0.84, 12x10x9 (3.8) 0.0038 / 0.0053,
+// 72^3 (2.4) 0.156 / 0.383; larger ones: 34^3 (2.8) 0.027 / 0.274, 65^3 (3.2)
+// 0.154 / 1.11, 131x131x33 (5.6) 0.50 / 77.  4.5 and 12 keep a margin for
+// single-RHS calls on small grids, where launches decide (5^3, 4.1 times the
+// points: 0.028 / 0.031 ms).
+static double pad_limit(const Geometry& g) {
+  auto smooth = [](int m) {
+    for (int f : {2, 3, 5})
+      while (m % f == 0) m /= f;
+    return m == 1;
+  };
+  return smooth(g.Mx) && smooth(g.My) && smooth(g.Mz) ? 4.5 : 12.0;
+}
+
 template <typename T>
 int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0, const int16_t* iocc_host, bool pad) {
   g.nx = nx; g.ny = ny; g.nz = nz;
   g.Mx = 2 * nx; g.My = 2 * ny; g.Mz = 2 * nz;
   g.nat = nat; g.nat0 = nat0; g.ipbc = ipbc;
-  if (pad && ipbc == 0 && nx % 2 == 0 && ny % 2 == 0 && nz % 2 == 0 && !env_flag("DDSCAT_B200_NOPAD") &&
-      !xpipe_supported<T>(g)) {
-    // pad to the register-FFT lengths when the padded grid has at most 2.5x the
-    // points of the 2n grid (the register pipeline is ~4x faster per point);
-    // even n only (the row passes move element pairs of 16 bytes)
+  if (pad && !env_flag("DDSCAT_B200_NOPAD") && !xpipe_supported<T>(g)) {
+    // pad to the register-FFT lengths unless the padded grid has more points
+    // than the register passes make up for (pad_limit)
     Geometry p = g;
     p.Mx = xpipe_len<T>(2 * nx); p.My = xpipe_len<T>(2 * ny); p.Mz = xpipe_len<T>(2 * nz);
-    if (p.Mx && p.My && p.Mz && (double)p.ngrid() <= 2.5 * (double)g.ngrid() && xpipe_supported<T>(p)) g = p;
+    if (p.Mx && p.My && p.Mz && (double)p.ngrid() <= pad_limit(g) * (double)g.ngrid() && xpipe_supported<T>(p)) g = p;
   }
   px = make_fft_plan(g.Mx);
   py = make_fft_plan(g.My);
@@ -657,8 +674,7 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
 
 template <typename T> int Engine<T>::ensure_workspace(int nrhs) {
   const size_t per_rhs_z = zhat_per_rhs();
-  // one middle-stage plane, 3 comps, one RHS: a kz plane (z-first) or a kx column plane (x-first)
-  const size_t per_plane = xpipe ? (size_t)3 * g.My * g.nz : (size_t)3 * g.ny * g.Mx;
+  const size_t per_plane = plane_per_rhs();
   const int nplanes_all = xpipe ? g.Mx : g.Mz;
   if (nrhs <= zcap && zhat) return 0;
   if (zhat) { cudaFree(zhat); bytes_allocated -= (size_t)zcap * per_rhs_z * sizeof(C); zhat = nullptr; }

@@ -1,4 +1,4 @@
-// x-first, transposed-layout MATVEC pipeline for power-of-two grids (sm_100a).
+// x-first, transposed-layout MATVEC pipeline on register-FFT axis lengths (sm_100a).
 //
 // Same operator as matvec.cu (cprod_cuda.f90:446-607 / ddscat_matvec_cuda.cu:
 // 104-118), organised so that every pass transforms along the contiguous axis
@@ -48,6 +48,7 @@ template <typename T> struct XParams {
   int tma_x;
   int* err;  // status word (Engine::d_err)
   int nx, ny, nz, Mx, My, Mz, nat, nat0;
+  int lda, ldb;  // row lengths of A (n_y) and B (n_z), rounded up to even
   const cplx<T>* x;
   size_t x_rs;
   cplx<T>* y;
@@ -144,9 +145,10 @@ __device__ __forceinline__ void tma_load_tile(const CUtensorMap* map, float2* ti
 
 // Tile <-> global moves of the row passes: N rows of RL consecutive elements
 // (row stride ld in global, RL+1 in the tile), two elements per 16-byte access.
-// Rows hold `valid` elements (RL or fewer at the grid edge; always even,
-// since every axis length n is even here and RL is even).  The global base and
-// ld are even in elements, so every pair is 16-byte aligned.
+// Rows hold `valid` elements (RL or fewer at the grid edge; always even:
+// rows are stored with an even length, an odd n followed by one element that
+// no pass uses, and RL is even).  The global base and ld are even in
+// elements, so every pair is 16-byte aligned.
 template <int RL, int N, typename C>
 __device__ __forceinline__ void store_pairs(C* g, int ld, int valid, const C* tile) {
   constexpr int RP = RL / 2;
@@ -276,8 +278,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
 #pragma unroll
   for (int i = 0; i < E; ++i) tile[(t + TT * i) * (RL + 1) + l] = v[i];
   __syncthreads();
-  C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * P.ny + iy0;
-  store_pairs<RL, N>(A, P.ny, P.ny - iy0, tile);
+  C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * P.lda + iy0;
+  store_pairs<RL, N>(A, P.lda, P.lda - iy0, tile);
 }
 
 // ------------------------------------------------------------- YF: y forward
@@ -293,7 +295,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
   const int iz0 = blockIdx.x * RL, iz = iz0 + l, kxl = blockIdx.y, kx = P.kx0 + kxl;
   const int rb = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3), rl = P.b_rhs0 + rb;
   if (xoff(P, rl)) return;
-  const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx + kx) * P.ny;
+  const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx + kx) * P.lda;
   C v[E];
   const bool zin = iz < P.nz;
 #pragma unroll
@@ -316,8 +318,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
 #pragma unroll
   for (int i = 0; i < E; ++i) tile[(t + TT * i) * (RL + 1) + l] = v[i];
   __syncthreads();
-  C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * P.nz + iz0;
-  store_pairs<RL, N>(B, P.nz, P.nz - iz0, tile);
+  C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * P.ldb + iz0;
+  store_pairs<RL, N>(B, P.ldb, P.ldb - iz0, tile);
 }
 
 // Green record at (kx, ky, kz) for the z-fastest layout, without the kz sign.
@@ -396,7 +398,7 @@ template <int BTY, typename T> __device__ __forceinline__ size_t zline_base(cons
     const int kxl = p / BTY;
     return (size_t)kxl * P.nz * BTY + (p - kxl * BTY);
   } else {
-    return (size_t)p * P.nz;
+    return (size_t)p * P.ldb;
   }
 }
 template <int BTY> constexpr int zline_stride() { return BTY > 0 ? BTY : 1; }
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   const int p = blockIdx.y * RL + l;
   const bool live = p < nlines;
   constexpr int zs = zline_stride<BTY>();
-  C* row = P.B + ((size_t)(rb * 3 + c) * P.nkx) * (size_t)P.My * P.nz + zline_base<BTY>(P, live ? p : 0);
+  C* row = P.B + ((size_t)(rb * 3 + c) * P.nkx) * (size_t)P.My * (BTY ? P.nz : P.ldb) + zline_base<BTY>(P, live ? p : 0);
   C v[E];
 #pragma unroll
   for (int i = 0; i < H; ++i)
@@ -550,7 +552,7 @@ template <typename T, int N, int BTY = 0> __global__ void __launch_bounds__(128,
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.y * Z3Shape<N>::RZ + l;
   const bool live = p < nlines;
-  const size_t cs = (size_t)nlines * P.nz;  // component stride of B
+  const size_t cs = (size_t)nlines * (BTY ? P.nz : P.ldb);  // component stride of B
   constexpr int zs = zline_stride<BTY>();
   C* row = P.B + (size_t)rb * 3 * cs + zline_base<BTY>(P, live ? p : 0);
   const int kxl = p / P.My;
@@ -644,7 +646,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.x * RZ + l;
   const bool live = p < nlines;
-  const size_t cs = (size_t)nlines * P.nz;  // component stride of B
+  const size_t cs = (size_t)nlines * P.ldb;  // component stride of B
   const int kxl = p / P.My;
   const int kx = P.kx0 + kxl, ky = p - kxl * P.My;
   // the block's octant lines: line ll is the contiguous record run of
@@ -666,7 +668,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
   const int rb1 = min(P.nrb_mid, ((int)blockIdx.y + 1) * P.zg_rch);
   for (int rb = (int)blockIdx.y * P.zg_rch; rb < rb1; ++rb) {
     if (xoff(P, P.b_rhs0 + rb)) continue;  // the same for every thread of the block
-    C* row = P.B + (size_t)rb * 3 * cs + (size_t)(live ? p : 0) * P.nz;
+    C* row = P.B + (size_t)rb * 3 * cs + (size_t)(live ? p : 0) * P.ldb;
     C v[3][E];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -740,8 +742,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
     }
   }
   if (!loaded) {
-    const C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * nz + iz0;
-    load_tile_pairs<RL, N>(B, nz, nz - iz0, tile);
+    const C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * P.ldb + iz0;
+    load_tile_pairs<RL, N>(B, P.ldb, P.ldb - iz0, tile);
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * (RL + 1) + l];
@@ -749,7 +751,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
   }
   line_fft<E, TT, -1, false, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy);
   if (iz < nz) {
-    C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * nz + iz) * P.Mx + kx) * P.ny;
+    C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * nz + iz) * P.Mx + kx) * P.lda;
 #pragma unroll
     for (int i = 0; i < H; ++i)
       if (t + TT * i < P.ny) A[t + TT * i] = v[i];  // keep iy < ny
@@ -881,8 +883,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
     }
   }
   if (!loaded) {
-    const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * ny + iy0;
-    load_tile_pairs<RL, N>(A, ny, ny - iy0, tile);
+    const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * P.lda + iy0;
+    load_tile_pairs<RL, N>(A, P.lda, P.lda - iy0, tile);
     cp_async_wait_all();  // the x and CXADIA chunks
     __syncthreads();
 #pragma unroll
@@ -1236,14 +1238,15 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// Map of B (rows of n_z complex floats, row stride n_z * 8 bytes) for the
+// Map of B (rows of n_z complex floats, row stride ld * 8 bytes) for the
 // 256-point y passes' tiles, or of A (rows of n_y) for the x passes: box
-// {16, 256}, 128-byte swizzle, zero fill.
-static bool encode_b_map(CUtensorMap* m, void* base, size_t rows, int nz) {
+// {16, 256}, 128-byte swizzle, zero fill.  ld is even, so the stride is a
+// multiple of 16 bytes; an odd n ends the row inside its last pair.
+static bool encode_b_map(CUtensorMap* m, void* base, size_t rows, int nz, int ld) {
   const auto enc = tensor_map_encoder();
-  if (!enc || rows > 0xffffffffull || (nz & 1)) return false;
+  if (!enc || rows > 0xffffffffull || (ld & 1)) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)nz, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)nz * 8};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 8};
   const cuuint32_t box[2] = {(cuuint32_t)TMA_COLS, (cuuint32_t)TMA_ROWS};
   const cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1276,7 +1279,8 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   P.x_rs = a.x_rs; P.y_rs = a.y_rs; P.a_rs = a.a_rs;
   P.io_full = a.io_full; P.a_full = a.a_full; P.conj = a.conj;
   P.inv = E.inv; P.iocc = E.iocc; P.rowq = E.rowq; P.mask = a.mask;
-  P.A = E.zhat; P.A_rs = (size_t)3 * g.nz * g.Mx * g.ny;
+  P.A = E.zhat; P.A_rs = (size_t)3 * g.nz * g.Mx * g.ldy();
+  P.lda = g.ldy(); P.ldb = g.ldz();
   P.B = E.slab;
   P.green = E.green; P.ipbc = g.ipbc;
   P.twx = E.twx; P.twy = E.twy; P.twz = E.twz;
@@ -1313,10 +1317,10 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   if constexpr (sizeof(T) == 4) {
     // the same for A (rows of n_y) in the 256-point x passes
     if (E.use_tma && (g.Mx == 256 || g.Mx == 512) && RX == TMA_COLS && E.d_err &&
-        encode_b_map(&P.tmA, E.zhat, (size_t)E.zcap * 3 * g.nz * g.Mx, g.ny))
+        encode_b_map(&P.tmA, E.zhat, (size_t)E.zcap * 3 * g.nz * g.Mx, g.ny, P.lda))
       P.tma_x = 1;
     if (E.use_tma && (g.My == 256 || g.My == 512) && RY == TMA_COLS && E.d_err &&
-        encode_b_map(&P.tmB, E.slab, (size_t)E.slab_nr * 3 * E.slab_B * g.My, g.nz)) {
+        encode_b_map(&P.tmB, E.slab, (size_t)E.slab_nr * 3 * E.slab_B * g.My, g.nz, P.ldb)) {
       P.tma = 1;
       smy = std::max(smy, (size_t)(g.My / TMA_ROWS) * TMA_TILE_BYTES + 1024);
     }

@@ -11,15 +11,18 @@
 // lives in the fixed array below instead of the engine's workspace.
 //
 // Limits and sharing:
-//  * The scratch (48 MiB, 6,291,456 complex floats) must hold the
-//    x-transformed grid and the half-padded spectrum of the prepared target:
-//    3*nz*Mx*ny + 3*My*nz*Mx complex floats on the x-first pipeline, with
-//    Mx, My the padded FFT lengths the prepare chose (2*nx, 2*ny, or the next
-//    register-FFT length for a padded axis), 3*Mz*ny*nx + 3*ny*Mx*Mz on the
-//    z-first one.  With M = 2n that is 18*NAT, so unpadded targets with
-//    NAT = NX*NY*NZ <= 349,525 sites (e.g. 64^3) fit; padded grids need more
-//    (72x72x64, NAT = 331,776, pads 144 to 192 and needs 9.7 M).  Targets
-//    that do not fit are rejected with status 601 before any launch.
+//  * The scratch (48 MiB, 6,291,456 complex floats) holds the x-transformed
+//    grid and the half-padded spectrum of the prepared target: on the x-first
+//    pipeline 3*nz*Mx*ny + 3*My*nz*Mx complex floats (ny and nz rounded up to
+//    even), with Mx, My the padded FFT lengths the prepare chose (2*nx, 2*ny,
+//    or the next register-FFT length for a padded axis), 3*Mz*ny*nx +
+//    3*ny*Mx*Mz on the z-first one.  With M = 2n that is 18*NAT, so targets
+//    with NAT = NX*NY*NZ <= 349,525 sites (e.g. 64^3) fit.  A finite target of
+//    even sides padded to at most 2.5 times the points of the 2n grid must fit
+//    whole (72x72x64, NAT = 331,776, pads 144 to 192 and needs 9.7 M); ragged
+//    and periodic targets within the NAT limit hold as many planes of the
+//    spectrum at a time as fit.  Targets beyond that are rejected with status
+//    601 before any launch.
 //  * The array is part of the library's device image: every GPU that loads
 //    the library holds these 48 MiB until the process exits.
 //  * Every call on a device uses the same array and it keeps the last call's
@@ -34,6 +37,7 @@
 //  * The call must be made with the device that was current at prepare (the
 //    prepared Green tensor and index tables live there); another current
 //    device is rejected with status 600.
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include "ddscat_b200.h"
@@ -97,16 +101,24 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_apply_noalloc_f32(int cwhat, const vo
   int rc = noalloc_scratch(dev, &scratch);
   if (rc) return rc;
   // A shallow copy of the prepared engine whose workspace is the fixed array:
-  // one RHS, every middle-stage plane in one batch.
+  // one RHS, the middle-stage planes in one batch where they fit.
   Engine<float> e = *prep;
-  const size_t za = e.zhat_per_rhs();
-  const size_t sb = e.xpipe ? (size_t)3 * e.g.My * e.g.nz * e.g.Mx : (size_t)3 * e.g.ny * e.g.Mx * e.g.Mz;
-  if (za + sb > (size_t)NOALLOC_SCRATCH_ELEMS) {
+  const Geometry& g = e.g;
+  const size_t za = e.zhat_per_rhs(), plane = e.plane_per_rhs();
+  const int planes = e.xpipe ? g.Mx : g.Mz;
+  const size_t room = (size_t)NOALLOC_SCRATCH_ELEMS - std::min(za, (size_t)NOALLOC_SCRATCH_ELEMS);
+  const int fit = (int)std::min<size_t>((size_t)planes, room / plane);
+  // Finite targets of even sides padded to at most 2.5 times the points of the
+  // 2n grid hold every plane at once or are refused.  For the others the NAT
+  // limit alone decides: their middle stage runs in as many plane batches as
+  // it takes.
+  const bool whole = g.ipbc == 0 && !((g.nx | g.ny | g.nz) & 1) && (double)g.ngrid() <= 2.5 * 8.0 * (double)g.nat;
+  if (fit < (whole ? planes : 1)) {
     char msg[240];
     std::snprintf(msg, sizeof(msg),
                   "the padded FFT grid of this target needs %zu complex floats of scratch; the fixed scratch (48 MiB) "
                   "holds at most %zu",
-                  za + sb, (size_t)NOALLOC_SCRATCH_ELEMS);
+                  za + plane * (size_t)planes, (size_t)NOALLOC_SCRATCH_ELEMS);
     set_error("apply_noalloc", msg);
     return 601;
   }
@@ -114,7 +126,7 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_apply_noalloc_f32(int cwhat, const vo
   e.zcap = 1;
   e.slab = scratch + za;
   e.slab_nr = 1;
-  e.slab_B = e.xpipe ? e.g.Mx : e.g.Mz;
+  e.slab_B = (int)ceil_div((size_t)planes, ceil_div((size_t)planes, (size_t)fit));  // balanced batches
   e.stream = static_cast<cudaStream_t>(stream);
   MvArgs<float> a;
   a.x = static_cast<const float2*>(x);

@@ -105,10 +105,12 @@ DDSCAT_CUDA_API int ddscat_b200_residual_f64(int nrhs, const void *b, const void
  * aoff may be NULL), launched on `stream` (a cudaStream_t, NULL for the legacy
  * default stream), with the device of the prepare current.  The MATVEC
  * scratch is a fixed 48 MiB array (6,291,456 complex floats) in the library's
- * device image; every GPU that loads the library holds it until exit.  It must
- * hold 3*nz*Mx*ny + 3*My*nz*Mx complex floats for the padded FFT lengths Mx,
- * My of the prepared grid (18*NAT when M = 2n: unpadded targets up to
- * NAT = 349,525 sites, e.g. 64^3; padded grids need more), else the call
+ * device image; every GPU that loads the library holds it until exit.  It
+ * holds 3*nz*Mx*ny + 3*My*nz*Mx complex floats for the padded FFT lengths Mx,
+ * My of the prepared grid (18*NAT when M = 2n: targets up to NAT = 349,525
+ * sites, e.g. 64^3; finite targets of even sides padded to at most 2.5 times
+ * the points of the 2n grid must fit whole, others within the NAT limit run
+ * their middle stage in plane batches), else the call
  * returns 601.  All calls share the array and it keeps the last call's
  * contents (nothing needs to start at zero); calls that overlap on the GPU
  * race, so serialise them.  The first call on a device (and the first after
