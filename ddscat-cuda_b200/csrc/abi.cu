@@ -84,7 +84,8 @@ struct BatchState {
 };
 static BatchState bs;
 static void release_batch() {
-  cudaFree(bs.b); cudaFree(bs.x); cudaFree(bs.adia); cudaFree(bs.aoff); cudaFree(bs.work);
+  if (bs.work) cudaStreamSynchronize(bs.ops.stream);  // no solve in flight on the buffers
+  dev_free(bs.b); dev_free(bs.x); dev_free(bs.adia); dev_free(bs.aoff); dev_free(bs.work);
   bs.ops.release();
   const double ms = bs.matvec_ms;
   const long long mr = bs.matvec_rhs;
@@ -103,7 +104,8 @@ struct F64State {
 static F64State f64;
 static void release_f64() {
   if (f64.ready) {
-    cudaFree(f64.x); cudaFree(f64.y); cudaFree(f64.b); cudaFree(f64.ad); cudaFree(f64.ao);
+    cudaStreamSynchronize(f64.eng.stream);
+    dev_free(f64.x); dev_free(f64.y); dev_free(f64.b); dev_free(f64.ad); dev_free(f64.ao);
     f64.ops.release();
     f64.eng.release();
   }
@@ -118,21 +120,25 @@ struct Batch64 {
 };
 static Batch64 b64;
 static void release_b64() {
-  cudaFree(b64.b); cudaFree(b64.x); cudaFree(b64.adia); cudaFree(b64.aoff); cudaFree(b64.work); cudaFree(b64.full);
+  if (b64.work) cudaStreamSynchronize(b64.ops.stream);
+  dev_free(b64.b); dev_free(b64.x); dev_free(b64.adia); dev_free(b64.aoff); dev_free(b64.work); dev_free(b64.full);
   b64.ops.release();
   b64 = Batch64{};
 }
 
 static void release_state() {
+  // callers may still run the operator on streams of their own (the
+  // allocation-free MATVEC): their work ends before its buffers are reused
+  if (s.ready || s.eng.green) cudaDeviceSynchronize();
   release_batch();
   release_b64();
   release_f64();
   delete[] s.h_iocc;
   s.h_iocc = nullptr;
   if (s.ready || s.eng.green) {
-    cudaFree(s.d_xf); cudaFree(s.d_yf); cudaFree(s.d_adia); cudaFree(s.d_aoff);
-    cudaFree(s.d_b); cudaFree(s.d_sx); cudaFree(s.d_sy); cudaFree(s.d_work);
-    cudaFree(s.d_adia_c); cudaFree(s.d_aoff_c);
+    dev_free(s.d_xf); dev_free(s.d_yf); dev_free(s.d_adia); dev_free(s.d_aoff);
+    dev_free(s.d_b); dev_free(s.d_sx); dev_free(s.d_sy); dev_free(s.d_work);
+    dev_free(s.d_adia_c); dev_free(s.d_aoff_c);
     s.ops.release();
     s.eng.release();
   }
@@ -166,7 +172,7 @@ static int allocate_runtime() {
   const size_t n = (size_t)3 * s.eng.g.nat, cn = (size_t)3 * s.eng.g.nat0;
   if (cn > (size_t)0x7fffffff) { set_error("allocate runtime", "3*NAT0 exceeds solver int range"); return 204; }
   cudaError_t e = cudaSuccess;
-  auto M = [&](C** p, size_t cnt) { if (e == cudaSuccess) e = cudaMalloc((void**)p, cnt * sizeof(C)); };
+  auto M = [&](C** p, size_t cnt) { if (e == cudaSuccess) e = dev_alloc((void**)p, cnt * sizeof(C)); };
   M(&s.d_xf, n); M(&s.d_yf, n); M(&s.d_adia, n); M(&s.d_aoff, n);
   M(&s.d_b, cn); M(&s.d_sx, cn); M(&s.d_sy, cn); M(&s.d_work, 13 * cn);
   M(&s.d_adia_c, cn); M(&s.d_aoff_c, cn);
@@ -466,11 +472,11 @@ static int ensure_batch(int R) {
   }
   release_batch();
   const size_t v = (size_t)R * n;
-  cudaError_t e = cudaMalloc((void**)&bs.b, v * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&bs.x, v * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&bs.adia, v * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&bs.aoff, v * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&bs.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(C));
+  cudaError_t e = dev_alloc((void**)&bs.b, v * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&bs.x, v * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&bs.adia, v * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&bs.aoff, v * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&bs.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(C));
   if (e != cudaSuccess) { release_batch(); set_cuda_error("batched solve workspace", e); return 1; }
   if (bs.ops.init(R, n, s.stream)) { release_batch(); return 1; }
   bs.R = R;
@@ -518,11 +524,11 @@ static int ensure_f64() {
     if (f64.eng.upload_green(h.data())) { release_f64(); return 1; }
   }
   const size_t cn = (size_t)3 * g.nat0;
-  cudaError_t e = cudaMalloc((void**)&f64.x, cn * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&f64.y, cn * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&f64.b, cn * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&f64.ad, cn * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&f64.ao, cn * sizeof(double2));
+  cudaError_t e = dev_alloc((void**)&f64.x, cn * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&f64.y, cn * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&f64.b, cn * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&f64.ad, cn * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&f64.ao, cn * sizeof(double2));
   if (e != cudaSuccess) { set_cuda_error("FP64 engine", e); release_f64(); return 1; }
   if (f64.ops.init(s.stream)) { release_f64(); return 1; }
   f64.eng.stream = s.stream;
@@ -543,12 +549,12 @@ static int ensure_b64(int R) {
   }
   release_b64();
   const size_t v = (size_t)R * n;
-  cudaError_t e = cudaMalloc((void**)&b64.b, v * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b64.x, v * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b64.adia, v * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b64.aoff, v * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b64.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&b64.full, (size_t)3 * s.eng.g.nat * sizeof(double2));
+  cudaError_t e = dev_alloc((void**)&b64.b, v * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&b64.x, v * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&b64.adia, v * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&b64.aoff, v * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&b64.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&b64.full, (size_t)3 * s.eng.g.nat * sizeof(double2));
   if (e != cudaSuccess) { release_b64(); set_cuda_error("FP64 batched solve workspace", e); return 1; }
   if (b64.ops.init(R, n, s.stream)) { release_b64(); return 1; }
   b64.R = R;
@@ -615,6 +621,7 @@ extern "C" {
 
 DDSCAT_CUDA_API int ddscat_cuda_release(void) {
   release_state();
+  mem_trim();
   clear_error();
   return 0;
 }
@@ -1035,10 +1042,10 @@ DDSCAT_CUDA_API int ddscat_b200_matvec_timing(int nrhs, int iters, int cwhat, fl
   }
   const size_t cn = (size_t)3 * s.eng.g.nat0;
   C *x = nullptr, *y = nullptr, *ad = nullptr;
-  cudaError_t e = cudaMalloc((void**)&x, cn * nrhs * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&y, cn * nrhs * sizeof(C));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ad, cn * nrhs * sizeof(C));
-  if (e != cudaSuccess) { cudaFree(x); cudaFree(y); cudaFree(ad); set_cuda_error("matvec_timing", e); return 401; }
+  cudaError_t e = dev_alloc((void**)&x, cn * nrhs * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&y, cn * nrhs * sizeof(C));
+  if (e == cudaSuccess) e = dev_alloc((void**)&ad, cn * nrhs * sizeof(C));
+  if (e != cudaSuccess) { dev_free(x); dev_free(y); dev_free(ad); set_cuda_error("matvec_timing", e); return 401; }
   {
     std::vector<C> h(cn);
     for (size_t i = 0; i < cn; ++i) h[i] = make_float2((float)((i * 2654435761u) % 1000) * 1e-3f, (float)(i % 7) * 0.1f);
@@ -1063,7 +1070,8 @@ DDSCAT_CUDA_API int ddscat_b200_matvec_timing(int nrhs, int iters, int cwhat, fl
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(x); cudaFree(y); cudaFree(ad);
+  if (rc) cudaStreamSynchronize(s.stream);
+  dev_free(x); dev_free(y); dev_free(ad);
   if (!rc && e != cudaSuccess) { set_cuda_error("matvec_timing", e); rc = 402; }
   if (!rc) rc = matvec_check(s.eng);
   *ms_per_call = ms / iters;
@@ -1115,10 +1123,10 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_amplitudes_f64(int nrhs, const v
   const bool dev = is_device_ptr(x);
   double2 *d_full = nullptr, *d_p = nullptr;
   cudaError_t e = cudaSuccess;
-  if (!dev) e = cudaMalloc((void**)&d_full, full * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_p, cn * sizeof(double2));
+  if (!dev) e = dev_alloc((void**)&d_full, full * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_p, cn * sizeof(double2));
   if (e != cudaSuccess) {
-    cudaFree(d_full);
+    dev_free(d_full);
     set_cuda_error("FP64 amplitudes workspace", e);
     return 711;
   }
@@ -1151,8 +1159,9 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_amplitudes_f64(int nrhs, const v
                                               term * (b[0] * sx.y + b[1] * sy.y + b[2] * sz.y));
     }
   }
-  cudaFree(d_full);
-  cudaFree(d_p);
+  if (rc) cudaStreamSynchronize(s.stream);
+  dev_free(d_full);
+  dev_free(d_p);
   return rc;
 }
 
@@ -1171,10 +1180,10 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_csca_f64(int nrhs, const void* x
   const bool dev = is_device_ptr(x);
   double2 *d_full = nullptr, *d_p = nullptr;
   cudaError_t e = cudaSuccess;
-  if (!dev) e = cudaMalloc((void**)&d_full, full * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_p, cn * sizeof(double2));
+  if (!dev) e = dev_alloc((void**)&d_full, full * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_p, cn * sizeof(double2));
   if (e != cudaSuccess) {
-    cudaFree(d_full);
+    dev_free(d_full);
     set_cuda_error("FP64 SCAT workspace", e);
     return 711;
   }
@@ -1205,8 +1214,9 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_csca_f64(int nrhs, const void* x
     }
     scat_integrate(idirs, sums.data(), ak2, (double)e02, cbksca + r, csca + r, cscag + 3 * r, cscag2 + r);
   }
-  cudaFree(d_full);
-  cudaFree(d_p);
+  if (rc) cudaStreamSynchronize(s.stream);
+  dev_free(d_full);
+  dev_free(d_p);
   return rc;
 }
 
@@ -1227,7 +1237,7 @@ static int make_inputs_entry(int cmdpol, int nrhs, const float* k, const void* e
   float2* tmp = nullptr;
   if (!dev) {
     const size_t per = (size_t)nrhs * full;
-    cudaError_t e = cudaMalloc((void**)&tmp, per * sizeof(float2) * ((b ? 1 : 0) + (adia ? 1 : 0)));
+    cudaError_t e = dev_alloc((void**)&tmp, per * sizeof(float2) * ((b ? 1 : 0) + (adia ? 1 : 0)));
     if (e != cudaSuccess) { set_cuda_error("make_inputs staging", e); return 612; }
     db = b ? tmp : nullptr;
     da = adia ? tmp + (b ? per : 0) : nullptr;
@@ -1241,7 +1251,8 @@ static int make_inputs_entry(int cmdpol, int nrhs, const float* k, const void* e
     if (e == cudaSuccess && adia) e = cudaMemcpy(adia, da, bytes, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) { set_cuda_error("make_inputs D2H", e); rc = 612; }
   }
-  cudaFree(tmp);
+  if (rc) cudaStreamSynchronize(s.stream);
+  dev_free(tmp);
   return rc;
 }
 
@@ -1558,8 +1569,8 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_ffweights_f32(int nw, const double* a
   const size_t full = (size_t)3 * g.nat;
   double* d_par = nullptr;
   C* d_w = dev ? static_cast<C*>(w) : nullptr;
-  cudaError_t ce = cudaMalloc((void**)&d_par, (size_t)6 * nw * sizeof(double));
-  if (ce == cudaSuccess && !dev) ce = cudaMalloc((void**)&d_w, (size_t)nw * full * sizeof(C));
+  cudaError_t ce = dev_alloc((void**)&d_par, (size_t)6 * nw * sizeof(double));
+  if (ce == cudaSuccess && !dev) ce = dev_alloc((void**)&d_w, (size_t)nw * full * sizeof(C));
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_par, aks, (size_t)3 * nw * sizeof(double), cudaMemcpyHostToDevice,
                                               s.stream);
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_par + 3 * (size_t)nw, em, (size_t)3 * nw * sizeof(double),
@@ -1581,7 +1592,8 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_ffweights_f32(int nw, const double* a
     }
     if (!rc && (ce = cudaStreamSynchronize(s.stream)) != cudaSuccess) { set_cuda_error("far-field weights", ce); rc = 722; }
   }
-  cudaFree(d_par);
-  if (!dev) cudaFree(d_w);
+  if (rc) cudaStreamSynchronize(s.stream);
+  dev_free(d_par);
+  if (!dev) dev_free(d_w);
   return rc;
 }

@@ -299,24 +299,25 @@ template <typename T> int BatchOps<T>::init(int R_, int n_, cudaStream_t s) {
   stream = s;
   nb = (int)std::max<size_t>(1, std::min<size_t>(ceil_div(n, BT), std::max(1, 592 / std::max(1, R))));
   coef_cap = (size_t)3 * R * 96;
-  cudaError_t e = cudaMalloc((void**)&d_part, (size_t)R * 8 * nb * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_out, (size_t)R * 8 * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_cnt, (size_t)R * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h_out, (size_t)R * 8 * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h_coef, coef_cap * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_coef, coef_cap * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h_mask, (size_t)MASKS * R * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_masks, (size_t)MASKS * R * sizeof(int));
+  cudaError_t e = dev_alloc((void**)&d_part, (size_t)R * 8 * nb * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_out, (size_t)R * 8 * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_cnt, (size_t)R * sizeof(unsigned));
+  if (e == cudaSuccess) e = host_alloc((void**)&h_out, (size_t)R * 8 * sizeof(double2));
+  if (e == cudaSuccess) e = host_alloc((void**)&h_coef, coef_cap * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_coef, coef_cap * sizeof(double2));
+  if (e == cudaSuccess) e = host_alloc((void**)&h_mask, (size_t)MASKS * R * sizeof(int));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_masks, (size_t)MASKS * R * sizeof(int));
   if (e != cudaSuccess) { set_cuda_error("batch buffers", e); return 1; }
   cudaMemset(d_cnt, 0, (size_t)R * sizeof(unsigned));
   return 0;
 }
 
 template <typename T> void BatchOps<T>::release() {
-  cudaFree(d_part); cudaFree(d_out); cudaFree(d_cnt); cudaFree(d_coef); cudaFree(d_masks);
-  if (h_out) cudaFreeHost(h_out);
-  if (h_coef) cudaFreeHost(h_coef);
-  if (h_mask) cudaFreeHost(h_mask);
+  if (d_part) cudaStreamSynchronize(stream);
+  dev_free(d_part); dev_free(d_out); dev_free(d_cnt); dev_free(d_coef); dev_free(d_masks);
+  if (h_out) host_free(h_out);
+  if (h_coef) host_free(h_coef);
+  if (h_mask) host_free(h_mask);
   *this = BatchOps<T>{};
 }
 
@@ -675,7 +676,7 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
   // device state
   const size_t nz2 = (size_t)(9 + 7 + 2) * R, nd = (size_t)2 * R, ni = (size_t)7 * R + 2;
   unsigned char* blk = nullptr;
-  cudaError_t e = cudaMalloc((void**)&blk, nz2 * sizeof(double2) + nd * sizeof(double) + ni * sizeof(int));
+  cudaError_t e = dev_alloc((void**)&blk, nz2 * sizeof(double2) + nd * sizeof(double) + ni * sizeof(int));
   if (e != cudaSuccess) { set_cuda_error("graph solve state", e); return 1; }
   QGState S;
   double2* z = reinterpret_cast<double2*>(blk);
@@ -706,7 +707,7 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
   const bool verbose = verbose_level() >= 2;
   const int scap = io.maxit + 64;
   unsigned long long* stamps = nullptr;
-  if (verbose && cudaMalloc((void**)&stamps, (size_t)(8 * scap + 1) * sizeof(unsigned long long)) != cudaSuccess)
+  if (verbose && dev_alloc((void**)&stamps, (size_t)(8 * scap + 1) * sizeof(unsigned long long)) != cudaSuccess)
     stamps = nullptr;
   auto stamp = [&](cudaStream_t s_, int slot, int bump) {
     if (stamps) k_qg_stamp<<<1, 1, 0, s_>>>(stamps, scap, slot, bump);
@@ -714,8 +715,8 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
   // partials of the MATVEC-fused vt^T A vt (x-first pipeline); else a separate sum kernel
   double2* xpart = nullptr;
   if (io.eng->xpipe) {
-    e = cudaMalloc((void**)&xpart, (size_t)R * xdot_blocks(io.eng->g) * sizeof(double2));
-    if (e != cudaSuccess) { cudaFree(blk); cudaFree(stamps); set_cuda_error("graph solve state", e); return 1; }
+    e = dev_alloc((void**)&xpart, (size_t)R * xdot_blocks(io.eng->g) * sizeof(double2));
+    if (e != cudaSuccess) { dev_free(blk); dev_free(stamps); set_cuda_error("graph solve state", e); return 1; }
   }
   cudaStream_t st = nullptr, st2 = nullptr;
   cudaStreamSynchronize(ops.stream);
@@ -732,9 +733,9 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
     e = cudaMemsetAsync(stamps, 0, (size_t)(8 * scap + 1) * sizeof(unsigned long long), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host vectors may be released afterwards
   if (e != cudaSuccess) {
-    if (st) cudaStreamDestroy(st);
+    if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
     if (st2) cudaStreamDestroy(st2);
-    cudaFree(blk); cudaFree(xpart); cudaFree(stamps);
+    dev_free(blk); dev_free(xpart); dev_free(stamps);
     set_cuda_error("graph solve streams and state", e);
     return 1;
   }
@@ -844,7 +845,7 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
     kq_pqv<C><<<dim3(ops.nb, R), BT, 0, st>>>(n, p, q, vt, atw, S.co, S.I, 2, ops.d_part, ops.d_out, ops.d_cnt);
     note_launch(2);
     int* h_active = nullptr;
-    e = cudaMallocHost((void**)&h_active, sizeof(int));
+    e = host_alloc((void**)&h_active, sizeof(int));
     long long launches = 0;
     const long long cap = (long long)maxit + 64;  // every RHS stops at maxit; the loop is bounded
     while (e == cudaSuccess && launches < cap) {
@@ -878,7 +879,7 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
                       ph[6] / cntv);
       }
     }
-    cudaFreeHost(h_active);
+    host_free(h_active);
     if (!rc) {
       std::vector<double> hd(nd);
       std::vector<int> hi(ni);
@@ -904,9 +905,9 @@ static int qmr_graph_loop(BatchIO<T>& io, BatchOps<T>& ops, std::vector<int>& nc
   cudaStreamSynchronize(st);
   cudaStreamDestroy(st);
   cudaStreamDestroy(st2);
-  cudaFree(blk);
-  cudaFree(xpart);
-  cudaFree(stamps);
+  dev_free(blk);
+  dev_free(xpart);
+  dev_free(stamps);
   return rc;
 }
 
@@ -1419,7 +1420,7 @@ template <typename T> struct PGGraph {
     for (int k = 0; k < 11; ++k) w[k] = w_[k];
     R = io->R; n = io->n;
     nz2 = (size_t)(6 + 7 + 2) * R; nd = (size_t)5 * R; ni = (size_t)11 * R + 4;
-    cudaError_t e = cudaMalloc((void**)&blk, nz2 * sizeof(double2) + nd * sizeof(double) + ni * sizeof(int));
+    cudaError_t e = dev_alloc((void**)&blk, nz2 * sizeof(double2) + nd * sizeof(double) + ni * sizeof(int));
     if (e != cudaSuccess) { set_cuda_error("graph solve state", e); return 1; }
     double2* z = reinterpret_cast<double2*>(blk);
     double2** zp[6] = {&S.alpha, &S.omega, &S.sigma, &S.rho0, &S.rho1, &S.beta};
@@ -1645,7 +1646,7 @@ template <typename T> struct PGGraph {
     if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
     if (st2) cudaStreamDestroy(st2);
     if (stw) cudaStreamDestroy(stw);
-    cudaFree(blk);
+    dev_free(blk);
     st = st2 = stw = nullptr;
     blk = nullptr;
   }
@@ -1682,8 +1683,8 @@ template <typename T> int pg_run(const std::vector<PGGraph<T>*>& gs) {
   cudaGraphExec_t exec = nullptr;
   int rc = 0;
   cudaError_t e = cudaStreamCreateWithFlags(&root, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_act, (size_t)nb * sizeof(int*) + sizeof(int));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h_sum, sizeof(int));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_act, (size_t)nb * sizeof(int*) + sizeof(int));
+  if (e == cudaSuccess) e = host_alloc((void**)&h_sum, sizeof(int));
   if (e == cudaSuccess) {
     d_sum = reinterpret_cast<int*>(d_act + nb);
     std::vector<int*> ha(nb);
@@ -1767,8 +1768,8 @@ template <typename T> int pg_run(const std::vector<PGGraph<T>*>& gs) {
   if (root) { cudaStreamSynchronize(root); cudaStreamDestroy(root); }
   for (auto ev : evs)
     if (ev) cudaEventDestroy(ev);
-  cudaFree(d_act);
-  cudaFreeHost(h_sum);
+  dev_free(d_act);
+  host_free(h_sum);
   return rc;
 }
 

@@ -28,6 +28,13 @@ void clear_error();
 int check_launch(const char* where);
 // console output level of the library (0 silent, 1 reference-style lines, 2 diagnostics)
 int verbose_level();
+// Blocks of device / pinned host memory from the library's reuse lists (mem.cu).
+// A block is freed only after the work that uses it has ended.
+cudaError_t dev_alloc(void** p, size_t bytes);
+void dev_free(void* p);
+cudaError_t host_alloc(void** p, size_t bytes);
+void host_free(void* p);
+void mem_trim();  // give every idle block back to the driver
 void raise_smem_limit(const void* f);  // thread-safe, once per kernel
 // an on/off environment switch: on when set to a non-empty value other than "0"
 bool env_flag(const char* name);

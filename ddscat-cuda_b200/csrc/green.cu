@@ -271,7 +271,7 @@ static double2* twiddles_d(int n) {
   const double pi = 3.14159265358979323846;
   for (int m = 0; m < n; ++m) h[m] = make_double2(std::cos(-2.0 * pi * m / n), std::sin(-2.0 * pi * m / n));
   double2* d = nullptr;
-  if (cudaMalloc((void**)&d, n * sizeof(double2)) != cudaSuccess) return nullptr;
+  if (dev_alloc((void**)&d, n * sizeof(double2)) != cudaSuccess) return nullptr;
   cudaMemcpy(d, h.data(), n * sizeof(double2), cudaMemcpyHostToDevice);
   return d;
 }
@@ -293,9 +293,9 @@ template <typename T> int Engine<T>::build_green(const GreenArgs<T>& ga) {
   double2 *a1 = nullptr, *a2 = nullptr;
   int* d_status = nullptr;
   int rc = 0;
-  cudaError_t e = cudaMalloc((void**)&a1, (size_t)6 * Mz * My * nxo * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&a2, (size_t)6 * Mz * nyo * nxo * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_status, sizeof(int));
+  cudaError_t e = dev_alloc((void**)&a1, (size_t)6 * Mz * My * nxo * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&a2, (size_t)6 * Mz * nyo * nxo * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_status, sizeof(int));
   if (e != cudaSuccess || !twx_d || !twy_d || !twz_d) {
     set_cuda_error("Green temporary allocation", e);
     rc = 2;
@@ -337,8 +337,8 @@ template <typename T> int Engine<T>::build_green(const GreenArgs<T>& ga) {
       rc = 14;
     }
   }
-  cudaFree(a1); cudaFree(a2); cudaFree(d_status);
-  cudaFree(twx_d); cudaFree(twy_d); cudaFree(twz_d);
+  dev_free(a1); dev_free(a2); dev_free(d_status);
+  dev_free(twx_d); dev_free(twy_d); dev_free(twz_d);
   return rc;
 }
 

@@ -129,10 +129,10 @@ int make_inputs(const Engine<float>& eng, int cmdpol, int nrhs, const float* k, 
   double2* d_e = nullptr;
   float2* d_tab = nullptr;
   int16_t* d_icomp = nullptr;
-  cudaError_t e = cudaMalloc((void**)&d_k, kv.size() * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_e, ev.size() * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_tab, tab.size() * sizeof(float2));
-  if (e == cudaSuccess && icomp_host) e = cudaMalloc((void**)&d_icomp, (size_t)g.nat * sizeof(int16_t));
+  cudaError_t e = dev_alloc((void**)&d_k, kv.size() * sizeof(double));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_e, ev.size() * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_tab, tab.size() * sizeof(float2));
+  if (e == cudaSuccess && icomp_host) e = dev_alloc((void**)&d_icomp, (size_t)g.nat * sizeof(int16_t));
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_k, kv.data(), kv.size() * sizeof(double), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_e, ev.data(), ev.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_tab, tab.data(), tab.size() * sizeof(float2), cudaMemcpyHostToDevice, st);
@@ -150,7 +150,8 @@ int make_inputs(const Engine<float>& eng, int cmdpol, int nrhs, const float* k, 
     if (check_launch("make_inputs")) rc = 613;
     else if ((e = cudaStreamSynchronize(st)) != cudaSuccess) { set_cuda_error("make_inputs", e); rc = 613; }
   }
-  cudaFree(d_k); cudaFree(d_e); cudaFree(d_tab); cudaFree(d_icomp);
+  if (rc) cudaStreamSynchronize(st);
+  dev_free(d_k); dev_free(d_e); dev_free(d_tab); dev_free(d_icomp);
   return rc;
 }
 

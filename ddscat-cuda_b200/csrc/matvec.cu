@@ -571,7 +571,7 @@ template <typename T> static cplx<T>* upload_twiddles(int n, size_t& bytes) {
     h[m] = mk<cplx<T>>(std::cos(a), std::sin(a));
   }
   cplx<T>* d = nullptr;
-  if (cudaMalloc((void**)&d, n * sizeof(cplx<T>)) != cudaSuccess) return nullptr;
+  if (dev_alloc((void**)&d, n * sizeof(cplx<T>)) != cudaSuccess) return nullptr;
   cudaMemcpy(d, h.data(), n * sizeof(cplx<T>), cudaMemcpyHostToDevice);
   bytes += n * sizeof(cplx<T>);
   return d;
@@ -651,10 +651,10 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
     rowq_h[r + 1] = rowq_h[r] + c;
   }
   cudaError_t e;
-  e = cudaMalloc((void**)&occ, (size_t)nat0 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&inv, (size_t)nat * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&iocc, (size_t)nat * sizeof(int16_t));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&rowq, ((size_t)nrows + 1) * sizeof(int));
+  e = dev_alloc((void**)&occ, (size_t)nat0 * sizeof(int));
+  if (e == cudaSuccess) e = dev_alloc((void**)&inv, (size_t)nat * sizeof(int));
+  if (e == cudaSuccess) e = dev_alloc((void**)&iocc, (size_t)nat * sizeof(int16_t));
+  if (e == cudaSuccess) e = dev_alloc((void**)&rowq, ((size_t)nrows + 1) * sizeof(int));
   if (e != cudaSuccess) { set_cuda_error("prepare: index maps", e); return 3; }
   bytes_allocated += (size_t)nat0 * 4 + (size_t)nat * 6 + ((size_t)nrows + 1) * 4;
   cudaMemcpy(occ, occ_h.data(), (size_t)nat0 * sizeof(int), cudaMemcpyHostToDevice);
@@ -662,7 +662,7 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   cudaMemcpy(rowq, rowq_h.data(), ((size_t)nrows + 1) * sizeof(int), cudaMemcpyHostToDevice);
   e = cudaMemcpy(iocc, iocc_host, (size_t)nat * sizeof(int16_t), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { set_cuda_error("prepare: index map H2D", e); return 3; }
-  e = cudaMalloc((void**)&green, g.green_count() * sizeof(C));
+  e = dev_alloc((void**)&green, g.green_count() * sizeof(C));
   if (e != cudaSuccess) { set_cuda_error("malloc resident Green", e); return 4; }
   bytes_allocated += g.green_count() * sizeof(C);
   // slab budget: FFT3D keeps the xy spectrum of all kz planes of up to 4 GiB
@@ -677,10 +677,11 @@ template <typename T> int Engine<T>::ensure_workspace(int nrhs) {
   const size_t per_plane = plane_per_rhs();
   const int nplanes_all = xpipe ? g.Mx : g.Mz;
   if (nrhs <= zcap && zhat) return 0;
-  if (zhat) { cudaFree(zhat); bytes_allocated -= (size_t)zcap * per_rhs_z * sizeof(C); zhat = nullptr; }
-  if (slab) { cudaFree(slab); bytes_allocated -= (size_t)slab_nr * slab_B * per_plane * sizeof(C); slab = nullptr; }
+  if (zhat || slab) cudaStreamSynchronize(stream);  // no MATVEC in flight on the old workspace
+  if (zhat) { dev_free(zhat); bytes_allocated -= (size_t)zcap * per_rhs_z * sizeof(C); zhat = nullptr; }
+  if (slab) { dev_free(slab); bytes_allocated -= (size_t)slab_nr * slab_B * per_plane * sizeof(C); slab = nullptr; }
   zcap = nrhs;
-  cudaError_t e = cudaMalloc((void**)&zhat, (size_t)zcap * per_rhs_z * sizeof(C));
+  cudaError_t e = dev_alloc((void**)&zhat, (size_t)zcap * per_rhs_z * sizeof(C));
   if (e != cudaSuccess) { zcap = 0; set_cuda_error("malloc z-spectrum workspace", e); return 1; }
   bytes_allocated += (size_t)zcap * per_rhs_z * sizeof(C);
   if (slices_layout) {
@@ -699,7 +700,7 @@ template <typename T> int Engine<T>::ensure_workspace(int nrhs) {
     else if (full_rhs <= slab_budget_elems) { slab_nr = (int)std::max<size_t>(1, slab_budget_elems / full_rhs); slab_B = nplanes_all; }
     else { slab_nr = 1; slab_B = (int)std::max<size_t>(1, slab_budget_elems / per_plane); }
   }
-  e = cudaMalloc((void**)&slab, (size_t)slab_nr * slab_B * per_plane * sizeof(C));
+  e = dev_alloc((void**)&slab, (size_t)slab_nr * slab_B * per_plane * sizeof(C));
   if (e != cudaSuccess) { set_cuda_error("malloc xy-slab workspace", e); return 1; }
   bytes_allocated += (size_t)slab_nr * slab_B * per_plane * sizeof(C);
   return 0;
@@ -836,20 +837,21 @@ template <typename T> int Engine<T>::interleave_green(const C* planar_dev) {
 
 template <typename T> int Engine<T>::upload_green(const void* host_green) {
   C* tmp = nullptr;
-  cudaError_t e = cudaMalloc((void**)&tmp, g.green_count() * sizeof(C));
+  cudaError_t e = dev_alloc((void**)&tmp, g.green_count() * sizeof(C));
   if (e == cudaSuccess) e = cudaMemcpy(tmp, host_green, g.green_count() * sizeof(C), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) { cudaFree(tmp); set_cuda_error("green H2D", e); return 4; }
+  if (e != cudaSuccess) { dev_free(tmp); set_cuda_error("green H2D", e); return 4; }
   int rc = interleave_green(tmp);
   e = cudaStreamSynchronize(stream);
-  cudaFree(tmp);
+  dev_free(tmp);
   if (rc || e != cudaSuccess) { if (!rc) set_cuda_error("green interleave", e); return 4; }
   return 0;
 }
 
 template <typename T> void Engine<T>::release() {
-  cudaFree(twx); cudaFree(twy); cudaFree(twz);
-  cudaFree(green); cudaFree(occ); cudaFree(inv); cudaFree(iocc); cudaFree(rowq);
-  cudaFree(zhat); cudaFree(slab); cudaFree(d_err);
+  cudaFree(d_err);  // waits for the device: nothing uses the engine's blocks any more
+  dev_free(twx); dev_free(twy); dev_free(twz);
+  dev_free(green); dev_free(occ); dev_free(inv); dev_free(iocc); dev_free(rowq);
+  dev_free(zhat); dev_free(slab);
   *this = Engine<T>{};
 }
 
@@ -864,10 +866,10 @@ int autotune_engine(Engine<float>& e, int iters, float* default_ms, float* best_
   const Geometry& g = e.g;
   const size_t cn = (size_t)3 * g.nat0;
   C *x = nullptr, *y = nullptr, *ad = nullptr;
-  cudaError_t err = cudaMalloc((void**)&x, cn * sizeof(C));
-  if (err == cudaSuccess) err = cudaMalloc((void**)&y, cn * sizeof(C));
-  if (err == cudaSuccess) err = cudaMalloc((void**)&ad, cn * sizeof(C));
-  if (err != cudaSuccess) { cudaFree(x); cudaFree(y); cudaFree(ad); set_cuda_error("autotune", err); return 1; }
+  cudaError_t err = dev_alloc((void**)&x, cn * sizeof(C));
+  if (err == cudaSuccess) err = dev_alloc((void**)&y, cn * sizeof(C));
+  if (err == cudaSuccess) err = dev_alloc((void**)&ad, cn * sizeof(C));
+  if (err != cudaSuccess) { dev_free(x); dev_free(y); dev_free(ad); set_cuda_error("autotune", err); return 1; }
   cudaMemsetAsync(x, 0, cn * sizeof(C), e.stream);
   cudaMemsetAsync(ad, 0, cn * sizeof(C), e.stream);
   MvArgs<float> a;
@@ -928,7 +930,8 @@ int autotune_engine(Engine<float>& e, int iters, float* default_ms, float* best_
   e.tune_zg = best.zg;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  cudaFree(x); cudaFree(y); cudaFree(ad);
+  if (rc) cudaStreamSynchronize(e.stream);
+  dev_free(x); dev_free(y); dev_free(ad);
   if (rc) return 1;
   *default_ms = dms;
   *best_ms = bms;

@@ -42,7 +42,7 @@ struct Target {
   void release() {
     ops.release();
     eng.release();
-    cudaFree(b); cudaFree(x); cudaFree(adia); cudaFree(work); cudaFree(full); cudaFree(occ);
+    dev_free(b); dev_free(x); dev_free(adia); dev_free(work); dev_free(full); dev_free(occ);
     if (st) cudaStreamDestroy(st);
     *this = Target{};
   }
@@ -98,7 +98,7 @@ int multi_solve(int nt, const int* dims, const int16_t* const* iocc, const float
           occ_h.push_back(j);
         }
     t.nat = nat;
-    if (cudaMalloc((void**)&t.occ, (size_t)nat0 * sizeof(int)) != cudaSuccess ||
+    if (dev_alloc((void**)&t.occ, (size_t)nat0 * sizeof(int)) != cudaSuccess ||
         cudaMemcpy(t.occ, occ_h.data(), (size_t)nat0 * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
       set_error("multi-target solve", "index map");
       cleanup();
@@ -122,11 +122,11 @@ int multi_solve(int nt, const int* dims, const int16_t* const* iocc, const float
     t.first = first;
     first += t.R;
     const size_t v = (size_t)t.R * t.n, full = (size_t)3 * nat;
-    cudaError_t e = cudaMalloc((void**)&t.b, v * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t.x, v * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t.adia, v * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(float2));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t.full, full * sizeof(float2));
+    cudaError_t e = dev_alloc((void**)&t.b, v * sizeof(float2));
+    if (e == cudaSuccess) e = dev_alloc((void**)&t.x, v * sizeof(float2));
+    if (e == cudaSuccess) e = dev_alloc((void**)&t.adia, v * sizeof(float2));
+    if (e == cudaSuccess) e = dev_alloc((void**)&t.work, (size_t)BATCH_WORK_VECTORS * v * sizeof(float2));
+    if (e == cudaSuccess) e = dev_alloc((void**)&t.full, full * sizeof(float2));
     if (e != cudaSuccess) { set_cuda_error("multi-target workspace", e); cleanup(); return 542; }
     if (t.ops.init(t.R, t.n, t.st)) { cleanup(); return 542; }
     lap(2, ta);

@@ -206,11 +206,11 @@ static int ff_sums_impl(const int* occ, int nx, int ny, int nz, int nat0, const 
   TC* tab = nullptr;
   double2 *partials = nullptr, *sums = nullptr;
   int rc = 0;
-  cudaError_t e = cudaMalloc((void**)&coords, (size_t)nat0 * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_dirs, (size_t)3 * chunk * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&tab, (size_t)chunk * ntab * sizeof(TC));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&partials, (size_t)chunk * NS * nblocks * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&sums, (size_t)chunk * NS * sizeof(double2));
+  cudaError_t e = dev_alloc((void**)&coords, (size_t)nat0 * sizeof(unsigned));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_dirs, (size_t)3 * chunk * sizeof(double));
+  if (e == cudaSuccess) e = dev_alloc((void**)&tab, (size_t)chunk * ntab * sizeof(TC));
+  if (e == cudaSuccess) e = dev_alloc((void**)&partials, (size_t)chunk * NS * nblocks * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&sums, (size_t)chunk * NS * sizeof(double2));
   if (e != cudaSuccess) { set_cuda_error("SCAT workspace", e); rc = 322; }
   if (!rc) {
     k_pack_coords<<<(unsigned)ceil_div(nat0, 256), 256, 0, s>>>(occ, nat0, nx, ny, coords);
@@ -239,7 +239,8 @@ static int ff_sums_impl(const int* occ, int nx, int ny, int nz, int nat0, const 
       if (e != cudaSuccess) { set_cuda_error("SCAT sums D2H", e); rc = 329; }
     }
   }
-  cudaFree(coords); cudaFree(d_dirs); cudaFree(tab); cudaFree(partials); cudaFree(sums);
+  if (rc) cudaStreamSynchronize(s);
+  dev_free(coords); dev_free(d_dirs); dev_free(tab); dev_free(partials); dev_free(sums);
   return rc;
 }
 
@@ -318,7 +319,7 @@ int incident_torque(Engine<T>& eng, const cplx<T>* p, const cplx<T>* e, const fl
   const int nat0 = eng.g.nat0;
   const int nblocks = (int)std::min<size_t>(ceil_div((size_t)nat0, 256), 1184);
   double* d = nullptr;
-  cudaError_t e1 = cudaMalloc((void**)&d, ((size_t)nblocks * 6 + 6) * sizeof(double));
+  cudaError_t e1 = dev_alloc((void**)&d, ((size_t)nblocks * 6 + 6) * sizeof(double));
   if (e1 != cudaSuccess) { set_cuda_error("torque workspace", e1); return 341; }
   SitePos pos;
   for (int i = 0; i < 3; ++i) { pos.x0[i] = x0[i]; pos.dx[i] = dx[i]; }
@@ -333,7 +334,8 @@ int incident_torque(Engine<T>& eng, const cplx<T>* p, const cplx<T>* e, const fl
     if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(s);
     if (e1 != cudaSuccess) { set_cuda_error("torque sums D2H", e1); rc = 343; }
   }
-  cudaFree(d);
+  if (rc) cudaStreamSynchronize(s);
+  dev_free(d);
   return rc;
 }
 
@@ -435,7 +437,7 @@ static int mueller_impl(int ndir, const R* ak, const cplx<R>* e01, const cplx<R>
   const size_t off_f = ((size_t)ndir * 3 * sizeof(R) + 15) & ~(size_t)15;  // 16-byte aligned f block
   const size_t nb = off_f + (size_t)ndir * (8 * sizeof(C) + 16 * sizeof(double));
   unsigned char* buf = nullptr;
-  cudaError_t e = cudaMalloc((void**)&buf, nb);
+  cudaError_t e = dev_alloc((void**)&buf, nb);
   if (e != cudaSuccess) { set_cuda_error("Mueller workspace", e); return 701; }
   R* d_em2 = reinterpret_cast<R*>(buf);
   C* d_f = reinterpret_cast<C*>(buf + off_f);
@@ -445,14 +447,14 @@ static int mueller_impl(int ndir, const R* ak, const cplx<R>* e01, const cplx<R>
   e = cudaMemcpy(d_em2, em2, (size_t)ndir * 3 * sizeof(R), cudaMemcpyHostToDevice);
   for (int k = 0; k < 4 && e == cudaSuccess; ++k)
     e = cudaMemcpy(d_f + (size_t)k * ndir, hf[k], (size_t)ndir * sizeof(C), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) { cudaFree(buf); set_cuda_error("Mueller H2D", e); return 702; }
+  if (e != cudaSuccess) { dev_free(buf); set_cuda_error("Mueller H2D", e); return 702; }
   k_mueller<R><<<(unsigned)ceil_div(ndir, 128), 128>>>(ndir, in, d_em2, d_f, d_f + ndir, d_f + 2 * (size_t)ndir,
                                                        d_f + 3 * (size_t)ndir, d_s, d_m);
   note_launch();
-  if (check_launch("Mueller kernel")) { cudaFree(buf); return 703; }
+  if (check_launch("Mueller kernel")) { dev_free(buf); return 703; }
   if (s_out) e = cudaMemcpy(s_out, d_s, (size_t)ndir * 4 * sizeof(C), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(m_out, d_m, (size_t)ndir * 16 * sizeof(double), cudaMemcpyDeviceToHost);
-  cudaFree(buf);
+  dev_free(buf);
   if (e != cudaSuccess) { set_cuda_error("Mueller D2H", e); return 702; }
   return 0;
 }

@@ -374,10 +374,10 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
   DPState* hS = nullptr;
   cudaEvent_t ev = nullptr;
   struct Free {
-    DPState*& a; DPState*& b; cudaEvent_t& e;
-    ~Free() { cudaFree(a); if (b) cudaFreeHost(b); if (e) cudaEventDestroy(e); }
-  } release{dS, hS, ev};
-  if (cudaMalloc((void**)&dS, sizeof(DPState)) != cudaSuccess || cudaMallocHost((void**)&hS, sizeof(DPState)) != cudaSuccess ||
+    DPState*& a; DPState*& b; cudaEvent_t& e; cudaStream_t st;
+    ~Free() { cudaStreamSynchronize(st); dev_free(a); if (b) host_free(b); if (e) cudaEventDestroy(e); }
+  } release{dS, hS, ev, io.stream};
+  if (dev_alloc((void**)&dS, sizeof(DPState)) != cudaSuccess || host_alloc((void**)&hS, sizeof(DPState)) != cudaSuccess ||
       cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     set_error(name, "scalar state allocation");
@@ -540,10 +540,10 @@ template <typename T> int solve_qmrccg(SolveIO<T>& io) {
   DQState* hS = nullptr;
   cudaEvent_t ev = nullptr;
   struct Free {
-    DQState*& a; DQState*& b; cudaEvent_t& e;
-    ~Free() { cudaFree(a); if (b) cudaFreeHost(b); if (e) cudaEventDestroy(e); }
-  } release{dS, hS, ev};
-  if (cudaMalloc((void**)&dS, sizeof(DQState)) != cudaSuccess || cudaMallocHost((void**)&hS, sizeof(DQState)) != cudaSuccess ||
+    DQState*& a; DQState*& b; cudaEvent_t& e; cudaStream_t st;
+    ~Free() { cudaStreamSynchronize(st); dev_free(a); if (b) host_free(b); if (e) cudaEventDestroy(e); }
+  } release{dS, hS, ev, io.stream};
+  if (dev_alloc((void**)&dS, sizeof(DQState)) != cudaSuccess || host_alloc((void**)&hS, sizeof(DQState)) != cudaSuccess ||
       cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     set_error(name, "scalar state allocation");

@@ -132,18 +132,19 @@ __global__ void __launch_bounds__(RED_THREADS) k_dots(int n, DotSpec<T> sp, doub
 template <typename T> int VecOps<T>::init(cudaStream_t s) {
   stream = s;
   nblocks = 8 * 148;  // capacity of the partials buffer; launch_dots sizes each launch to one resident wave
-  cudaError_t e = cudaMalloc((void**)&d_red, (size_t)RED_MAXK * nblocks * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_out, RED_MAXK * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&d_count, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&h_out, RED_MAXK * sizeof(double2));
+  cudaError_t e = dev_alloc((void**)&d_red, (size_t)RED_MAXK * nblocks * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_out, RED_MAXK * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&d_count, sizeof(unsigned));
+  if (e == cudaSuccess) e = host_alloc((void**)&h_out, RED_MAXK * sizeof(double2));
   if (e != cudaSuccess) { set_cuda_error("reduction buffers", e); return 1; }
   cudaMemset(d_count, 0, sizeof(unsigned));
   return 0;
 }
 
 template <typename T> void VecOps<T>::release() {
-  cudaFree(d_red); cudaFree(d_out); cudaFree(d_count);
-  if (h_out) cudaFreeHost(h_out);
+  if (d_red) cudaStreamSynchronize(stream);
+  dev_free(d_red); dev_free(d_out); dev_free(d_count);
+  if (h_out) host_free(h_out);
   d_red = d_out = nullptr; d_count = nullptr; h_out = nullptr;
 }
 
