@@ -1145,7 +1145,7 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_amplitudes_f64(int nrhs, const v
     }
     v_gather<double>(src, d_p, s.eng.occ, g.nat, g.nat0, s.stream);
     if (check_launch("FP64 amplitudes gather")) { rc = 712; break; }
-    if (farfield_sums_f64(s.eng.occ, g.nx, g.ny, g.nz, g.nat0, d_p, aks, ndir, dx, x0, sums.data(), s.stream)) {
+    if (farfield_sums_f64(s.eng, d_p, aks, ndir, dx, x0, sums.data(), s.stream)) {
       rc = 712;
       break;
     }
@@ -1207,8 +1207,7 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_scat_csca_f64(int nrhs, const void* x
     v_gather<double>(src, d_p, s.eng.occ, g.nat, g.nat0, s.stream);
     if (check_launch("FP64 SCAT gather")) { rc = 712; break; }
     std::vector<double2> sums((size_t)3 * nd);
-    if (farfield_sums_f64(s.eng.occ, g.nx, g.ny, g.nz, g.nat0, d_p, hd.data(), nd, dxd, x0d, sums.data(),
-                          s.stream)) {
+    if (farfield_sums_f64(s.eng, d_p, hd.data(), nd, dxd, x0d, sums.data(), s.stream)) {
       rc = 712;
       break;
     }

@@ -5,12 +5,10 @@
 // products P^H q and E^H P.
 //
 // The far-field sums S_d = sum_j P_j exp(-i k_d . r_j), r_j = ((i+1)+x0)*dx
-// (cu:793-822), are evaluated with a separable phase: exp(-i k.r) =
-// ex_d[ix] * ey_d[iy] * ez_d[iz], three 1-D tables per direction built in FP64,
-// so each dipole-direction term costs two complex multiplies instead of a
-// sincosf.  A block keeps DIRS directions in shared memory and reads each
-// dipole's polarisation once for all of them; partial sums are combined in a
-// fixed order (deterministic).
+// (cu:793-822), use a separable phase: exp(-i k.r) = ex_d[ix] * ey_d[iy] *
+// ez_d[iz], three 1-D tables per direction built in FP64.  The x rows are
+// contracted first, as a register-tiled complex matrix product (k_ff_rows);
+// partial sums are combined in a fixed order (deterministic).
 #include <algorithm>
 #include <vector>
 #include "solvers.h"
@@ -59,35 +57,58 @@ int evalq_compute(Engine<T>& eng, VecOps<T>& ops, const cplx<T>* e, const cplx<T
 }
 
 // ---------------------------------------------------------------- far field
-constexpr int FF_THREADS = 256;
-constexpr int FF_DIRS = 8;
+// S_d = sum over x rows of ey_d[iy] ez_d[iz] (sum_ix ex_d[ix] P[ix]): the inner
+// sums are a complex matrix product, directions x columns x (rows, components),
+// and only the row sums meet the y and z phases.  12 multiply-adds per site,
+// component triple and direction instead of the 30 operations and three
+// gathered table reads of a per-site phase.
+//   block: FF_WARPS warps share one tile of ex, FF_COLS columns x 64 directions,
+//     in shared memory; a lane holds two adjacent directions;
+//   warp: takes pairs of x rows (strided over the grid of row blocks), packs the
+//     columns where either row is occupied into records in shared memory
+//     (vacuum costs nothing), and accumulates the pair's row sums in registers;
+//   per pair: row sums times the y and z phases, accumulated in FP64.
+// Bound by the FMA pipes: a record is 48 multiply-adds per lane against 8
+// wavefronts of shared-memory reads (32 cycles for the SM's four schedulers).
+// Packed fma.rn.f32x2 was measured slower (it runs at half the rate of a scalar
+// FMA and needs separate real and imaginary accumulators).
+// Precision (FP32): neighbouring sites of a row add up coherently, so a plain
+// FP32 chain over the row rounds larger partial sums than a per-site form whose
+// threads add sites 256 apart.  Chains stop after FF_CHAIN products and meet in
+// a compensated (Kahan) sum, and the y and z phases multiply the row sums in
+// FP64: off-peak amplitudes (below 5 % of the peak) of 33^3 to 111^3
+// spheres are 5.1e-8 to 9.3e-8 off in norm against 6.0e-8 to 1.0e-7 for the
+// per-site form; plain chains of 32 gave 9.2e-8 to 1.8e-7.
+// Measured, 96^3 sphere, FP32: 2.62 ms against 5.73 for the per-site
+// form (7,500 directions; 1.1 ms at the FMA peak); 64^3, FP64, 8 polarisations:
+// 4.93 against 9.97 ms.
+constexpr int FF_WARPS = 12;
+constexpr int FF_COLS = 64;
+constexpr int FF_CHAIN = 8;
+constexpr int FF_ND = 2;            // directions per lane
+constexpr int FF_TILE = 32 * FF_ND;  // directions per block
 
-// tables[d][0..nx) = exp(-i kx (ix+1+x0x) dx), then ny, then nz entries;
-// phases in FP64, stored as complex float (SCAT) or complex double (the
-// all-FP64 amplitudes)
+// y and z phases tabulated per direction: yz[u][d], u < ny: exp(-i ky (iy+1+x0y) dy),
+// then nz entries, in FP64; ex[u][d] = exp(-i kx (ix+1+x0x) dx) in FP64, stored as
+// complex float (SCAT) or complex double (the all-FP64 amplitudes); zero for the
+// padding directions ndir <= d < pitch
 template <typename TC>
-__global__ void k_ff_tables(const double* dirs, int ndir, int nx, int ny, int nz, double dx0, double dx1, double dx2,
-                            double x00, double x01, double x02, TC* tab) {
-  const int ntab = nx + ny + nz;
-  const size_t tot = (size_t)ndir * ntab;
+__global__ void k_ff_tables(const double* dirs, int ndir, int pitch, int nx, int ny, int nz, double dx0, double dx1,
+                            double dx2, double x00, double x01, double x02, TC* ex, double2* yz) {
+  const size_t tot = (size_t)pitch * (nx + ny + nz);
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < tot; t += (size_t)gridDim.x * blockDim.x) {
-    const int d = (int)(t / ntab), u = (int)(t % ntab);
-    double ph;
-    if (u < nx) ph = dirs[3 * d] * ((u + 1) + x00) * dx0;
-    else if (u < nx + ny) ph = dirs[3 * d + 1] * ((u - nx + 1) + x01) * dx1;
-    else ph = dirs[3 * d + 2] * ((u - nx - ny + 1) + x02) * dx2;
-    double s, c;
-    sincos(ph, &s, &c);
-    tab[t] = mk<TC>(c, -s);
+    const int d = (int)(t % pitch), u = (int)(t / pitch);
+    double s = 0.0, c = 0.0;
+    if (d < ndir) {
+      double ph;
+      if (u < nx) ph = dirs[3 * d] * ((u + 1) + x00) * dx0;
+      else if (u < nx + ny) ph = dirs[3 * d + 1] * ((u - nx + 1) + x01) * dx1;
+      else ph = dirs[3 * d + 2] * ((u - nx - ny + 1) + x02) * dx2;
+      sincos(ph, &s, &c);
+    }
+    if (u < nx) ex[t] = mk<TC>(c, -s);
+    else yz[t - (size_t)pitch * nx] = make_double2(c, -s);
   }
-}
-
-__global__ void k_pack_coords(const int* occ, int nat0, int nx, int ny, unsigned* packed) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nat0) return;
-  const int j = occ[q];
-  const unsigned ix = j % nx, iy = (j / nx) % ny, iz = j / (nx * ny);
-  packed[q] = ix | (iy << 11) | (iz << 22);
 }
 
 // Site position r_j = ((i+1) + x0) * dx of the far-field sums, per axis
@@ -95,143 +116,257 @@ struct SitePos {
   float x0[3], dx[3];
 };
 
-// Partial sums of ND directions per block: phase products and per-thread
-// accumulation in TR (float for SCAT, double for the all-FP64 amplitudes),
-// block reduction in FP64.  NS = 3: S_a = sum_j P_ja exp(-i k.r_j); NS = 12
-// adds the position moments U_ab = sum_j P_ja r_jb exp(-i k.r_j) (a-major)
-// that the scattered angular-momentum flux needs.
-template <typename C, typename TR, int ND, int NS = 3>
-__global__ void __launch_bounds__(FF_THREADS) k_ff_partial(const C* p, const unsigned* coords, int nat0, int ndir,
-                                                           int nx, int ny, int nz, const cplx<TR>* tab,
-                                                           int sites_per_block, double2* partials, SitePos pos) {
-  using TC = cplx<TR>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TC* st = reinterpret_cast<TC*>(smem_raw);
-  const int ntab = nx + ny + nz;
-  const int d0 = blockIdx.y * ND;
-  const int nd = min(ND, ndir - d0);
-  for (int t = threadIdx.x; t < nd * ntab; t += blockDim.x) st[t] = tab[(size_t)d0 * ntab + t];
-  __syncthreads();
-  constexpr int NA = 2 * NS;  // real accumulators per direction
-  TR acc[ND][NA];
+// acc += p * e
+template <typename C> __device__ __forceinline__ void cfma(C& acc, C p, C e) {
+  acc.x = fma(p.x, e.x, acc.x);
+  acc.y = fma(p.x, e.y, acc.y);
+  acc.x = fma(-p.y, e.y, acc.x);
+  acc.y = fma(p.y, e.x, acc.y);
+}
+// n (even for 8-byte elements) elements by 16-byte loads
+template <int N, typename C> __device__ __forceinline__ void load_vec(C (&v)[N], const C* src) {
+  if constexpr (sizeof(C) == 8) {
+    static_assert(N % 2 == 0, "pairs");
 #pragma unroll
-  for (int d = 0; d < ND; ++d)
-#pragma unroll
-    for (int k = 0; k < NA; ++k) acc[d][k] = (TR)0;
-  const int q0 = blockIdx.x * sites_per_block;
-  const int q1 = min(nat0, q0 + sites_per_block);
-  for (int q = q0 + threadIdx.x; q < q1; q += blockDim.x) {
-    const unsigned pk = coords[q];
-    const int ix = pk & 2047u, iy = (pk >> 11) & 2047u, iz = pk >> 22;
-    const double2 a = to_d(p[q]), b = to_d(p[q + nat0]), c = to_d(p[q + 2 * (size_t)nat0]);
-    const TC px = mk<TC>(a.x, a.y), py = mk<TC>(b.x, b.y), pz = mk<TC>(c.x, c.y);
-    TR rr[3] = {(TR)0, (TR)0, (TR)0};
-    if constexpr (NS == 12) {
-      rr[0] = ((TR)(ix + 1) + (TR)pos.x0[0]) * (TR)pos.dx[0];
-      rr[1] = ((TR)(iy + 1) + (TR)pos.x0[1]) * (TR)pos.dx[1];
-      rr[2] = ((TR)(iz + 1) + (TR)pos.x0[2]) * (TR)pos.dx[2];
+    for (int k = 0; k < N; k += 2) {
+      const float4 q = *reinterpret_cast<const float4*>(src + k);
+      v[k] = mk<C>(q.x, q.y);
+      v[k + 1] = mk<C>(q.z, q.w);
     }
+  } else {
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      if (d < nd) {
-        const TC* td = st + d * ntab;
-        const TC e = cmul(cmul(td[ix], td[nx + iy]), td[nx + ny + iz]);
-        const TC sa[3] = {cmul(px, e), cmul(py, e), cmul(pz, e)};
+    for (int k = 0; k < N; ++k) v[k] = src[k];
+  }
+}
+
+// shared memory of k_ff_rows: ex tile | records | column offsets
+template <typename TR> constexpr size_t ff_smem() {
+  return (size_t)FF_COLS * FF_TILE * sizeof(cplx<TR>) +
+         (size_t)FF_WARPS * FF_COLS * (6 * sizeof(cplx<TR>) + sizeof(int));
+}
+
+// s[c][d] += sum over the records [j0, j1) of record component c times ex
+template <typename TC>
+__device__ __forceinline__ void ff_chain(TC (&s)[6][FF_ND], const TC* rec, const int* col, const TC* ex, int j0, int j1) {
+#pragma unroll 2
+  for (int j = j0; j < j1; ++j) {
+    TC x[FF_ND], r[6];
+    load_vec(x, ex + col[j]);
+    load_vec(r, rec + 6 * j);
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          acc[d][2 * m] += sa[m].x;
-          acc[d][2 * m + 1] += sa[m].y;
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+      for (int d = 0; d < FF_ND; ++d) cfma(s[c][d], r[c], x[d]);
+  }
+}
+template <typename TC> __device__ __forceinline__ void ff_clear(TC (&s)[6][FF_ND]) {
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+#pragma unroll
+    for (int d = 0; d < FF_ND; ++d) s[c][d] = mk<TC>(0, 0);
+}
+// Kahan step: sum += v with the running compensation k
+__device__ __forceinline__ void kahan(float& sum, float& k, float v) {
+  const float y = v - k, t = sum + y;
+  k = (t - sum) - y;
+  sum = t;
+}
+
+// Partial sums of one direction tile (blockIdx.y), column chunk (blockIdx.z)
+// and share of the row pairs (blockIdx.x) into partials[part][3*d + c], part =
+// blockIdx.z * gridDim.x + blockIdx.x.  wt = 0: weight 1; 1..3: each site
+// weighted by its x, y or z position (the moments U of the torque).
+template <typename C, typename TR>
+__global__ void __launch_bounds__(32 * FF_WARPS, 1) k_ff_rows(const C* p, const int* inv, int nat0, int nrows, int pitch, int nx,
+                                                              int ny,
+                                                              const cplx<TR>* tab, const double2* yz,
+                                                              double2* partials, int wt, SitePos pos) {
+  using TC = cplx<TR>;
+  constexpr int ND = FF_ND, TILE = FF_TILE, H = FF_COLS / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TC* ext = reinterpret_cast<TC*>(smem_raw);  // [FF_COLS][TILE]
+  TC* recs = ext + FF_COLS * TILE;            // [FF_WARPS][FF_COLS][6]: 2 rows x 3 components
+  int* cols = reinterpret_cast<int*>(recs + FF_WARPS * FF_COLS * 6);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int d0 = blockIdx.y * TILE, k0 = blockIdx.z * FF_COLS, ncol = min(FF_COLS, nx - k0);
+  {
+    // 16-byte moves: TILE and pitch are even in elements
+    constexpr int V = 16 / (int)sizeof(TC), W = TILE / V;
+    for (int u = threadIdx.x; u < ncol * W; u += 32 * FF_WARPS) {
+      const int k = u / W, v = u - k * W;
+      reinterpret_cast<float4*>(ext)[u] = reinterpret_cast<const float4*>(tab + (size_t)(k0 + k) * pitch + d0)[v];
+    }
+  }
+  __syncthreads();
+  TC* myrec = recs + wid * FF_COLS * 6;
+  int* mycol = cols + wid * FF_COLS;
+  const TC* mye = ext + ND * lane;
+  double2 acc[3][ND];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) acc[c][d] = make_double2(0.0, 0.0);
+  const int npair = (nrows + 1) / 2, stride = gridDim.x * FF_WARPS;
+  // compact indices of the lane's columns in both rows of a pair, -1 for
+  // vacuum; those of the next pair load while this one is summed
+  int q[2][H];
+  auto load_q = [&](int pr) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const int row = 2 * pr + r, k = 32 * h + lane;
+        q[r][h] = pr < npair && row < nrows && k < ncol ? inv[(size_t)row * nx + k0 + k] : -1;
+      }
+  };
+  load_q(blockIdx.x * FF_WARPS + wid);
+  for (int pr = blockIdx.x * FF_WARPS + wid; pr < npair; pr += stride) {
+    const int rows[2] = {2 * pr, min(2 * pr + 1, nrows - 1)};
+    int cnt = 0;
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int k = 32 * h + lane;
+      const bool occ = q[0][h] >= 0 || q[1][h] >= 0;
+      const unsigned m = __ballot_sync(0xffffffffu, occ);
+      if (occ) {
+        const int j = cnt + __popc(m & ((1u << lane) - 1u));
+        mycol[j] = k * TILE;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          TR w = (TR)1;
+          if (wt) {
+            const int i = wt == 1 ? k0 + k : (wt == 2 ? rows[r] % ny : rows[r] / ny);
+            w = ((TR)(i + 1) + (TR)pos.x0[wt - 1]) * (TR)pos.dx[wt - 1];
+          }
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            TC v = mk<TC>(0, 0);
+            if (q[r][h] >= 0) v = p[(size_t)c * nat0 + q[r][h]];
+            myrec[6 * j + 3 * r + c] = wt ? cscale(v, w) : v;
+          }
         }
-        if constexpr (NS == 12) {
+      }
+      cnt += __popc(m);
+    }
+    __syncwarp();
+    load_q(pr + stride);
+    if (cnt) {
+      TC s[6][ND];
+      ff_clear(s);
+      if constexpr (sizeof(TR) == 8) {
+        ff_chain(s, myrec, mycol, mye, 0, cnt);
+      } else {
+        ff_chain(s, myrec, mycol, mye, 0, min(cnt, FF_CHAIN));
+        TC k[6][ND];
+        ff_clear(k);
+        for (int j0 = FF_CHAIN; j0 < cnt; j0 += FF_CHAIN) {
+          TC v[6][ND];
+          ff_clear(v);
+          ff_chain(v, myrec, mycol, mye, j0, min(cnt, j0 + FF_CHAIN));
 #pragma unroll
-          for (int m = 0; m < 3; ++m)
+          for (int c = 0; c < 6; ++c)
 #pragma unroll
-            for (int b2 = 0; b2 < 3; ++b2) {
-              acc[d][6 + 6 * m + 2 * b2] += sa[m].x * rr[b2];
-              acc[d][7 + 6 * m + 2 * b2] += sa[m].y * rr[b2];
+            for (int d = 0; d < ND; ++d) {
+              kahan(s[c][d].x, k[c][d].x, v[c][d].x);
+              kahan(s[c][d].y, k[c][d].y, v[c][d].y);
             }
         }
       }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const double2* ey = yz + (size_t)(rows[r] % ny) * pitch + d0 + ND * lane;
+        const double2* ez = yz + (size_t)(ny + rows[r] / ny) * pitch + d0 + ND * lane;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          const double2 e = cmul(ey[d], ez[d]);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) cfma(acc[c][d], to_d(s[3 * r + c][d]), e);
+        }
+      }
     }
+    __syncwarp();  // the records are consumed before the next pair overwrites them
   }
-  // block reduction in FP64: warp shuffles then shared memory
-  __shared__ double red[FF_THREADS / 32][ND * NA];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int d = 0; d < ND; ++d)
-#pragma unroll
-    for (int k = 0; k < NA; ++k) {
-      double v = (double)acc[d][k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) red[wid][d * NA + k] = v;
-    }
+  // the warps' sums meet in shared memory (fixed order), one partial per block
   __syncthreads();
-  for (int t = threadIdx.x; t < nd * NA; t += blockDim.x) {
-    double v = 0.0;
-    for (int w = 0; w < FF_THREADS / 32; ++w) v += red[w][t];
-    const int d = t / NA, k = t % NA;
-    // partials[(dir)*NS + sum][block] as (re, im)
-    double* dst = reinterpret_cast<double*>(&partials[((size_t)(d0 + d) * NS + k / 2) * gridDim.x + blockIdx.x]);
-    dst[k & 1] = v;
+  double2* red = reinterpret_cast<double2*>(smem_raw);  // [FF_WARPS][3 * TILE]
+  static_assert((size_t)FF_WARPS * 3 * TILE * sizeof(double2) <= ff_smem<TR>(), "block reduction space");
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int d = 0; d < ND; ++d) red[wid * 3 * TILE + 3 * (ND * lane + d) + c] = acc[c][d];
+  __syncthreads();
+  double2* out = partials + (size_t)(blockIdx.z * gridDim.x + blockIdx.x) * 3 * pitch + (size_t)3 * d0;
+  for (int t = threadIdx.x; t < 3 * TILE; t += 32 * FF_WARPS) {
+    double2 v = red[t];
+#pragma unroll
+    for (int w = 1; w < FF_WARPS; ++w) v = cadd(v, red[w * 3 * TILE + t]);
+    out[t] = v;
   }
 }
 
-__global__ void k_ff_final(const double2* partials, int nblocks, int rows, double2* sums) {
+// sums[d][base + step*c] = the parts' partials in part order
+__global__ void k_ff_final(const double2* partials, int nparts, int rows, int part_stride, int ns, int base, int step,
+                           double2* sums) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   double2 s = make_double2(0, 0);
-  for (int b = 0; b < nblocks; ++b) {
-    const double2 v = partials[(size_t)r * nblocks + b];
-    s.x += v.x;
-    s.y += v.y;
-  }
-  sums[r] = s;
+  for (int b = 0; b < nparts; ++b) s = cadd(s, partials[(size_t)b * part_stride + r]);
+  const int d = r / 3, c = r - 3 * d;
+  sums[(size_t)d * ns + base + step * c] = s;
 }
 
 // Far-field sums of a compact polarisation p (device) over ndir directions,
-// phases and per-thread sums in TR, ND directions per block; NS sums per
-// direction (3: S, 12: S and the position moments U), sums_host[dir][NS].
-template <typename C, typename TR, int ND, int NS = 3>
-static int ff_sums_impl(const int* occ, int nx, int ny, int nz, int nat0, const C* p, const double* dirs_host, int ndir,
-                        const double dx[3], const double x0[3], double2* sums_host, cudaStream_t s) {
+// phases and row sums in TR; NS sums per direction (3: S, 12: S and the position
+// moments U_ab = sum_j P_ja r_jb exp(-i k.r_j), a-major), sums_host[dir][NS].
+template <typename C, typename TR, int NS = 3>
+static int ff_sums_impl(const int* inv, int nx, int ny, int nz, int nat0, const C* p,
+                        const double* dirs_host, int ndir, const double dx[3], const double x0[3], double2* sums_host,
+                        cudaStream_t s) {
   using TC = cplx<TR>;
-  if (nx > 2047 || ny > 2047 || nz > 1023) { set_error("GPU SCAT", "grid too large for packed coordinates"); return 322; }
-  const int chunk = 4096;  // directions per launch
-  const int sites_per_block = FF_THREADS * 32;
-  const int nblocks = (int)ceil_div(nat0, sites_per_block);
-  const int ntab = nx + ny + nz;
-  unsigned* coords = nullptr;
+  if (nx > 2047 || ny > 2047 || nz > 1023) { set_error("GPU SCAT", "grid too large for the far-field sums"); return 322; }
+  constexpr int TILE = FF_TILE;
+  const int chunk = std::min(4096, (int)ceil_div(std::max(ndir, 1), TILE) * TILE);  // directions per launch
+  const int nrows = ny * nz, npair = (nrows + 1) / 2, kch = (int)ceil_div(nx, FF_COLS), ntab = nx + ny + nz;
+  // row blocks: at least 4 waves of one block per SM where each warp still
+  // gets two row pairs (the ex tile is loaded once per block)
+  auto row_blocks = [&](int tiles) {
+    const size_t want = ceil_div((size_t)4 * 148, (size_t)tiles * kch);
+    return (int)std::max<size_t>(1, std::min<size_t>(want, ceil_div((size_t)npair, 2 * FF_WARPS)));
+  };
+  size_t npartial = 0;
+  for (int off = 0; off < ndir; off += chunk) {
+    const int tiles = (int)ceil_div(std::min(chunk, ndir - off), TILE);
+    npartial = std::max(npartial, (size_t)row_blocks(tiles) * kch * 3 * tiles * TILE);
+  }
   double* d_dirs = nullptr;
   TC* tab = nullptr;
-  double2 *partials = nullptr, *sums = nullptr;
+  double2 *yz = nullptr, *partials = nullptr, *sums = nullptr;
   int rc = 0;
-  cudaError_t e = dev_alloc((void**)&coords, (size_t)nat0 * sizeof(unsigned));
-  if (e == cudaSuccess) e = dev_alloc((void**)&d_dirs, (size_t)3 * chunk * sizeof(double));
-  if (e == cudaSuccess) e = dev_alloc((void**)&tab, (size_t)chunk * ntab * sizeof(TC));
-  if (e == cudaSuccess) e = dev_alloc((void**)&partials, (size_t)chunk * NS * nblocks * sizeof(double2));
+  cudaError_t e = dev_alloc((void**)&d_dirs, (size_t)3 * chunk * sizeof(double));
+  if (e == cudaSuccess) e = dev_alloc((void**)&tab, (size_t)chunk * nx * sizeof(TC));
+  if (e == cudaSuccess) e = dev_alloc((void**)&yz, (size_t)chunk * (ny + nz) * sizeof(double2));
+  if (e == cudaSuccess) e = dev_alloc((void**)&partials, npartial * sizeof(double2));
   if (e == cudaSuccess) e = dev_alloc((void**)&sums, (size_t)chunk * NS * sizeof(double2));
   if (e != cudaSuccess) { set_cuda_error("SCAT workspace", e); rc = 322; }
   if (!rc) {
-    k_pack_coords<<<(unsigned)ceil_div(nat0, 256), 256, 0, s>>>(occ, nat0, nx, ny, coords);
-    note_launch();
-    const size_t sm = (size_t)ND * ntab * sizeof(TC);
-    cudaFuncSetAttribute((const void*)k_ff_partial<C, TR, ND, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
+    raise_smem_limit((const void*)k_ff_rows<C, TR>);
     SitePos pos;
     for (int k = 0; k < 3; ++k) { pos.x0[k] = (float)x0[k]; pos.dx[k] = (float)dx[k]; }
     for (int off = 0; off < ndir && !rc; off += chunk) {
-      const int cnt = std::min(chunk, ndir - off);
+      const int cnt = std::min(chunk, ndir - off), tiles = (int)ceil_div(cnt, TILE), pitch = tiles * TILE;
+      const int nb = row_blocks(tiles);
       cudaMemcpyAsync(d_dirs, dirs_host + (size_t)3 * off, (size_t)3 * cnt * sizeof(double), cudaMemcpyHostToDevice, s);
-      k_ff_tables<TC><<<(unsigned)std::min<size_t>(ceil_div((size_t)cnt * ntab, 256), 4096), 256, 0, s>>>(
-          d_dirs, cnt, nx, ny, nz, dx[0], dx[1], dx[2], x0[0], x0[1], x0[2], tab);
+      k_ff_tables<TC><<<(unsigned)std::min<size_t>(ceil_div((size_t)pitch * ntab, 256), 4096), 256, 0, s>>>(
+          d_dirs, cnt, pitch, nx, ny, nz, dx[0], dx[1], dx[2], x0[0], x0[1], x0[2], tab, yz);
       note_launch();
-      dim3 grid((unsigned)nblocks, (unsigned)ceil_div(cnt, ND));
-      k_ff_partial<C, TR, ND, NS><<<grid, FF_THREADS, sm, s>>>(p, coords, nat0, cnt, nx, ny, nz, tab,
-                                                               sites_per_block, partials, pos);
-      note_launch();
-      k_ff_final<<<(unsigned)ceil_div((size_t)cnt * NS, 128), 128, 0, s>>>(partials, nblocks, cnt * NS, sums);
-      note_launch();
+      for (int wt = 0; wt <= (NS == 12 ? 3 : 0); ++wt) {
+        k_ff_rows<C, TR><<<dim3((unsigned)nb, (unsigned)tiles, (unsigned)kch), 32 * FF_WARPS, ff_smem<TR>(), s>>>(
+            p, inv, nat0, nrows, pitch, nx, ny, tab, yz, partials, wt, pos);
+        note_launch();
+        k_ff_final<<<(unsigned)ceil_div((size_t)cnt * 3, 128), 128, 0, s>>>(partials, nb * kch, cnt * 3, 3 * pitch, NS,
+                                                                            wt ? 2 + wt : 0, wt ? 3 : 1, sums);
+        note_launch();
+      }
       if (check_launch("SCAT far-field sums")) { rc = 325; break; }
       e = cudaMemcpyAsync(sums_host + (size_t)NS * off, sums, (size_t)NS * cnt * sizeof(double2), cudaMemcpyDeviceToHost,
                           s);
@@ -240,7 +375,7 @@ static int ff_sums_impl(const int* occ, int nx, int ny, int nz, int nat0, const 
     }
   }
   if (rc) cudaStreamSynchronize(s);
-  dev_free(coords); dev_free(d_dirs); dev_free(tab); dev_free(partials); dev_free(sums);
+  dev_free(d_dirs); dev_free(tab); dev_free(yz); dev_free(partials); dev_free(sums);
   return rc;
 }
 
@@ -250,16 +385,16 @@ int farfield_sums(Engine<T>& eng, const cplx<T>* p, const float* dirs_host, int 
   std::vector<double> hd((size_t)3 * std::max(ndir, 0));
   for (size_t i = 0; i < hd.size(); ++i) hd[i] = (double)dirs_host[i];
   const double dxd[3] = {dx[0], dx[1], dx[2]}, x0d[3] = {x0[0], x0[1], x0[2]};
-  return ff_sums_impl<cplx<T>, float, FF_DIRS>(eng.occ, eng.g.nx, eng.g.ny, eng.g.nz, eng.g.nat0, p, hd.data(), ndir,
-                                               dxd, x0d, sums_host, s);
+  return ff_sums_impl<cplx<T>, float>(eng.inv, eng.g.nx, eng.g.ny, eng.g.nz, eng.g.nat0, p, hd.data(), ndir,
+                                      dxd, x0d, sums_host, s);
 }
 
 template <typename T>
 int farfield_torque_sums(Engine<T>& eng, const cplx<T>* p, const double* dirs_host, int ndir, const float dx[3],
                          const float x0[3], double2* sums_host, cudaStream_t s) {
   const double dxd[3] = {dx[0], dx[1], dx[2]}, x0d[3] = {x0[0], x0[1], x0[2]};
-  return ff_sums_impl<cplx<T>, float, 2, 12>(eng.occ, eng.g.nx, eng.g.ny, eng.g.nz, eng.g.nat0, p, dirs_host, ndir, dxd,
-                                             x0d, sums_host, s);
+  return ff_sums_impl<cplx<T>, float, 12>(eng.inv, eng.g.nx, eng.g.ny, eng.g.nz, eng.g.nat0, p, dirs_host,
+                                          ndir, dxd, x0d, sums_host, s);
 }
 
 // Torque of the incident field E on the dipoles P (compact), per block:
@@ -344,9 +479,10 @@ template int farfield_torque_sums<float>(Engine<float>&, const float2*, const do
 template int incident_torque<float>(Engine<float>&, const float2*, const float2*, const float*, const float*,
                                     const double*, double*, cudaStream_t);
 
-int farfield_sums_f64(const int* occ, int nx, int ny, int nz, int nat0, const double2* p, const double* dirs_host,
-                      int ndir, const double dx[3], const double x0[3], double2* sums_host, cudaStream_t s) {
-  return ff_sums_impl<double2, double, 4>(occ, nx, ny, nz, nat0, p, dirs_host, ndir, dx, x0, sums_host, s);
+int farfield_sums_f64(const Engine<float>& eng, const double2* p, const double* dirs_host, int ndir,
+                      const double dx[3], const double x0[3], double2* sums_host, cudaStream_t s) {
+  return ff_sums_impl<double2, double>(eng.inv, eng.g.nx, eng.g.ny, eng.g.nz, eng.g.nat0, p, dirs_host, ndir,
+                                       dx, x0, sums_host, s);
 }
 
 // --------------------------------------------------------------------------
@@ -477,7 +613,5 @@ template int evalq_compute<double>(Engine<double>&, VecOps<double>&, const doubl
                                    const double2*, int, double2*, double, double2*, double2*);
 template int farfield_sums<float>(Engine<float>&, const float2*, const float*, int, const float[3], const float[3],
                                   double2*, cudaStream_t);
-template int farfield_sums<double>(Engine<double>&, const double2*, const float*, int, const float[3], const float[3],
-                                   double2*, cudaStream_t);
 
 }  // namespace ddb

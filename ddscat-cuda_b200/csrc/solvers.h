@@ -63,9 +63,9 @@ int incident_torque(Engine<T>& eng, const cplx<T>* p, const cplx<T>* e, const fl
                     const double k[3], double gamma[6], cudaStream_t s);
 
 // The same sums with FP64 phases and FP64 accumulation (all-FP64 amplitudes);
-// occ: compact -> site map of the grid, p: compact complex-double polarisation.
-int farfield_sums_f64(const int* occ, int nx, int ny, int nz, int nat0, const double2* p, const double* dirs_host,
-                      int ndir, const double dx[3], const double x0[3], double2* sums_host, cudaStream_t s);
+// p: compact complex-double polarisation of the engine's target.
+int farfield_sums_f64(const Engine<float>& eng, const double2* p, const double* dirs_host, int ndir,
+                      const double dx[3], const double x0[3], double2* sums_host, cudaStream_t s);
 
 // Amplitude and Mueller matrices per scattering direction from f_ml (host in / out).
 int mueller_compute(int ndir, const float* ak, const float2* e01, const float2* e02, const float* em2,
