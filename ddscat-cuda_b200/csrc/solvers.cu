@@ -6,12 +6,14 @@
 // scalars, FP64 inner products, the reliable-residual policy (true residual
 // every 20 iterations and on claimed convergence, restart when the recursion
 // gap >= 1e-3 or on false convergence, cu:543-556), the same MATVEC counting
-// and the same error codes.  Scalars are combined on the host from the
+// and the same error codes.  PBCGS2 and QMRCCG keep their scalars on the device;
+// those of the others are combined on the host from the
 // device-reduced inner products (one small D2H per product, no full-vector
 // transfers inside the loops).
 #include <chrono>
 #include <complex>
 #include "engine.h"
+#include "reduce.cuh"
 #include "solvers.h"
 
 namespace ddb {
@@ -132,11 +134,12 @@ template <typename T> struct Ctx {
 
 // QMRCCG with the FP64 recurrence scalars held on the GPU: one iteration is
 // the p/q step, A p, the vt/wt step, A wt, one launch of the four inner
-// products, the scalar recurrence in a single thread, the d/s/x/r step and
-// |r|^2; the host waits once per iteration, for the residual it prints and
-// tests (the reference waits for every inner-product group, cu:1079-1092).
-// Same recurrence, reliable-residual checks, restart rule and MATVEC count as
-// the reference (cu:434-443, cu:1071-1103).
+// products and the d/s/x/r step with |r|^2; the block that finishes a sum last
+// also does the scalar step that needs it.  The host waits once per iteration,
+// for the residual it prints and tests (the reference waits for every
+// inner-product group, cu:1079-1092).  Same recurrence, reliable-residual
+// checks, restart rule and MATVEC count as the reference (cu:434-443,
+// cu:1071-1103).
 struct DQState {
   double2 gamma, ksi, rho, eps, mu, tau, lambda, kappa, theta;
   // coefficients: p = co0 p + co1 vt, q = co2 q + co3 atw, vt = co4 vt + A p,
@@ -170,8 +173,7 @@ __host__ __device__ inline void dq_step_coefficients(DQState& S) {
 }
 
 // the scalar recurrence of cu:442 from |vt|^2, |wt|^2, vt^T wt, vt^T A wt
-__global__ void k_dq_recur(DQState* SP, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ inline void dq_recur(DQState* SP, const double2* out) {
   DQState S = *SP;
   const double2 gamma0 = S.gamma, ksi0 = S.ksi, rho0 = S.rho, tau0 = S.tau, kappa0 = S.kappa;
   S.gamma = make_double2(sqrt(fmax(0.0, out[0].x)), 0.0);
@@ -206,8 +208,7 @@ __global__ void k_dq_recur(DQState* SP, const double2* out) {
   if (!st) dq_step_coefficients(S);
   *SP = S;
 }
-__global__ void k_dq_resid(DQState* S, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ inline void dq_resid(DQState* S, const double2* out) {
   double v = out[0].x;
   if (v < 0.0 && v > -1e-12) v = 0.0;
   S->resid = sqrt(v > 0.0 ? v : 0.0) / S->bnorm;
@@ -235,30 +236,117 @@ __global__ void k_dq_vw(int n, C* vt, C* wt, const C* ap, const C* q, const DQSt
     wt[i] = dq_lin(wt[i], c5, q[i], one);
   }
 }
+// the four inner products of an iteration, then the scalar recurrence
 template <typename C>
-__global__ void k_dq_dsxr(int n, C* d, C* s, C* x, C* r, const C* p, const C* ap, const DQState* S) {
+__global__ void __launch_bounds__(RED_THREADS) k_dq_dots(int n, const C* vt, const C* wt, const C* atw, DQState* S,
+                                                         double2* part, double2* out, unsigned* cnt) {
+  double2 acc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] = make_double2(0.0, 0.0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double2 v = to_d(vt[i]), w = to_d(wt[i]), a = to_d(atw[i]);
+    acc[0].x += v.x * v.x + v.y * v.y;
+    acc[1].x += w.x * w.x + w.y * w.y;
+    acc[2].x += v.x * w.x - v.y * w.y;
+    acc[2].y += v.x * w.y + v.y * w.x;
+    acc[3].x += v.x * a.x - v.y * a.y;
+    acc[3].y += v.x * a.y + v.y * a.x;
+  }
+  reduce_tail<4>(acc, 4, part, out, cnt, [=](const double2* o) { dq_recur(S, o); });
+}
+// the d/s/x/r step with |r|^2 and the residual
+template <typename C>
+__global__ void __launch_bounds__(RED_THREADS) k_dq_dsxr(int n, C* d, C* s, C* x, C* r, const C* p, const C* ap,
+                                                         DQState* S, double2* part, double2* out, unsigned* cnt) {
   if (S->status) return;
   const double2 th = S->co[6], ka = S->co[7], one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0);
+  double2 acc[1] = {make_double2(0.0, 0.0)};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const C dn = dq_lin(d[i], th, p[i], ka);
     const C sn = dq_lin(s[i], th, ap[i], ka);
     d[i] = dn;
     s[i] = sn;
     x[i] = dq_lin(x[i], one, dn, one);
-    r[i] = dq_lin(r[i], one, sn, mone);
+    const C rn = dq_lin(r[i], one, sn, mone);
+    r[i] = rn;
+    const double2 e = to_d(rn);
+    acc[0].x += e.x * e.x + e.y * e.y;
   }
+  reduce_tail<1>(acc, 1, part, out, cnt, [=](const double2* o) { dq_resid(S, o); });
 }
+
+// blocks of a kernel with a sum: one resident wave, within the partials buffer
+template <typename T> static unsigned sum_grid(const VecOps<T>& o, int n, int per_sm) {
+  return (unsigned)std::min<size_t>(ceil_div((size_t)std::max(n, 1), RED_THREADS),
+                                    (size_t)std::min(o.nblocks, 148 * per_sm));
+}
+
+// The iterations of a solver as one CUDA graph.  An iteration is 14 to 30
+// launches, most of them shorter than the 3 us the host takes for a launch on
+// small grids (32^3: 175 us of kernels in 280 us per iteration).  The first
+// iteration runs launch by launch (one-time kernel set-up), the second is
+// captured and every later one is a single launch.  Not with per-MATVEC output
+// (its events are read between the MATVECs).  If the capture is not possible
+// the iterations keep running launch by launch.
+struct IterGraph {
+  cudaStream_t cap = nullptr;
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  unsigned long long kernels = 0;
+  int products = 0;
+  bool off = false;
+  ~IterGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    if (cap) cudaStreamDestroy(cap);
+  }
+  // Runs body (one iteration on io.stream / eng.stream / ops.stream), as a graph
+  // from its second call on; nc counts the iteration's products.
+  template <typename T, typename F> int run(SolveIO<T>& io, int& nc, int it, F body) {
+    if (off || io.verbose || it < 2) return body();
+    if (!exec && !capture(io, nc, body)) {
+      off = true;
+      cudaGetLastError();
+      clear_error();
+      return body();
+    }
+    nc += products;
+    note_launch(kernels);
+    const cudaError_t e = cudaGraphLaunch(exec, io.stream);
+    if (e != cudaSuccess) { set_cuda_error("iteration graph", e); return -1; }
+    return 0;
+  }
+  template <typename T, typename F> bool capture(SolveIO<T>& io, int& nc, F body) {
+    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) { cap = nullptr; return false; }
+    if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
+    const cudaStream_t st = io.stream, es = io.eng->stream, os = io.ops->stream;
+    const unsigned long long l0 = launch_total();
+    const int n0 = nc;
+    io.stream = io.eng->stream = io.ops->stream = cap;
+    const int rc = body();
+    io.stream = st; io.eng->stream = es; io.ops->stream = os;
+    kernels = launch_total() - l0;
+    products = nc - n0;
+    nc = n0;
+    note_launch(0ull - kernels);  // recorded, not run
+    const bool ended = cudaStreamEndCapture(cap, &graph) == cudaSuccess && graph;
+    return ended && rc == 0 && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+  }
+};
 
 static inline unsigned dq_grid(int n) { return (unsigned)std::min<size_t>(ceil_div((size_t)std::max(n, 1), 256), 148 * 16); }
 
 // ---------------------------------------------------------------- PBCGS2 (cu:459-480, cu:1168-1278)
 // ZBCG2 = BiCGStab(2) with the reference's reliable updates and restarts, its
-// FP64 scalars held on the GPU (DPState): the inner products land in device
-// memory, single-thread kernels form rho/beta, sigma/alpha, the residual norm
-// and the 3 x 3 minimal-residual step, and the vector updates read their
-// coefficients from the state.  The host waits once per iteration (for the
-// residual, the breakdown status and the reliable-update tests); the
-// reference waits for every inner product (cu:1190-1255).
+// FP64 scalars held on the GPU (DPState).  30 launches per iteration: the block
+// that finishes an inner product last forms rho/beta, sigma/alpha, the residual
+// norm or the 3 x 3 minimal-residual step, the vector updates read their
+// coefficients from the state, and the updates of X and r_0 carry |r_0|^2 (44
+// launches with single-thread scalar kernels and one kernel per update).  The
+// host waits once per iteration (for the residual, the breakdown status and the
+// reliable-update tests); the reference waits for every inner product
+// (cu:1190-1255).  32^3 sphere, PBCGS2 + EVALQ + SCAT through the drop-in entry
+// points: 4.54 -> 3.23 ms with the iterations as a graph (IterGraph).
 struct DPState {
   double2 alpha, omega, sigma, rho0, rho1, beta;
   double2 one, mone;
@@ -273,13 +361,11 @@ __host__ __device__ inline double2 dp_conj(double2 a) { return make_double2(a.x,
 __host__ __device__ inline double2 dp_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __host__ __device__ inline double2 dp_sc(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
 
-__global__ void k_dp_begin(DPState* S) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  S->rho0 = dq_neg(dq_mul(S->omega, S->rho0));
-}
-// rho1 = rr^H r_{k-1}, beta = alpha rho1 / rho0, rho0 = rho1
-__global__ void k_dp_rho(DPState* S, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || S->status) return;
+// start of an iteration (first): rho0 = -omega rho0; then rho1 = rr^H r_{k-1},
+// beta = alpha rho1 / rho0, rho0 = rho1
+__device__ inline void dp_rho(DPState* S, const double2* out, bool first) {
+  if (first) S->rho0 = dq_neg(dq_mul(S->omega, S->rho0));
+  if (S->status) return;
   S->rho1 = out[0];
   if (dq_zero(S->rho0)) { S->status = 95; return; }
   S->beta = dq_mul(S->alpha, dq_div(S->rho1, S->rho0));
@@ -287,16 +373,15 @@ __global__ void k_dp_rho(DPState* S, const double2* out) {
   S->co[0] = dq_neg(S->beta);
 }
 // sigma = rr^H u_k, alpha = rho1 / sigma
-__global__ void k_dp_sigma(DPState* S, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || S->status) return;
+__device__ inline void dp_sigma(DPState* S, const double2* out) {
+  if (S->status) return;
   S->sigma = out[0];
   if (dq_zero(S->sigma)) { S->status = 98; return; }
   S->alpha = dq_div(S->rho1, S->sigma);
   S->co[1] = S->alpha;
   S->co[2] = dq_neg(S->alpha);
 }
-__global__ void k_dp_rnrm(DPState* S, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || S->status) return;
+__device__ inline void dp_rnrm(DPState* S, const double2* out) {
   S->rnrm = sqrt(fmax(0.0, out[0].x));
   S->mxnrmx = fmax(S->mxnrmx, S->rnrm);
   S->mxnrmr = fmax(S->mxnrmr, S->rnrm);
@@ -304,8 +389,8 @@ __global__ void k_dp_rnrm(DPState* S, const double2* out) {
 // the convex polynomial of cu:471-472 from the Gram matrix r_i^H r_j (lower
 // triangle r0r0, r1r0, r1r1, r2r0, r2r1, r2r2 in out[0..5]) and the
 // reliable-update tests of cu:474
-__global__ void k_dp_gram(DPState* SP, const double2* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || SP->status) return;
+__device__ inline void dp_gram(DPState* SP, const double2* out) {
+  if (SP->status) return;
   DPState S = *SP;
   double2 Zm[3][3];
   Zm[0][0] = out[0]; Zm[1][0] = out[1]; Zm[1][1] = out[2];
@@ -347,20 +432,83 @@ __global__ void k_dp_gram(DPState* SP, const double2* out) {
   S.resid = S.rnrm0 > 0.0 ? S.rnrm / S.rnrm0 : 0.0;
   *SP = S;
 }
-// d = cd d + ca a + cb b with coefficients read from device memory (null:
-// term absent; a zero cd drops d), k_lincomb's arithmetic
+// rr^H v with the scalar step it feeds: step 0 rho of the first half, 1 rho of
+// the second, 2 sigma
 template <typename C>
-__global__ void k_dp_lin(int n, C* d, const double2* cd, const C* a, const double2* ca, const C* b,
-                         const double2* cb, const int* status) {
-  if (*status) return;
-  const double2 zd = cd ? *cd : make_double2(0.0, 0.0), za = ca ? *ca : make_double2(0.0, 0.0),
-                zb = cb ? *cb : make_double2(0.0, 0.0);
+__global__ void __launch_bounds__(RED_THREADS) k_dp_dot(int n, const C* rr, const C* v, int step, DPState* S,
+                                                        double2* part, double2* out, unsigned* cnt) {
+  double2 acc[1] = {make_double2(0.0, 0.0)};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    C v = mk<C>(0, 0);
-    if (!dq_zero(zd)) v = zmulv(zd, d[i]);
-    if (a) v = cadd(v, zmulv(za, a[i]));
-    if (b) v = cadd(v, zmulv(zb, b[i]));
-    d[i] = v;
+    const double2 a = to_d(rr[i]), b = to_d(v[i]);
+    acc[0].x += a.x * b.x + a.y * b.y;
+    acc[0].y += a.x * b.y - a.y * b.x;
+  }
+  reduce_tail<1>(acc, 1, part, out, cnt, [=](const double2* o) {
+    if (step == 2) dp_sigma(S, o);
+    else dp_rho(S, o, step == 0);
+  });
+}
+// u_j = r_j - beta u_j, j < K
+template <typename C, int K>
+__global__ void k_dp_u(int n, C* u0, const C* r0, C* u1, const C* r1, const DPState* S) {
+  if (S->status) return;
+  const double2 mb = S->co[0], one = make_double2(1.0, 0.0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    u0[i] = dq_lin(u0[i], mb, r0[i], one);
+    if (K > 1) u1[i] = dq_lin(u1[i], mb, r1[i], one);
+  }
+}
+// X += alpha u0, r_j -= alpha u_{j+1} (j < K), and |r_0|
+template <typename C, int K>
+__global__ void __launch_bounds__(RED_THREADS) k_dp_xr(int n, C* X, const C* u0, C* r0, const C* u1, C* r1,
+                                                       const C* u2, DPState* S, double2* part, double2* out,
+                                                       unsigned* cnt) {
+  if (S->status) return;
+  const double2 al = S->co[1], mal = S->co[2], one = make_double2(1.0, 0.0);
+  double2 acc[1] = {make_double2(0.0, 0.0)};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    X[i] = dq_lin(X[i], one, u0[i], al);
+    const C rn = dq_lin(r0[i], one, u1[i], mal);
+    r0[i] = rn;
+    if (K > 1) r1[i] = dq_lin(r1[i], one, u2[i], mal);
+    const double2 e = to_d(rn);
+    acc[0].x += e.x * e.x + e.y * e.y;
+  }
+  reduce_tail<1>(acc, 1, part, out, cnt, [=](const double2* o) { dp_rnrm(S, o); });
+}
+// the Hermitian Gram matrix r_i^H r_j, lower triangle (cu:1215-1220), and the
+// minimal-residual step
+template <typename C>
+__global__ void __launch_bounds__(RED_THREADS) k_dp_gram(int n, const C* r0, const C* r1, const C* r2, DPState* S,
+                                                         double2* part, double2* out, unsigned* cnt) {
+  double2 acc[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) acc[q] = make_double2(0.0, 0.0);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double2 v[3] = {to_d(r0[i]), to_d(r1[i]), to_d(r2[i])};
+    int q = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b <= a; ++b, ++q) {
+        acc[q].x += v[a].x * v[b].x + v[a].y * v[b].y;
+        acc[q].y += v[a].x * v[b].y - v[a].y * v[b].x;
+      }
+  }
+  reduce_tail<6>(acc, 6, part, out, cnt, [=](const double2* o) { dp_gram(S, o); });
+}
+// u0 -= Y1 u1 + Y2 u2 ; X += Y1 r0 + Y2 r1 ; r0 -= Y1 r1 + Y2 r2
+template <typename C>
+__global__ void k_dp_poly(int n, C* u0, const C* u1, const C* u2, C* X, C* r0, const C* r1, const C* r2,
+                          const DPState* S) {
+  if (S->status) return;
+  const double2 one = make_double2(1.0, 0.0);
+  auto lin3 = [&](C d, C a, double2 za, C b, double2 zb) { return cadd(cadd(zmulv(one, d), zmulv(za, a)), zmulv(zb, b)); };
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const C a0 = r0[i], a1 = r1[i];
+    u0[i] = lin3(u0[i], u1[i], S->my1, u2[i], S->my2);
+    X[i] = lin3(X[i], a0, S->y1, a1, S->y2);
+    r0[i] = lin3(a0, a1, S->my1, r2[i], S->my2);
   }
 }
 
@@ -407,61 +555,36 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
   if (upload()) return 93;
   double resid = S.resid;
   const int n = c.n;
-  const unsigned gb = dq_grid(n);
-  const int* dst = &dS->status;
-  auto lin = [&](C* d, const double2* cd, const C* a, const double2* ca, const C* b = nullptr,
-                 const double2* cb = nullptr) {
-    k_dp_lin<C><<<gb, 256, 0, c.st()>>>(n, d, cd, a, ca, b, cb, dst);
-    note_launch();
+  const VecOps<T>& vo = *io.ops;
+  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, 8), gr = sum_grid(vo, n, 6), gg = sum_grid(vo, n, 3);
+  auto dot = [&](const C* v, int step) {
+    k_dp_dot<C><<<gd, RED_THREADS, 0, c.st()>>>(n, rr, v, step, dS, vo.d_red, vo.d_out, vo.d_count);
   };
-  const double2 *one = &dS->one, *mbeta = &dS->co[0], *calpha = &dS->co[1], *cmalpha = &dS->co[2];
+  IterGraph ig;
   int it = 0;
   while (resid > io.tol && it < io.maxit) {
     ++it;
-    k_dp_begin<<<1, 32, 0, c.st()>>>(dS);
-    note_launch();
-    for (int k = 1; k <= 2; ++k) {
-      {
-        const C* A1[1] = {rr};
-        const C* B1[1] = {r[k - 1]};
-        const int cj[1] = {1};
-        if (io.ops->dots_dev(n, 1, A1, B1, cj)) return 94;
-      }
-      k_dp_rho<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-      note_launch();
-      for (int j = 0; j < k; ++j) lin(u[j], mbeta, r[j], one);  // u_j = r_j - beta u_j
-      MV(u[k - 1], u[k], 96);
-      {
-        const C* A1[1] = {rr};
-        const C* B1[1] = {u[k]};
-        const int cj[1] = {1};
-        if (io.ops->dots_dev(n, 1, A1, B1, cj)) return 97;
-      }
-      k_dp_sigma<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-      note_launch();
-      lin(X, one, u[0], calpha);                                                  // X += alpha u0
-      for (int j = 0; j < k; ++j) lin(r[j], one, u[j + 1], cmalpha);              // r_j -= alpha u_{j+1}
-      MV(r[k - 1], r[k], 99);
-      {
-        const C* A1[1] = {r[0]};
-        const int cj[1] = {1};
-        if (io.ops->dots_dev(n, 1, A1, A1, cj)) return 100;
-      }
-      k_dp_rnrm<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-      note_launch();
-    }
-    {  // Hermitian Gram matrix r_i^H r_j, lower triangle (cu:1215-1220)
-      const C* A6[6] = {r[0], r[1], r[1], r[2], r[2], r[2]};
-      const C* B6[6] = {r[0], r[0], r[1], r[0], r[1], r[2]};
-      const int cj[6] = {1, 1, 1, 1, 1, 1};
-      if (io.ops->dots_dev(n, 6, A6, B6, cj)) return 101;
-    }
-    k_dp_gram<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-    note_launch();
-    // u0 -= Y1 u1 + Y2 u2 ; X += Y1 r0 + Y2 r1 ; r0 -= Y1 r1 + Y2 r2
-    lin(u[0], one, u[1], &dS->my1, u[2], &dS->my2);
-    lin(X, one, r[0], &dS->y1, r[1], &dS->y2);
-    lin(r[0], one, r[1], &dS->my1, r[2], &dS->my2);
+    const int brc = ig.run(io, c.nc, it, [&]() -> int {
+      dot(r[0], 0);
+      k_dp_u<C, 1><<<gb, 256, 0, c.st()>>>(n, u[0], r[0], nullptr, nullptr, dS);
+      MV(u[0], u[1], 96);
+      dot(u[1], 2);
+      k_dp_xr<C, 1><<<gr, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], nullptr, nullptr, dS, vo.d_red, vo.d_out,
+                                                    vo.d_count);
+      MV(r[0], r[1], 99);
+      dot(r[1], 1);
+      k_dp_u<C, 2><<<gb, 256, 0, c.st()>>>(n, u[0], r[0], u[1], r[1], dS);
+      MV(u[1], u[2], 96);
+      dot(u[2], 2);
+      k_dp_xr<C, 2><<<gr, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], r[1], u[2], dS, vo.d_red, vo.d_out,
+                                                    vo.d_count);
+      MV(r[1], r[2], 99);
+      k_dp_gram<C><<<gg, RED_THREADS, 0, c.st()>>>(n, r[0], r[1], r[2], dS, vo.d_red, vo.d_out, vo.d_count);
+      k_dp_poly<C><<<gb, 256, 0, c.st()>>>(n, u[0], u[1], u[2], X, r[0], r[1], r[2], dS);
+      note_launch(10);
+      return 0;
+    });
+    if (brc) return brc < 0 ? 103 : brc;
     if (check_launch(name)) return 103;
     if (cudaMemcpyAsync(hS, dS, sizeof(DPState), cudaMemcpyDeviceToHost, c.st()) != cudaSuccess ||
         cudaEventRecord(ev, c.st()) != cudaSuccess || cudaEventSynchronize(ev) != cudaSuccess) {
@@ -594,33 +717,23 @@ template <typename T> int solve_qmrccg(SolveIO<T>& io) {
   double resid = c.nrm(r) / bnorm;
   CK(55);
   const int n = c.n;
-  const unsigned gb = dq_grid(n);
+  const VecOps<T>& vo = *io.ops;
+  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, 4), gr = sum_grid(vo, n, 6);
+  IterGraph ig;
   int it = 0;
   while (it < io.maxit && resid > io.tol) {
     ++it;
-    k_dq_pq<C><<<gb, 256, 0, c.st()>>>(n, p, q, vt, atw, dS);
-    note_launch();
-    MV(p, ap, 56);
-    k_dq_vw<C><<<gb, 256, 0, c.st()>>>(n, vt, wt, ap, q, dS);
-    note_launch();
-    MV(wt, atw, 57);
-    {
-      const C* A4[4] = {vt, wt, vt, vt};
-      const C* B4[4] = {vt, wt, wt, atw};
-      const int cj[4] = {1, 1, 0, 0};
-      if (io.ops->dots_dev(n, 4, A4, B4, cj)) return 57;
-    }
-    k_dq_recur<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-    note_launch();
-    k_dq_dsxr<C><<<gb, 256, 0, c.st()>>>(n, d, s, xs, r, p, ap, dS);
-    note_launch();
-    {
-      const C* A1[1] = {r};
-      const int cj[1] = {1};
-      if (io.ops->dots_dev(n, 1, A1, A1, cj)) return 59;
-    }
-    k_dq_resid<<<1, 32, 0, c.st()>>>(dS, io.ops->d_out);
-    note_launch();
+    const int brc = ig.run(io, c.nc, it, [&]() -> int {
+      k_dq_pq<C><<<gb, 256, 0, c.st()>>>(n, p, q, vt, atw, dS);
+      MV(p, ap, 56);
+      k_dq_vw<C><<<gb, 256, 0, c.st()>>>(n, vt, wt, ap, q, dS);
+      MV(wt, atw, 57);
+      k_dq_dots<C><<<gd, RED_THREADS, 0, c.st()>>>(n, vt, wt, atw, dS, vo.d_red, vo.d_out, vo.d_count);
+      k_dq_dsxr<C><<<gr, RED_THREADS, 0, c.st()>>>(n, d, s, xs, r, p, ap, dS, vo.d_red, vo.d_out, vo.d_count);
+      note_launch(4);
+      return 0;
+    });
+    if (brc) return brc < 0 ? 59 : brc;
     if (check_launch(name)) return 59;
     if (cudaMemcpyAsync(hS, dS, sizeof(DQState), cudaMemcpyDeviceToHost, c.st()) != cudaSuccess ||
         cudaEventRecord(ev, c.st()) != cudaSuccess || cudaEventSynchronize(ev) != cudaSuccess) {

@@ -9,11 +9,9 @@
 // round trip is needed to combine chunks.
 #include <algorithm>
 #include "engine.h"
+#include "reduce.cuh"
 
 namespace ddb {
-
-constexpr int RED_THREADS = 256;
-constexpr int RED_MAXK = 8;
 
 template <typename T> struct DotSpec {
   const cplx<T>* a[RED_MAXK];
@@ -24,21 +22,10 @@ template <typename T> struct DotSpec {
   int k;
 };
 
-__device__ __forceinline__ double2 warp_sum(double2 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
-
 // KM: the largest product count of the launch (registers scale with it)
 template <typename T, int KM>
 __global__ void __launch_bounds__(RED_THREADS) k_dots(int n, DotSpec<T> sp, double2* partials, double2* out,
                                                       unsigned* count) {
-  __shared__ double2 wsum[RED_MAXK][RED_THREADS / 32];
-  __shared__ bool last;
   double2 acc[KM];
 #pragma unroll
   for (int q = 0; q < KM; ++q) acc[q] = make_double2(0.0, 0.0);
@@ -88,45 +75,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_dots(int n, DotSpec<T> sp, doub
       term(q, sp.a[q][i], sp.b[q][i], sp.c[q], i);
     }
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < KM; ++q) {  // compile-time indices: acc stays in registers
-    if (q >= sp.k) break;
-    double2 v = warp_sum(acc[q]);
-    if (lane == 0) wsum[q][wid] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    for (int q = 0; q < sp.k; ++q) {
-      double2 v = (lane < RED_THREADS / 32) ? wsum[q][lane] : make_double2(0.0, 0.0);
-      v = warp_sum(v);
-      if (lane == 0) partials[(size_t)q * gridDim.x + blockIdx.x] = v;
-    }
-  }
-  __threadfence();
-  if (threadIdx.x == 0) last = (atomicInc(count, gridDim.x - 1) == gridDim.x - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // the last block sums the partials in block order (deterministic)
-  for (int q = 0; q < sp.k; ++q) {
-    double2 v = make_double2(0.0, 0.0);
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-      const volatile double* pp = reinterpret_cast<volatile double*>(partials + (size_t)q * gridDim.x + b);
-      v.x += pp[0];
-      v.y += pp[1];
-    }
-    v = warp_sum(v);
-    if (lane == 0) wsum[q][wid] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    for (int q = 0; q < sp.k; ++q) {
-      double2 v = (lane < RED_THREADS / 32) ? wsum[q][lane] : make_double2(0.0, 0.0);
-      v = warp_sum(v);
-      if (lane == 0) out[q] = v;
-    }
-  }
+  reduce_tail<KM>(acc, sp.k, partials, out, count, NoPost{});
 }
 
 template <typename T> int VecOps<T>::init(cudaStream_t s) {

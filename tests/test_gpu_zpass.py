@@ -23,7 +23,7 @@ def test_zpass_with_staged_rows_solves(monkeypatch, dims, least):
     R = 5
     b = ((rng.normal(size=(R, 3 * nat)) + 1j * rng.normal(size=(R, 3 * nat))) * np.tile(iocc, 3)).astype(np.complex64)
     # different diagonals: the RHS converge, and are masked, at different iterations
-    adia = np.stack([np.full(3 * nat, (8.0 + 6 * r) - 2.0j) for r in range(R)]).astype(np.complex64)
+    adia = np.stack([np.full(3 * nat, (14.0 + 8 * r) - 3.0j) for r in range(R)]).astype(np.complex64)
     dda = D.DDA()
     dda.prepare_green(*dims, iocc, (0.3, 0.0, 0.0))
     x = np.zeros_like(b)
