@@ -1379,12 +1379,14 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_adjoint_f32(int nrhs, const void* p, 
   }
   cudaError_t e = cudaMemsetAsync(bs.x, 0, (size_t)nrhs * bs.n * sizeof(C), s.stream);
   if (e != cudaSuccess) { set_cuda_error("adjoint", e); return 533; }
-  // adjoint solve A lam = s: one-MATVEC QMRCCG with residual replacement
+  // adjoint solve A lam = s: one-MATVEC QMRCCG with residual replacement,
+  // device-driven (48^3, 3 RHS: 5.58 -> 5.19 ms; the host-driven form makes 231
+  // launches and waits 59 times)
   BatchIO<float> io;
   io.eng = &s.eng; io.ops = &bs.ops; io.R = nrhs; io.n = bs.n;
   io.b = bs.b; io.x = bs.x; io.adia = bs.adia; io.aoff = nullptr;
   io.work = bs.work; io.nwork = BATCH_WORK_VECTORS - 2;
-  io.maxit = maxit; io.tol = (double)tol; io.verbose = verbose_level() >= 2; io.replace = 1; io.sym = 1;
+  io.maxit = maxit; io.tol = (double)tol; io.verbose = verbose_level() >= 2; io.replace = 1; io.sym = 1; io.graph = 1;
   BatchResult res;
   int rc = solve_batch_qmrccg<float>(io, res);
   if (!rc) rc = matvec_check(s.eng);
@@ -1484,7 +1486,7 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_adjoint_fwd_f32(int nsrc, const void*
   io.eng = &s.eng; io.ops = &bs.ops; io.R = R; io.n = bs.n;
   io.b = bs.b; io.x = bs.x; io.adia = bs.adia; io.aoff = nullptr;
   io.work = bs.work; io.nwork = BATCH_WORK_VECTORS;
-  io.maxit = maxit; io.tol = (double)tol; io.verbose = verbose_level() >= 2; io.replace = 1; io.sym = 1;
+  io.maxit = maxit; io.tol = (double)tol; io.verbose = verbose_level() >= 2; io.replace = 1; io.sym = 1; io.graph = 1;
   BatchResult res;
   int rc = solve_batch_qmrccg<float>(io, res);
   if (!rc) rc = matvec_check(s.eng);
