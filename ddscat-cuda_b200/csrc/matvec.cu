@@ -577,6 +577,70 @@ template <typename T> static cplx<T>* upload_twiddles(int n, size_t& bytes) {
   return d;
 }
 
+// ---------------------------------------------------------------- index maps
+// compact index q = rank of an occupied site in site order; rowq[r] = occupied
+// sites before x row r (the sites of consecutive rows occupy one contiguous
+// compact range).  One warp per row; bound by the H2D copy of IOCC.  Host loops
+// over the sites took 1.4 ms of a prepare at 96x80x96 (prepare + MATVEC 7.49 ->
+// 6.12 ms).
+__global__ void k_row_counts(const int16_t* iocc, int nx, int nrows, int* rowq) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps) {
+    int c = 0;
+    for (int x0 = 0; x0 < nx; x0 += 32)
+      c += __popc(__ballot_sync(0xffffffffu, x0 + lane < nx && iocc[(size_t)r * nx + x0 + lane] != 0));
+    if (lane == 0) rowq[r + 1] = c;
+  }
+}
+// rowq[0..nrows] = prefix sums of the counts in rowq[1..nrows] (one block of 1024)
+__global__ void __launch_bounds__(1024) k_row_scan(int* rowq, int nrows) {
+  __shared__ int wsum[32];
+  __shared__ int base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) { base = 0; rowq[0] = 0; }
+  __syncthreads();
+  for (int r0 = 0; r0 < nrows; r0 += 1024) {
+    const int r = r0 + threadIdx.x;
+    int v = r < nrows ? rowq[r + 1] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) wsum[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+      int w = wsum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
+      }
+      wsum[lane] = w;
+    }
+    __syncthreads();
+    if (r < nrows) rowq[r + 1] = base + (wid ? wsum[wid - 1] : 0) + v;
+    __syncthreads();
+    if (threadIdx.x == 0) base += wsum[31];
+    __syncthreads();
+  }
+}
+__global__ void k_row_maps(const int16_t* iocc, int nx, int nrows, const int* rowq, int* occ, int* inv) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += warps) {
+    int q = rowq[r];
+    for (int x0 = 0; x0 < nx; x0 += 32) {
+      const int ix = x0 + lane, j = r * nx + ix;
+      const bool o = ix < nx && iocc[(size_t)r * nx + ix] != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, o);
+      const int p = q + __popc(m & ((1u << lane) - 1u));
+      if (ix < nx) inv[j] = o ? p : -1;
+      if (o) occ[p] = j;
+      q += __popc(m);
+    }
+  }
+}
+
 // Largest ratio of padded to 2n grid points at which the register pipeline is
 // the faster one.  The generic passes cost 0.10-0.13 ns per point when 2n has
 // the factors 2, 3, 5 only and 0.27 ns and more with larger ones (their
@@ -631,25 +695,8 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   twy = upload_twiddles<T>(g.My, bytes_allocated);
   twz = upload_twiddles<T>(g.Mz, bytes_allocated);
   if (!twx || !twy || !twz) { set_error("prepare", "twiddle allocation failed"); return 1; }
-  std::vector<int> occ_h, inv_h((size_t)nat, -1);
-  occ_h.reserve(nat0);
-  for (int j = 0; j < nat; ++j)
-    if (iocc_host[j] != 0) { inv_h[j] = (int)occ_h.size(); occ_h.push_back(j); }
-  if ((int)occ_h.size() != nat0) {
-    char msg[160];
-    std::snprintf(msg, sizeof(msg), "IOCC contains %zu occupied sites but NAT0=%d", occ_h.size(), nat0);
-    set_error("occupied-index map", msg);
-    return 2;
-  }
-  // compact index of the first occupied site of every x row: the sites of
-  // consecutive rows occupy one contiguous compact range
+  // index maps, built on the device from IOCC
   const int nrows = nat / nx;
-  std::vector<int> rowq_h((size_t)nrows + 1, 0);
-  for (int r = 0; r < nrows; ++r) {
-    int c = 0;
-    for (int ix = 0; ix < nx; ++ix) c += iocc_host[(size_t)r * nx + ix] != 0;
-    rowq_h[r + 1] = rowq_h[r] + c;
-  }
   cudaError_t e;
   e = dev_alloc((void**)&occ, (size_t)nat0 * sizeof(int));
   if (e == cudaSuccess) e = dev_alloc((void**)&inv, (size_t)nat * sizeof(int));
@@ -657,11 +704,24 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   if (e == cudaSuccess) e = dev_alloc((void**)&rowq, ((size_t)nrows + 1) * sizeof(int));
   if (e != cudaSuccess) { set_cuda_error("prepare: index maps", e); return 3; }
   bytes_allocated += (size_t)nat0 * 4 + (size_t)nat * 6 + ((size_t)nrows + 1) * 4;
-  cudaMemcpy(occ, occ_h.data(), (size_t)nat0 * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(inv, inv_h.data(), (size_t)nat * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(rowq, rowq_h.data(), ((size_t)nrows + 1) * sizeof(int), cudaMemcpyHostToDevice);
   e = cudaMemcpy(iocc, iocc_host, (size_t)nat * sizeof(int16_t), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) { set_cuda_error("prepare: index map H2D", e); return 3; }
+  const unsigned rb = (unsigned)std::min<size_t>(ceil_div((size_t)nrows, 8), 148 * 16);
+  k_row_counts<<<rb, 256>>>(iocc, nx, nrows, rowq);
+  k_row_scan<<<1, 1024>>>(rowq, nrows);
+  note_launch(2);
+  int occupied = 0;
+  e = cudaMemcpy(&occupied, rowq + nrows, sizeof(int), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) { set_cuda_error("prepare: index maps", e); return 3; }
+  if (occupied != nat0) {
+    char msg[160];
+    std::snprintf(msg, sizeof(msg), "IOCC contains %d occupied sites but NAT0=%d", occupied, nat0);
+    set_error("occupied-index map", msg);
+    return 2;
+  }
+  k_row_maps<<<rb, 256>>>(iocc, nx, nrows, rowq, occ, inv);
+  note_launch();
+  if (check_launch("prepare: index maps")) return 3;
   e = dev_alloc((void**)&green, g.green_count() * sizeof(C));
   if (e != cudaSuccess) { set_cuda_error("malloc resident Green", e); return 4; }
   bytes_allocated += g.green_count() * sizeof(C);
