@@ -126,6 +126,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // at most N of this thread's committed groups still in flight
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Programmatic dependent launch: pdl_launch lets the next kernel of the stream
+// start its blocks once every block of this one has called it or ended;
+// pdl_wait returns when the kernels before this one have ended and their writes
+// are visible.  Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Wait for the phase of parity `par` to complete, at most `limit` polls;
 // returns false if it did not complete in that time.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t par, int limit) {

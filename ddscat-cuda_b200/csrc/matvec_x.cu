@@ -231,6 +231,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
   C* lines = reinterpret_cast<C*>(smem_raw);  // RL * lsx
   const int iy0 = blockIdx.x * RL, iy = iy0 + l, iz = blockIdx.y;
   const int rl = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const int S = P.io_full ? P.nat : P.nat0;
   const C* x = P.x + (size_t)rl * P.x_rs + (size_t)c * S;
@@ -294,6 +296,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
   C* lines = reinterpret_cast<C*>(smem_raw);
   const int iz0 = blockIdx.x * RL, iz = iz0 + l, kxl = blockIdx.y, kx = P.kx0 + kxl;
   const int rb = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3), rl = P.b_rhs0 + rb;
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx + kx) * P.lda;
   C v[E];
@@ -419,6 +423,8 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   C* lines = reinterpret_cast<C*>(smem_raw);  // [3][RL][lsz]
   C* my = lines + (size_t)(c * RL + l) * P.lsz;
   const int rb = blockIdx.x, rl = P.b_rhs0 + rb;
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.y * RL + l;
@@ -548,6 +554,8 @@ template <typename T, int N, int BTY = 0> __global__ void __launch_bounds__(128,
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* my = reinterpret_cast<C*>(smem_raw) + (size_t)l * P.lsz;
   const int rb = blockIdx.x, rl = P.b_rhs0 + rb;
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.y * Z3Shape<N>::RZ + l;
@@ -684,6 +692,8 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
     }
     cp_async_commit();
   };
+  pdl_launch();
+  pdl_wait();
   int rb = next_rb((int)blockIdx.y * P.zg_rch);
   if (rb >= rb1) return;  // every RHS of the chunk masked
   fetch(rb, 0);
@@ -755,6 +765,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
   C* lines = reinterpret_cast<C*>(smem_raw);
   const int iz0 = blockIdx.x * RL, iz = iz0 + l, kxl = blockIdx.y, kx = P.kx0 + kxl;
   const int rb = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3), rl = P.b_rhs0 + rb;
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const int nz = P.nz;
   C v[E];
@@ -867,6 +879,8 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
   C* as = xs + MAXC;
   const int iy0 = blockIdx.x * RL, iy = iy0 + l, iz = blockIdx.y;
   const int rl = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
+  pdl_launch();
+  pdl_wait();
   if (xoff(P, rl)) return;
   const int ny = P.ny;
   const int S = P.io_full ? P.nat : P.nat0;
@@ -1247,11 +1261,21 @@ static size_t xy_smem(int nxl, int nyl, int lsx, int lsy) {
   return ((size_t)PLANE + std::max((size_t)(256 / TX) * lsx, (size_t)(256 / TY) * lsy)) * sizeof(float2);
 }
 
-template <typename T> static int xlaunch(const void* f, dim3 g, int th, size_t sm, cudaStream_t st, XParams<T>& P) {
+template <typename T> static int xlaunch(const void* f, dim3 g, int th, size_t sm, cudaStream_t st, XParams<T>& P, bool pdl = false) {
   raise_smem_limit(f);
   void* args[] = {(void*)&P};
   note_launch();
-  cudaError_t e = cudaLaunchKernel(f, g, dim3(th), args, sm, st);
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = g;
+  lc.blockDim = dim3(th);
+  lc.dynamicSmemBytes = sm;
+  lc.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at;
+  lc.numAttrs = pdl ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelExC(&lc, f, args);
   if (e != cudaSuccess) { set_cuda_error("MATVEC launch", e); return 1; }
   return 0;
 }
@@ -1417,6 +1441,13 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
     }
     return 0;
   }
+  // Programmatic dependent launches where the passes are so short that starting
+  // one counts: up to PDL_ELEMS elements of A.  16^3, one RHS: 22.7 -> 17.0 us
+  // per MATVEC, 64^3 64.4 -> 63.1; above, blocks that wait for the pass before
+  // them cost a little (51x75x39 with 12 RHS 53.9 -> 54.4 ms per solve, 128^3
+  // with 8 RHS 258.5 -> 260.5 ms).
+  constexpr size_t PDL_ELEMS = (size_t)4 << 20;
+  const bool pdl = (size_t)a.nrhs * P.A_rs <= PDL_ELEMS;
   for (int r0 = 0; r0 < a.nrhs; r0 += E.zcap) {
     const int nr = std::min(E.zcap, a.nrhs - r0);
     P.rhs0 = r0;
@@ -1424,7 +1455,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
     P.y = a.y + (size_t)r0 * a.y_rs;
     P.adia = a.adia + (size_t)r0 * a.a_rs;
     P.aoff = a.aoff ? a.aoff + (size_t)r0 * a.a_rs : nullptr;
-    if (xlaunch<T>(fxf, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smx, E.stream, P))
+    if (xlaunch<T>(fxf, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smx, E.stream, P, pdl))
       return 21;
     for (int rb0 = 0; rb0 < nr; rb0 += E.slab_nr) {
       const int nrb = std::min(E.slab_nr, nr - rb0);
@@ -1434,7 +1465,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
         P.kx0 = kx0;
         P.nkx = std::min(E.slab_B, g.Mx - kx0);
         if (xlaunch<T>(fyf, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy,
-                       E.stream, P))
+                       E.stream, P, pdl))
           return 22;
         // ZG3R: RHS chunks so that the grid has at least 4 waves of 3 blocks per SM
         const size_t nlb = ceil_div((size_t)P.nkx * g.My, RZ3);
@@ -1442,18 +1473,18 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
         P.zg_rch = (int)ceil_div((size_t)nrb, (size_t)nchunk);
         const bool use_r = fzg3r && P.zg_rch >= E.zg3r_min;
         if (use_r ? xlaunch<T>(fzg3r, dim3((unsigned)nlb, (unsigned)ceil_div((size_t)nrb, (size_t)P.zg_rch)), 128, smzr,
-                               E.stream, P)
+                               E.stream, P, pdl)
             : fzg3 ? xlaunch<T>(fzg3, dim3((unsigned)nrb, (unsigned)ceil_div((size_t)P.nkx * g.My, RZ3)), 128, smz,
-                              E.stream, P)
+                              E.stream, P, pdl)
                  : xlaunch<T>(fzg, dim3((unsigned)nrb, (unsigned)ceil_div((size_t)P.nkx * g.My, RZ)), 3 * TZ * RZ,
-                              smz, E.stream, P))
+                              smz, E.stream, P, pdl))
           return 23;
         if (xlaunch<T>(fyi, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy,
-                       E.stream, P))
+                       E.stream, P, pdl))
           return 24;
       }
     }
-    if (xlaunch<T>(fxi, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smxi, E.stream, P))
+    if (xlaunch<T>(fxi, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smxi, E.stream, P, pdl))
       return 25;
   }
   return 0;
