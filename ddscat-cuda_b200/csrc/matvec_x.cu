@@ -143,25 +143,41 @@ __device__ __forceinline__ void tma_load_tile(const CUtensorMap* map, float2* ti
         : "memory");
 }
 
+// Row stride (elements of C) of a transpose tile of N rows x RL columns.  The
+// threads of a line read and write rows t, t+1, ... of their column l, so the
+// lanes of one shared-memory wavefront (16 of 8 bytes, 8 of 16 bytes) hold
+// lanes/TT columns: a stride of RL plus that many elements puts them in
+// different banks.  (RL + 1, right for TT = 16, cost 4-way conflicts at TT = 4
+// and 2-way at TT = 8: the 96-point y pass ran its shared memory at 93 % and DRAM
+// at 37 %.)  Per MATVEC with the wider rows:
+// 45x37x31 47.3 -> 40.3 us, 64^3 67.4 -> 63.2; batched solves 64x56x48 116.5 ->
+// 112.2 ms, 48^3 4.81 -> 4.51.
+constexpr int tile_stride(int RL, int TT, int bytes) {
+  const int lanes = bytes == 8 ? 16 : 8;
+  return RL + (lanes / TT > 1 ? lanes / TT : 1);
+}
+
 // Tile <-> global moves of the row passes: N rows of RL consecutive elements
-// (row stride ld in global, RL+1 in the tile), two elements per 16-byte access.
+// (row stride ld in global, TS in the tile), two elements per 16-byte access.
 // Rows hold `valid` elements (RL or fewer at the grid edge; always even:
 // rows are stored with an even length, an odd n followed by one element that
 // no pass uses, and RL is even).  The global base and ld are even in
-// elements, so every pair is 16-byte aligned.
-template <int RL, int N, typename C>
+// elements, so every pair is 16-byte aligned; so are the tile's where TS is even.
+template <int RL, int N, int TS, typename C>
 __device__ __forceinline__ void store_pairs(C* g, int ld, int valid, const C* tile) {
   constexpr int RP = RL / 2;
 #pragma unroll 4
   for (int u = threadIdx.x; u < N * RP; u += 256) {
     const int r = u / RP, ll = 2 * (u % RP);
     if (ll < valid) {
-      const C a = tile[r * (RL + 1) + ll], b = tile[r * (RL + 1) + ll + 1];
-      if constexpr (sizeof(C) == 8) {
+      if constexpr (sizeof(C) == 8 && TS % 2 == 0) {
+        *reinterpret_cast<float4*>(g + (size_t)r * ld + ll) = *reinterpret_cast<const float4*>(tile + r * TS + ll);
+      } else if constexpr (sizeof(C) == 8) {
+        const C a = tile[r * TS + ll], b = tile[r * TS + ll + 1];
         *reinterpret_cast<float4*>(g + (size_t)r * ld + ll) = make_float4(a.x, a.y, b.x, b.y);
       } else {
-        g[(size_t)r * ld + ll] = a;
-        g[(size_t)r * ld + ll + 1] = b;
+        g[(size_t)r * ld + ll] = tile[r * TS + ll];
+        g[(size_t)r * ld + ll + 1] = tile[r * TS + ll + 1];
       }
     }
   }
@@ -172,7 +188,7 @@ __device__ __forceinline__ void store_pairs(C* g, int ld, int valid, const C* ti
 // instructions than 8-byte cp.async copies).  Rows hold `valid` elements, an
 // even count, and the global base and ld are even in elements, so every
 // complex-float pair is 16-byte aligned.
-template <int RL, int N, typename C>
+template <int RL, int N, int TS, typename C>
 __device__ __forceinline__ void load_tile_pairs(const C* g, int ld, int valid, C* tile) {
   static_assert((N * RL / 2) % 256 == 0, "tiles of whole 256-thread rounds");
   if constexpr (sizeof(C) == 8) {
@@ -187,8 +203,12 @@ __device__ __forceinline__ void load_tile_pairs(const C* g, int ld, int valid, C
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int u = threadIdx.x + 256 * k, r = u / RP, ll = 2 * (u - r * RP);
-      tile[r * (RL + 1) + ll] = mk<C>(q[k].x, q[k].y);
-      tile[r * (RL + 1) + ll + 1] = mk<C>(q[k].z, q[k].w);
+      if constexpr (TS % 2 == 0) {
+        *reinterpret_cast<float4*>(tile + r * TS + ll) = q[k];
+      } else {
+        tile[r * TS + ll] = mk<C>(q[k].x, q[k].y);
+        tile[r * TS + ll + 1] = mk<C>(q[k].z, q[k].w);
+      }
     }
   } else {  // complex double: one 16-byte element per load
     constexpr int K = N * RL / 256;
@@ -201,7 +221,7 @@ __device__ __forceinline__ void load_tile_pairs(const C* g, int ld, int valid, C
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int u = threadIdx.x + 256 * k, r = u / RL, ll = u - r * RL;
-      tile[r * (RL + 1) + ll] = q[k];
+      tile[r * TS + ll] = q[k];
     }
   }
 }
@@ -224,10 +244,10 @@ template <int MAXC, typename C> __device__ __forceinline__ void stage_chunk_asyn
 template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
-  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL;
+  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
-  C* tile = reinterpret_cast<C*>(smem_raw);   // [kx][RL+1], aliases the line scratch
+  C* tile = reinterpret_cast<C*>(smem_raw);   // [kx][TS], aliases the line scratch
   C* lines = reinterpret_cast<C*>(smem_raw);  // RL * lsx
   const int iy0 = blockIdx.x * RL, iy = iy0 + l, iz = blockIdx.y;
   const int rl = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
@@ -278,10 +298,10 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
     }
   }
 #pragma unroll
-  for (int i = 0; i < E; ++i) tile[(t + TT * i) * (RL + 1) + l] = v[i];
+  for (int i = 0; i < E; ++i) tile[(t + TT * i) * TS + l] = v[i];
   __syncthreads();
   C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * P.lda + iy0;
-  store_pairs<RL, N>(A, P.lda, P.lda - iy0, tile);
+  store_pairs<RL, N, TS>(A, P.lda, P.lda - iy0, tile);
 }
 
 // ------------------------------------------------------------- YF: y forward
@@ -289,7 +309,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
 template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
-  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL;
+  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
@@ -320,10 +340,10 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
     }
   }
 #pragma unroll
-  for (int i = 0; i < E; ++i) tile[(t + TT * i) * (RL + 1) + l] = v[i];
+  for (int i = 0; i < E; ++i) tile[(t + TT * i) * TS + l] = v[i];
   __syncthreads();
   C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * P.ldb + iz0;
-  store_pairs<RL, N>(B, P.ldb, P.ldb - iz0, tile);
+  store_pairs<RL, N, TS>(B, P.ldb, P.ldb - iz0, tile);
 }
 
 // Green record at (kx, ky, kz) for the z-fastest layout, without the kz sign.
@@ -758,7 +778,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
 template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
-  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL;
+  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
@@ -798,10 +818,10 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
   }
   if (!loaded) {
     const C* B = P.B + ((size_t)(rb * 3 + c) * P.nkx + kxl) * (size_t)P.My * P.ldb + iz0;
-    load_tile_pairs<RL, N>(B, P.ldb, P.ldb - iz0, tile);
+    load_tile_pairs<RL, N, TS>(B, P.ldb, P.ldb - iz0, tile);
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * (RL + 1) + l];
+    for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();  // the tile is consumed before the line scratch reuses it
   }
   line_fft<E, TT, -1, false, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy);
@@ -868,7 +888,7 @@ constexpr int XI_STAGE_MAX = 2048;  // largest staged chunk of the XI pass (elem
 template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
-  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL;
+  constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   constexpr int MAXC = RL * (N / 2);
   constexpr bool STAGE = MAXC <= XI_STAGE_MAX;  // larger rows keep direct loads (shared memory)
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -941,11 +961,11 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
   }
   if (!loaded) {
     const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx) * P.lda + iy0;
-    load_tile_pairs<RL, N>(A, P.lda, P.lda - iy0, tile);
+    load_tile_pairs<RL, N, TS>(A, P.lda, P.lda - iy0, tile);
     cp_async_wait_all();  // the x and CXADIA chunks
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * (RL + 1) + l];
+    for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();
   }
   line_fft<E, TT, -1, false, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx);
@@ -1367,7 +1387,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   P.lsz = fzg3 ? line_stride(g.Mz / TZ, TZ, RZ3, false, TZ >= 8)
                : std::max(line_stride(g.Mz / TZ, TZ, RZ, false, TZ >= 8), g.Mz);
   // the transpose tile and the line scratch share one region
-  P.tlx = (int)std::max((size_t)g.Mx * (RX + 1), (size_t)RX * P.lsx);
+  P.tlx = (int)std::max((size_t)g.Mx * tile_stride(RX, TX, sizeof(C)), (size_t)RX * P.lsx);
   // a tensor tile of the x passes (32 KB at a 1024-byte boundary) fits in front of the XI chunks
   if (g.Mx == 256 || g.Mx == 512)
     P.tlx = std::max(P.tlx, (int)(((size_t)(g.Mx / TMA_ROWS) * TMA_TILE_BYTES + 1024) / sizeof(C)));
@@ -1376,7 +1396,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   // out (MAXC = RL * N/2 elements, which is RX * nx only when Mx = 2 nx)
   const size_t xi_maxc = (size_t)RX * (g.Mx / 2);
   const size_t smxi = smx + (xi_maxc <= (size_t)XI_STAGE_MAX ? 2 * xi_maxc * sizeof(C) : 0);
-  size_t smy = std::max((size_t)g.My * (RY + 1), (size_t)RY * P.lsy) * sizeof(C);
+  size_t smy = std::max((size_t)g.My * tile_stride(RY, TY, sizeof(C)), (size_t)RY * P.lsy) * sizeof(C);
   // tensor tiles for the 256-point y passes (FP32, five-pass B layout): the
   // slab as rows of n_z; the tile needs 32 KB at a 1024-byte boundary
   P.tma = 0;
