@@ -1,4 +1,4 @@
-// Register-resident line FFT for power-of-two lengths N = E*T in {16..512}.
+// Register-resident line FFT for lengths N = E*T in {16..512}.
 //
 // A line is held by T threads, thread t owning elements t + T*i (i < E).  The
 // transform is the four-step factorisation N = E*T: an E-point DFT in
@@ -16,33 +16,39 @@
 namespace ddb {
 
 #include "w96.inc"
+#include "w160.inc"
 
-// W_K^m for DIR: exp(DIR * 2*pi*i*m/K), K divides 96
+// W_K^m for DIR: exp(DIR * 2*pi*i*m/K), K divides 96 or 160
 template <int K, int DIR, typename C> DDB_HD C wk(int m) {
-  static_assert(96 % K == 0, "in-register DFT sizes must divide 96");
-  const int q = (m * (96 / K)) % 96;
-  return mk<C>(w96re(q), DIR < 0 ? w96im(q) : -w96im(q));
+  static_assert(96 % K == 0 || 160 % K == 0, "in-register DFT sizes must divide 96 or 160");
+  if constexpr (96 % K == 0) {
+    const int q = (m * (96 / K)) % 96;
+    return mk<C>(w96re(q), DIR < 0 ? w96im(q) : -w96im(q));
+  } else {
+    const int q = (m * (160 / K)) % 160;
+    return mk<C>(w160re(q), DIR < 0 ? w160im(q) : -w160im(q));
+  }
 }
 
 // x * W_K^m: the multiples of pi/4 are a rotation, a negation or the radix-8
 // forms (m is a compile-time constant after unrolling, so the branches fold)
 template <int K, int DIR, typename C> __device__ __forceinline__ C cmul_wk(C x, int m) {
-  const int q = (m * (96 / K)) % 96;
+  const int q = (8 * m) % (8 * K);  // in units of 1/(8 K) of a turn
   using R = decltype(x.x);
   const R m1 = (R)-1.0;
   if (q == 0) return x;
-  if (q == 48) return mk2<C>(m1 * x.x, m1 * x.y);
-  if (q == 24) return rot4<DIR>(x);
-  if (q == 72) return rot4<-DIR>(x);
-  if (q == 12) return w8_1<DIR>(x);
-  if (q == 36) return w8_3<DIR>(x);
-  if (q == 60) return w8_3<-DIR>(x);  // exp(5 i pi/4) = exp(-3 i pi/4)
-  if (q == 84) return w8_1<-DIR>(x);  // exp(7 i pi/4) = exp(-i pi/4)
+  if (q == 4 * K) return mk2<C>(m1 * x.x, m1 * x.y);
+  if (q == 2 * K) return rot4<DIR>(x);
+  if (q == 6 * K) return rot4<-DIR>(x);
+  if (q == K) return w8_1<DIR>(x);
+  if (q == 3 * K) return w8_3<DIR>(x);
+  if (q == 5 * K) return w8_3<-DIR>(x);  // exp(5 i pi/4) = exp(-3 i pi/4)
+  if (q == 7 * K) return w8_1<-DIR>(x);  // exp(7 i pi/4) = exp(-i pi/4)
   return cmul(x, wk<K, DIR, C>(m));
 }
 
 // first factor of the four-step split K = K1 * K2 of an in-register DFT
-template <int K> constexpr int dft_split() { return (K == 16 || K == 12) ? 4 : 8; }
+template <int K> constexpr int dft_split() { return (K == 16 || K == 12 || K == 20) ? 4 : 8; }
 
 template <int K, int DIR, typename C> __device__ __forceinline__ void dftr(C* v) {
   if constexpr (K == 1) {
@@ -54,8 +60,10 @@ template <int K, int DIR, typename C> __device__ __forceinline__ void dftr(C* v)
     bfly8<DIR>(v);
   } else if constexpr (K == 3) {
     bfly3<DIR>(v);
+  } else if constexpr (K == 5) {
+    bfly5<DIR>(v);
   } else {
-    // K = K1*K2 (16 = 4*4, 32 = 8*4, 12 = 4*3, 24 = 8*3): element K2*a + b ; output c + K1*d
+    // K = K1*K2 (16 = 4*4, 32 = 8*4, 12 = 4*3, 24 = 8*3, 20 = 4*5, 40 = 8*5): element K2*a + b ; output c + K1*d
     constexpr int K1 = dft_split<K>();
     constexpr int K2 = K / K1;
     C Y[K2][K1];
@@ -261,14 +269,20 @@ template <> struct RegShape<512> { static constexpr int E = 32, T = 16; };
 template <> struct RegShape<48> { static constexpr int E = 12, T = 4; };
 template <> struct RegShape<96> { static constexpr int E = 24, T = 4; };
 template <> struct RegShape<192> { static constexpr int E = 24, T = 8; };
+// 5 * 2^k lengths (x-first pipeline only)
+template <> struct RegShape<80> { static constexpr int E = 20, T = 4; };
+template <> struct RegShape<160> { static constexpr int E = 40, T = 4; };
+template <> struct RegShape<320> { static constexpr int E = 40, T = 8; };
 
 inline bool reg_supported(int n) { return n == 16 || n == 32 || n == 64 || n == 128 || n == 256 || n == 512; }
-inline bool xreg_supported(int n) { return reg_supported(n) || n == 48 || n == 96 || n == 192; }
+inline bool xreg_supported(int n) {
+  return reg_supported(n) || n == 48 || n == 96 || n == 192 || n == 80 || n == 160 || n == 320;
+}
 // threads per line of the register shape of length n (RegShape<n>::T)
 inline int reg_threads(int n) {
   switch (n) {
-    case 16: case 32: case 48: case 96: return 4;
-    case 64: case 128: case 192: return 8;
+    case 16: case 32: case 48: case 96: case 80: case 160: return 4;
+    case 64: case 128: case 192: case 320: return 8;
     default: return 16;
   }
 }

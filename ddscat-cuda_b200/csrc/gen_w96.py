@@ -1,12 +1,14 @@
-"""Writes w96.inc: exp(-2 pi i m / 96), m = 0..95, as 21-digit decimal literals.
+"""Writes w<L>.inc: exp(-2 pi i m / L), m = 0..L-1, as 21-digit decimal literals.
 
-96 is divisible by every in-register DFT size the line FFTs use (2, 3, 4, 8,
-12, 16, 24, 32), so wk<K>(m) = W96^(m * 96 / K).  The values are computed with
-Python's decimal module at 40 digits (pi from Machin's formula, cos and sin
-from their Taylor series), so every literal is correctly rounded.
+96 is divisible by the in-register DFT sizes 2, 3, 4, 8, 12, 16, 24 and 32 of the
+line FFTs, 160 by 5, 20 and 40: wk<K>(m) = W_L^(m * L / K).  The values are
+computed with Python's decimal module at 40 digits (pi from Machin's formula,
+cos and sin from their Taylor series), so every literal is correctly rounded.
 
     python gen_w96.py > w96.inc
+    python gen_w96.py 160 > w160.inc
 """
+import sys
 from decimal import Decimal, getcontext
 
 getcontext().prec = 40
@@ -56,17 +58,18 @@ def lit(v):
 
 
 def main():
+    L = int(sys.argv[1]) if len(sys.argv) > 1 else 96
     re, im = [], []
-    for m in range(96):
-        c, s = cos_sin(2 * PI * m / 96)
-        if m % 24 == 0:
-            c, s = [Decimal(1), Decimal(0), Decimal(-1), Decimal(0)][m // 24], [Decimal(0), Decimal(1), Decimal(0), Decimal(-1)][m // 24]
+    for m in range(L):
+        c, s = cos_sin(2 * PI * m / L)
+        if m % (L // 4) == 0:
+            c, s = [Decimal(1), Decimal(0), Decimal(-1), Decimal(0)][m // (L // 4)], [Decimal(0), Decimal(1), Decimal(0), Decimal(-1)][m // (L // 4)]
         re.append(c)
         im.append(-s)
-    out = ["// exp(-2*pi*i*m/96) = w96re(m) + i*w96im(m); exact decimal literals (21 digits), from gen_w96.py."]
-    for name, vals in (("w96re", re), ("w96im", im)):
+    out = [f"// exp(-2*pi*i*m/{L}) = w{L}re(m) + i*w{L}im(m); exact decimal literals (21 digits), from gen_w96.py."]
+    for name, vals in ((f"w{L}re", re), (f"w{L}im", im)):
         out.append(f"DDB_HD constexpr double {name}(int m) {{")
-        out.append("  switch (((m % 96) + 96) % 96) {")
+        out.append(f"  switch (((m % {L}) + {L}) % {L}) {{")
         for m, v in enumerate(vals):
             out.append(f"    case {m}: return {lit(v)};")
         out.append("    default: return 0.0;")

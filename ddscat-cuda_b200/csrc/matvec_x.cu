@@ -95,7 +95,7 @@ template <int N> struct XShape {
   static constexpr int E = RegShape<N>::E, TT = RegShape<N>::T, H = E / 2;
   static constexpr int RL = 256 / TT;
   static constexpr int RZ = (128 / TT) > 1 ? 128 / TT : 1;  // ZG lines per block (3*TT*RZ threads)
-  static constexpr int ZG_MINB = E >= 32 ? 1 : (E >= 24 ? 2 : 3);  // ZG blocks per SM the registers must allow (FP32)
+  static constexpr int ZG_MINB = E >= 32 ? 1 : (E > 16 ? 2 : 3);  // ZG blocks per SM the registers must allow (FP32)
   static constexpr bool PAIR = TT >= 8;                      // 128-bit transpose stores (conflict-free for TT >= 8)
 };
 
@@ -1253,12 +1253,20 @@ template <typename T> static const void* xkernel(XPass p, int n, int my = 0) {
     case 32: return xk<T, 32>(p, my);
     case 48: return xk<T, 48>(p, my);
     case 64: return xk<T, 64>(p, my);
+    case 80: return xk<T, 80>(p, my);
     case 96: return xk<T, 96>(p, my);
     case 128: return xk<T, 128>(p, my);
     case 192: return xk<T, 192>(p, my);
     case 256: return xk<T, 256>(p, my);
+    // FP64: the shared memory of the 160-, 320- and 512-point passes is too large
+    case 160:
+      if constexpr (sizeof(T) == 4) return xk<T, 160>(p, my);
+      return nullptr;
+    case 320:
+      if constexpr (sizeof(T) == 4) return xk<T, 320>(p, my);
+      return nullptr;
     case 512:
-      if constexpr (sizeof(T) == 4) return xk<T, 512>(p, my);  // FP64: shared memory of the 512 passes too large
+      if constexpr (sizeof(T) == 4) return xk<T, 512>(p, my);
       return nullptr;
     default: return nullptr;
   }
@@ -1302,10 +1310,17 @@ template <typename T> static int xlaunch(const void* f, dim3 g, int th, size_t s
 
 bool xzg3_supported(int Mz) { return xkernel<float>(XPass::ZG3, Mz) != nullptr; }
 
+// The axis lengths of the pipeline (FP64: up to 256 but 160, by shared memory).
+// The 5 * 2^k ones close the gaps of up to 1.5 between 2^k and 3 * 2^k (of 2
+// above 256); ms per RHS at 8 RHS per call with and without them: 36^3 0.0151 /
+// 0.0245, 72^3 0.136 / 0.154, 80^3 0.149 / 0.165, 150x150x40 0.252 / 0.530.
+template <typename T> static bool xpipe_length(int n) {
+  return xreg_supported(n) && (sizeof(T) == 4 || (n <= 256 && n != 160));
+}
+
 template <typename T> bool xpipe_supported(const Geometry& g) {
   if (env_flag("DDSCAT_B200_ZFIRST")) return false;
-  // FP64: axis lengths up to 256 (the shared memory of the 512-point passes is too large in complex double)
-  auto ok = [](int n) { return xreg_supported(n) && (sizeof(T) == 4 || n <= 256); };
+  auto ok = [](int n) { return xpipe_length<T>(n); };
   return ok(g.Mx) && ok(g.My) && ok(g.Mz);
 }
 
@@ -1538,8 +1553,8 @@ template <typename T> int interleave_green_zfast(Engine<T>& E, const cplx<T>* pl
 }
 
 template <typename T> int xpipe_len(int m) {
-  for (int L : {16, 32, 48, 64, 96, 128, 192, 256, 512})
-    if (L >= m && xreg_supported(L) && (sizeof(T) == 4 || L <= 256)) return L;
+  for (int L : {16, 32, 48, 64, 80, 96, 128, 160, 192, 256, 320, 512})
+    if (L >= m && xpipe_length<T>(L)) return L;
   return 0;
 }
 
