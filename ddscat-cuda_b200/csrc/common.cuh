@@ -112,6 +112,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
+// Shared -> global counterpart (after fence.proxy.async); returns when the
+// copies have read shared memory.
+__device__ __forceinline__ void bulk_s2g_wait(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)), "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
 // Per-thread asynchronous 8-byte global -> shared copy (zero-fills when !ok;
 // src must still be a valid address); completed by cp_async_wait_all.
 __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {

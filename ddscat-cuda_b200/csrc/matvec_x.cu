@@ -438,6 +438,12 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RZ;
   constexpr int GT = 3 * TT;  // Green-phase threads per line
+  // FP32 rows of the 96- and 192-point passes move by bulk copies: a 64x56x48
+  // batched solve 113.4 -> 108.3 ms, 48^3 with 8 RHS 0.0287 -> 0.0275 ms per
+  // RHS-MATVEC, 96^3 0.179 -> 0.177.  Not at 80, 160 and 320 points, where rows
+  // are short or one block per SM waits for its copies (36^3 0.0151 -> 0.0153,
+  // 72^3 0.136 -> 0.140), nor at 512 (128-byte loads).
+  constexpr bool BULK = sizeof(C) == 8 && BTY == 0 && E == 24;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = (threadIdx.x / TT) % RL, c = threadIdx.x / (TT * RL);
   C* lines = reinterpret_cast<C*>(smem_raw);  // [3][RL][lsz]
@@ -452,9 +458,30 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   constexpr int zs = zline_stride<BTY>();
   C* row = P.B + ((size_t)(rb * 3 + c) * P.nkx) * (size_t)P.My * (BTY ? P.nz : P.ldb) + zline_base<BTY>(P, live ? p : 0);
   C v[E];
+  if constexpr (BULK) {
+    // one bulk copy per line: the TT < 16 threads of a line load 32 or 64 bytes
+    // of its row at a time, so a warp's loads would touch 4 or 8 cache lines each
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      mbar_arrive_expect_tx(&bar, (unsigned)(3 * min(RL, nlines - (int)blockIdx.y * RL) * P.ldb * (int)sizeof(C)));
+    }
+    __syncthreads();
+    if (t == 0 && live) bulk_g2s(my, row, (unsigned)(P.ldb * (int)sizeof(C)), &bar);
+    // one decision for the whole block: every thread's bounded wait succeeded
+    if (!__syncthreads_and(mbar_wait(&bar, 0, TMA_WAIT_POLLS))) {
+      if (threadIdx.x == 0) atomicOr(P.err, 1);
+      mbar_wait(&bar, 0, TMA_WAIT_POLLS);
+      return;
+    }
 #pragma unroll
-  for (int i = 0; i < H; ++i)
-    v[i] = live && t + TT * i < P.nz ? row[(t + TT * i) * zs] : mk<C>(0, 0);  // iz < nz <= N/2
+    for (int i = 0; i < H; ++i) v[i] = live && t + TT * i < P.nz ? my[t + TT * i] : mk<C>(0, 0);
+    __syncwarp();  // the row is read before the line scratch reuses it
+  } else {
+#pragma unroll
+    for (int i = 0; i < H; ++i)
+      v[i] = live && t + TT * i < P.nz ? row[(t + TT * i) * zs] : mk<C>(0, 0);  // iz < nz <= N/2
+  }
   line_fft<E, TT, +1, false, true, S_::PAIR>(v, my, t, P.twz);
 #pragma unroll
   for (int i = 0; i < E; ++i) my[t + TT * i] = v[i];
@@ -507,7 +534,14 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   for (int i = 0; i < E; ++i) v[i] = my[t + TT * i];
   __syncwarp();
   line_fft<E, TT, -1, false, false, S_::PAIR>(v, my, t, P.twz);
-  if (live) {
+  if constexpr (BULK) {
+#pragma unroll
+    for (int i = 0; i < H; ++i)
+      if (t + TT * i < P.nz) my[t + TT * i] = v[i];  // keep iz < nz
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (t == 0 && live) bulk_s2g_wait(row, my, (unsigned)(P.ldb * (int)sizeof(C)));
+  } else if (live) {
 #pragma unroll
     for (int i = 0; i < H; ++i)
       if (t + TT * i < P.nz) row[(t + TT * i) * zs] = v[i];  // keep iz < nz
