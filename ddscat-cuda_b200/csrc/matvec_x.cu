@@ -701,11 +701,16 @@ __device__ __forceinline__ void zg3_green_s(const C* rec, int t, C (&v)[3][E]) {
   }
 }
 
-// Row buffer of a line: N/2 elements and, for TT < 16, TT more, so that the
-// lines of a half-warp read different banks.
+// Row buffer of a line: N/2 elements.  The lines of a half-warp read different
+// banks: with TT = 8 the odd lines exchange neighbouring groups of 8 elements
+// (padding instead would leave 2 blocks per SM at N = 128: three need
+// (18.0 + 48.8 + 8 + 1) KB each of the SM's 228), with TT = 4 lines are 4
+// elements apart.
 template <int N> struct ZRow {
-  static constexpr int STRIDE = N / 2 + (XShape<N>::TT < 16 ? XShape<N>::TT : 0);
+  static constexpr int STRIDE = N / 2 + (XShape<N>::TT == 4 ? 4 : 0);
   static constexpr int PAIRS = (N / 4 + XShape<N>::TT - 1) / XShape<N>::TT;  // 16-byte copies per thread and row
+  // exchanged groups of the odd lines (N/2 is a multiple of 16)
+  static constexpr int SWAP = XShape<N>::TT == 8 && N % 32 == 0 ? 8 : 0;
 };
 
 template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(XParams<T> P) {
@@ -734,6 +739,9 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
   // the TT threads of a line copy its row of component c for RHS rb to the
   // line's buffer (16-byte pairs; rows have an even length)
   C* buf = gs + (size_t)RZ * LREC + (size_t)l * ZRow<N>::STRIDE;
+  const int swap = l & 1 ? ZRow<N>::SWAP : 0;
+  const C* const even = buf + t + swap;  // element t + TT*i, i even / odd
+  const C* const odd = buf + t - swap;
   const C* lrow = P.B + (size_t)(live ? p : 0) * P.ldb;
   auto fetch = [&](int rb, int c) {
     if (live) {
@@ -741,7 +749,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
 #pragma unroll
       for (int k = 0; k < ZRow<N>::PAIRS; ++k) {
         const int o = 2 * (t + TT * k);
-        if (o < P.ldb) cp_async16(buf + o, src + o);
+        if (o < P.ldb) cp_async16(buf + (o ^ swap), src + o);
       }
     }
     cp_async_commit();
@@ -780,7 +788,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
       const R sc = c == 0 ? sx : (c == 1 ? sy : (R)1);
 #pragma unroll
       for (int i = 0; i < H; ++i)
-        v[c][i] = live && t + TT * i < P.nz ? cscale(buf[t + TT * i], sc) : mk<C>(0, 0);  // iz < nz <= N/2
+        v[c][i] = live && t + TT * i < P.nz ? cscale((i & 1 ? odd : even)[TT * i], sc) : mk<C>(0, 0);  // iz < nz <= N/2
       __syncwarp();  // the buffer is read before the next row overwrites it
       if (c < 2) fetch(rb, c + 1);
       else if (nrb < rb1) fetch(nrb, 0);
@@ -1466,7 +1474,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   // ZG3R (Green lines staged once per block and reused for a chunk of RHS):
   // IPBC=0, batches of at least 4 RHS (DDSCAT_B200_NOZG3R=1 keeps ZG3)
   const void* fzg3r = fzg3 && g.ipbc == 0 && !env_flag("DDSCAT_B200_NOZG3R") ? xkernel<T>(XPass::ZG3R, g.Mz) : nullptr;
-  const size_t smzr = smz + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ < 16 ? TZ : 0)) * sizeof(C);
+  const size_t smzr = smz + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ == 4 ? 4 : 0)) * sizeof(C);
   const void* fxf = xkernel<T>(XPass::XF, g.Mx);
   const void* fyf = xkernel<T>(XPass::YF, g.My);
   const void* fzg = xkernel<T>(XPass::ZG, g.Mz);
