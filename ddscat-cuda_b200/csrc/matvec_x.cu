@@ -928,7 +928,10 @@ template <typename T> __device__ __forceinline__ void xdot_reduce(const XParams<
 // the registers allow one block per SM anyway.  ms per RHS-MATVEC staged and not, 8
 // RHS: 48^3 0.0262 / 0.0275, 96^3 0.170 / 0.177, 160x30x30 0.0315 / 0.0330; at 160
 // points a second chunk buffer costs more than it gives (66^3 0.136 / 0.133).
-constexpr bool xi_staged(int n, int TT) { return 256 / TT * (n / 2) <= 3072 || n == 320; }
+// FP64: up to 2048 elements (3072 and the tile exceed the shared memory).
+constexpr bool xi_staged(int n, int TT, size_t elem) {
+  return elem == 8 ? 256 / TT * (n / 2) <= 3072 || n == 320 : 256 / TT * (n / 2) <= 2048;
+}
 
 // block: RL rows (iy) x TT; grid (ceil(ny/RL), nz, 3*nr)
 // shared memory: tile / line scratch [tlx] | x chunk | CXADIA chunk
@@ -937,7 +940,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   constexpr int MAXC = RL * (N / 2);
-  constexpr bool STAGE = xi_staged(N, TT);  // the other rows keep direct loads (shared memory)
+  constexpr bool STAGE = xi_staged(N, TT, sizeof(C));  // the other rows keep direct loads (shared memory)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
@@ -1457,7 +1460,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   // XI: the x and CXADIA chunks of RX rows, each sized as the kernel lays them
   // out (MAXC = RL * N/2 elements, which is RX * nx only when Mx = 2 nx)
   const size_t xi_maxc = (size_t)RX * (g.Mx / 2);
-  const size_t smxi = smx + (xi_staged(g.Mx, TX) ? 2 * xi_maxc * sizeof(C) : 0);
+  const size_t smxi = smx + (xi_staged(g.Mx, TX, sizeof(C)) ? 2 * xi_maxc * sizeof(C) : 0);
   size_t smy = std::max((size_t)g.My * tile_stride(RY, TY, sizeof(C)), (size_t)RY * P.lsy) * sizeof(C);
   // tensor tiles for the 256-point y passes (FP32, five-pass B layout): the
   // slab as rows of n_z; the tile needs 32 KB at a 1024-byte boundary

@@ -49,7 +49,7 @@ def test_cpu_supplied_spectrum(dims):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(40, 38, 37), (70, 9, 33), (9, 36, 75)])
+@pytest.mark.parametrize("dims", [(40, 38, 37), (70, 9, 33), (9, 36, 75), (96, 5, 8), (48, 6, 6)])
 def test_fp64_and_batches(dims):
     iocc, ak, _ = _inputs(dims)
     nat = iocc.size
