@@ -130,7 +130,7 @@ template <typename T> struct Engine {
   // device status word of the MATVEC kernels (0 = ok): a kernel whose bounded
   // wait for an asynchronous tile copy ran out sets it (matvec_check)
   int* d_err = nullptr;
-  // tile moves of the FP32 256-point y passes by the tensor memory accelerator
+  // tile moves of the FP32 x and y passes by the tensor memory accelerator
   // (DDSCAT_B200_NOTMA=1 selects the per-thread copies)
   int use_tma = 1;
   // smallest RHS chunk per block for which the z pass stages its Green lines

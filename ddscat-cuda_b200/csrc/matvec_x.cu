@@ -5,7 +5,7 @@
 // of its input with the T threads of a line inside one warp (register line
 // FFTs, fftreg.cuh), and the axis change is done by a shared-memory tile
 // transpose on the load or store side, keeping global accesses in 128-byte
-// segments (at the 256- and 512-point shapes the tiles move between shared and
+// segments (at most lengths from 64 the tiles move between shared and
 // global memory by the tensor memory accelerator):
 //   XF : x (compact or full) rows  -> x-FFT(+i), pad-skip -> A[c][iz][kx][iy]
 //   YF : A y-rows (n_y)            -> y-FFT(+i)           -> B[c][kx][ky][iz]
@@ -38,10 +38,10 @@
 namespace ddb {
 
 template <typename T> struct XParams {
-  // B as a 2-D tensor of rows of n_z 8-byte complex floats, box {16, 256},
-  // 128-byte swizzle: the tiles of the 256-point y passes (tma != 0)
+  // B as a 2-D tensor of rows of n_z 8-byte complex floats, 16 columns per box,
+  // 128-byte swizzle: the tiles of the y passes (tma != 0)
   alignas(64) CUtensorMap tmB;
-  // A as rows of n_y complex floats, box {16, 256}: the tiles of the 256-point
+  // A as rows of n_y complex floats: the tiles of the
   // x passes (tma_x != 0)
   alignas(64) CUtensorMap tmA;
   int tma;
@@ -99,48 +99,78 @@ template <int N> struct XShape {
   static constexpr bool PAIR = TT >= 8;                      // 128-bit transpose stores (conflict-free for TT >= 8)
 };
 
-// ---- tensor-memory-accelerator tiles of the 256-point y passes (FP32)
-// A y-pass tile holds 256 rows (ky) of 16 consecutive z positions: 128 bytes
-// per row, stored with the 128-byte swizzle (16-byte chunk j of row r at chunk
-// j ^ (r & 7)), the layout a box of {16, 256} 8-byte elements has in shared
-// memory.  The tile base is 1024-byte aligned.  Threads write and read it
-// through tma_slot; the tensor map covers this GPU's own B buffer and no
-// multicast is used.
-constexpr int TMA_ROWS = 256, TMA_COLS = 16;
-constexpr unsigned TMA_TILE_BYTES = TMA_ROWS * TMA_COLS * 8;
+// ---- tensor-memory-accelerator tiles of the x and y passes (FP32)
+// A tile holds N rows of RL columns (RL consecutive z positions of B in the y
+// passes, y positions of A in the x passes) as RL/16 boxes of 16 columns: 128
+// bytes per row, stored with the 128-byte swizzle (16-byte chunk j of row r at
+// chunk j ^ (r & 7)), the layout a tensor-map box of 16 8-byte elements has in
+// shared memory.  A box has N rows, or N/2 where N > 256; every box starts on
+// 1024 bytes (the swizzle phase r & 7 is the same in each).  Threads write and
+// read the tile through tma_slot; the tensor maps cover this GPU's own A and B
+// buffers and no multicast is used.
+// The per-thread copies these replace (16-byte shared-memory reads with global
+// stores, and the reverse) are a third of the shared-memory and L1 wavefronts of
+// a pass, and at 64 to 192 points L1 was the limit (79-81 % busy at 128 points,
+// DRAM 38-66 %).  ms per RHS-MATVEC with and without, 8 RHS: 64^3 0.0451 / 0.0480,
+// 96^3 0.159 / 0.170, 150x150x40 0.232 / 0.253, 48^3 0.0256 / 0.0263.  Lengths below
+// 64 keep the per-thread copies (passes of microseconds, where a tensor copy's
+// latency shows), and so do 80 and 160: their 4 threads per line meet two to a
+// bank in the swizzled rows (66^3 0.141 / 0.133, 36^3 with one RHS 0.0373 / 0.0342).
+constexpr int TMA_COLS = 16;
 constexpr int TMA_WAIT_POLLS = 1 << 24;  // bounded wait for a tile load (seconds at most)
-__device__ __forceinline__ int tma_slot(int r, int col) {
-  return r * TMA_COLS + (((col >> 1) ^ (r & 7)) << 1) + (col & 1);
+constexpr int tma_box_rows(int n) { return n > 256 ? n / 2 : n; }
+constexpr bool tma_length(int n, size_t elem) { return n >= 64 && n != 80 && n != 160 && elem == 8; }
+constexpr size_t tma_tile_bytes(int n, int cols) { return (size_t)n * cols * 8; }
+template <int N> __device__ __forceinline__ int tma_slot(int r, int col) {
+  return (col / TMA_COLS) * (N * TMA_COLS) + r * TMA_COLS + ((((col % TMA_COLS) >> 1) ^ (r & 7)) << 1) + (col & 1);
 }
 __device__ __forceinline__ float2* tma_tile(unsigned char* smem) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(smem);
   return reinterpret_cast<float2*>((a + 1023) & ~(uintptr_t)1023);
 }
-// A tile of N = 256 or 512 rows is N/256 boxes of 256 rows, each 32 KB and
-// 1024-byte aligned (the swizzle phase r & 7 is the same in every box).
-template <int N> constexpr bool tma_rows_ok() { return N == 256 || N == 512; }
-// store the tile's boxes at (x = inner position, y = first row) of the map;
-// the issuing thread waits until the copies have read the tile (the CTA keeps
-// its shared memory)
-template <int N> __device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, const float2* tile, int x, int y) {
+// boxes of 16 columns that hold at least one of the tile's `valid` columns
+template <int RL> __device__ __forceinline__ int tma_boxes(int valid) {
+  return min(RL / TMA_COLS, (valid + TMA_COLS - 1) / TMA_COLS);
+}
+// store the tile's boxes at (x = inner position, y = first row) of the map
+// (columns beyond the grid are clipped by it); the issuing thread waits until
+// the copies have read the tile (the CTA keeps its shared memory)
+template <int N, int RL>
+__device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, const float2* tile, int x, int y, int valid) {
+  constexpr int BR = tma_box_rows(N);
+  const int nb = tma_boxes<RL>(valid);
 #pragma unroll
-  for (int b = 0; b < N / TMA_ROWS; ++b)
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x),
-                 "r"(y + b * TMA_ROWS), "r"(smem_addr(tile + (size_t)b * TMA_ROWS * TMA_COLS))
-                 : "memory");
+  for (int c = 0; c < RL / TMA_COLS; ++c) {
+    if (c >= nb) break;
+#pragma unroll
+    for (int b = 0; b < N / BR; ++b)
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map),
+                   "r"(x + c * TMA_COLS), "r"(y + b * BR),
+                   "r"(smem_addr(tile + (size_t)(c * N + b * BR) * TMA_COLS))
+                   : "memory");
+  }
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
-// load the tile's boxes, completing on bar (which expects N/256 * 32 KB)
-template <int N>
-__device__ __forceinline__ void tma_load_tile(const CUtensorMap* map, float2* tile, int x, int y, uint64_t* bar) {
+// load the tile's boxes with `valid` columns in the grid, completing on bar
+// (columns beyond the grid read as 0; boxes without any keep what was there)
+template <int N, int RL>
+__device__ __forceinline__ void tma_load_tile(const CUtensorMap* map, float2* tile, int x, int y, int valid,
+                                              uint64_t* bar) {
+  constexpr int BR = tma_box_rows(N);
+  const int nb = tma_boxes<RL>(valid);
+  mbar_arrive_expect_tx(bar, (unsigned)(nb * N * TMA_COLS * 8));
 #pragma unroll
-  for (int b = 0; b < N / TMA_ROWS; ++b)
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_addr(tile + (size_t)b * TMA_ROWS * TMA_COLS)),
-        "l"(map), "r"(x), "r"(y + b * TMA_ROWS), "r"(smem_addr(bar))
-        : "memory");
+  for (int c = 0; c < RL / TMA_COLS; ++c) {
+    if (c >= nb) break;
+#pragma unroll
+    for (int b = 0; b < N / BR; ++b)
+      asm volatile(
+          "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+              smem_addr(tile + (size_t)(c * N + b * BR) * TMA_COLS)),
+          "l"(map), "r"(x + c * TMA_COLS), "r"(y + b * BR), "r"(smem_addr(bar))
+          : "memory");
+  }
 }
 
 // Row stride (elements of C) of a transpose tile of N rows x RL columns.  The
@@ -284,16 +314,16 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
   }
   line_fft<E, TT, +1, false, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx);
   __syncthreads();  // all line scratch consumed before the tile reuses it
-  if constexpr (tma_rows_ok<N>() && RL == TMA_COLS && sizeof(C) == 8) {
+  if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma_x) {
-      // swizzled tile, then one tensor store of its 256 x 16 elements (rows
+      // swizzled tile, then tensor stores of its boxes (rows
       // beyond n_y are clipped by the map)
       C* tt = tma_tile(smem_raw);
 #pragma unroll
-      for (int i = 0; i < E; ++i) tt[tma_slot(t + TT * i, l)] = v[i];
+      for (int i = 0; i < E; ++i) tt[tma_slot<N>(t + TT * i, l)] = v[i];
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
-      if (threadIdx.x == 0) tma_store_tile<N>(&P.tmA, tt, iy0, ((rl * 3 + c) * P.nz + iz) * P.Mx);
+      if (threadIdx.x == 0) tma_store_tile<N, RL>(&P.tmA, tt, iy0, ((rl * 3 + c) * P.nz + iz) * P.Mx, P.ny - iy0);
       return;
     }
   }
@@ -326,16 +356,16 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
   for (int i = 0; i < H; ++i) v[i] = zin && t + TT * i < P.ny ? A[t + TT * i] : mk<C>(0, 0);  // iy < ny <= N/2
   line_fft<E, TT, +1, false, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy);
   __syncthreads();
-  if constexpr (tma_rows_ok<N>() && RL == TMA_COLS && sizeof(C) == 8) {
+  if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma) {
-      // swizzled tile, then one tensor store of its 256 x 16 elements (z
+      // swizzled tile, then tensor stores of its boxes (z
       // positions beyond n_z are clipped by the map)
       C* tt = tma_tile(smem_raw);
 #pragma unroll
-      for (int i = 0; i < E; ++i) tt[tma_slot(t + TT * i, l)] = v[i];
+      for (int i = 0; i < E; ++i) tt[tma_slot<N>(t + TT * i, l)] = v[i];
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncthreads();
-      if (threadIdx.x == 0) tma_store_tile<N>(&P.tmB, tt, iz0, ((rb * 3 + c) * P.nkx + kxl) * P.My);
+      if (threadIdx.x == 0) tma_store_tile<N, RL>(&P.tmB, tt, iz0, ((rb * 3 + c) * P.nkx + kxl) * P.My, P.nz - iz0);
       return;
     }
   }
@@ -833,17 +863,15 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
   const int nz = P.nz;
   C v[E];
   bool loaded = false;
-  if constexpr (tma_rows_ok<N>() && RL == TMA_COLS && sizeof(C) == 8) {
+  if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma) {
-      // one tensor load of the 256 x 16 tile (z positions beyond n_z read as 0)
+      // tensor loads of the tile (z positions beyond n_z read as 0)
       __shared__ __align__(8) uint64_t bar;
       C* tt = tma_tile(smem_raw);
       if (threadIdx.x == 0) mbar_init(&bar, 1);
       __syncthreads();
-      if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(&bar, (N / TMA_ROWS) * TMA_TILE_BYTES);
-        tma_load_tile<N>(&P.tmB, tt, iz0, ((rb * 3 + c) * P.nkx + kxl) * P.My, &bar);
-      }
+      if (threadIdx.x == 0)
+        tma_load_tile<N, RL>(&P.tmB, tt, iz0, ((rb * 3 + c) * P.nkx + kxl) * P.My, nz - iz0, &bar);
       // one decision for the whole block: every thread's bounded wait succeeded
       if (!__syncthreads_and(mbar_wait(&bar, 0, TMA_WAIT_POLLS))) {
         // the copy did not complete in the allowed time: report it, wait once
@@ -853,7 +881,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
         return;
       }
 #pragma unroll
-      for (int i = 0; i < E; ++i) v[i] = tt[tma_slot(t + TT * i, l)];
+      for (int i = 0; i < E; ++i) v[i] = tt[tma_slot<N>(t + TT * i, l)];
       __syncthreads();  // the tile is consumed before the line scratch reuses it
       loaded = true;
     }
@@ -981,18 +1009,16 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
   }
   C v[E];
   bool loaded = false;
-  if constexpr (tma_rows_ok<N>() && RL == TMA_COLS && sizeof(C) == 8) {
+  if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma_x) {
-      // one tensor load of the 256 x 16 tile of A (rows beyond n_y read as 0),
+      // tensor loads of the tile of A (rows beyond n_y read as 0),
       // while the x and CXADIA chunks arrive by per-thread copies
       __shared__ __align__(8) uint64_t bar;
       C* tt = tma_tile(smem_raw);
       if (threadIdx.x == 0) mbar_init(&bar, 1);
       __syncthreads();
-      if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(&bar, (N / TMA_ROWS) * TMA_TILE_BYTES);
-        tma_load_tile<N>(&P.tmA, tt, iy0, ((rl * 3 + c) * P.nz + iz) * P.Mx, &bar);
-      }
+      if (threadIdx.x == 0)
+        tma_load_tile<N, RL>(&P.tmA, tt, iy0, ((rl * 3 + c) * P.nz + iz) * P.Mx, ny - iy0, &bar);
       cp_async_wait_all();  // the x and CXADIA chunks
       // one decision for the whole block (the barrier also publishes every
       // thread's chunk copies): every thread's bounded wait succeeded
@@ -1004,7 +1030,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
         return;
       }
 #pragma unroll
-      for (int i = 0; i < E; ++i) v[i] = tt[tma_slot(t + TT * i, l)];
+      for (int i = 0; i < E; ++i) v[i] = tt[tma_slot<N>(t + TT * i, l)];
       __syncthreads();
       loaded = true;
     }
@@ -1390,16 +1416,16 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// Map of B (rows of n_z complex floats, row stride ld * 8 bytes) for the
-// 256-point y passes' tiles, or of A (rows of n_y) for the x passes: box
-// {16, 256}, 128-byte swizzle, zero fill.  ld is even, so the stride is a
+// Map of B (rows of n_z complex floats, row stride ld * 8 bytes) for the tiles
+// of the y passes of length m, or of A (rows of n_y) for the x passes: box
+// {16, tma_box_rows(m)}, 128-byte swizzle, zero fill.  ld is even, so the stride is a
 // multiple of 16 bytes; an odd n ends the row inside its last pair.
-static bool encode_b_map(CUtensorMap* m, void* base, size_t rows, int nz, int ld) {
+static bool encode_b_map(CUtensorMap* m, void* base, size_t rows, int nz, int ld, int len) {
   const auto enc = tensor_map_encoder();
   if (!enc || rows > 0xffffffffull || (ld & 1)) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)nz, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 8};
-  const cuuint32_t box[2] = {(cuuint32_t)TMA_COLS, (cuuint32_t)TMA_ROWS};
+  const cuuint32_t box[2] = {(cuuint32_t)TMA_COLS, (cuuint32_t)tma_box_rows(len)};
   const cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1453,28 +1479,26 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
                : std::max(line_stride(g.Mz / TZ, TZ, RZ, false, TZ >= 8), g.Mz);
   // the transpose tile and the line scratch share one region
   P.tlx = (int)std::max((size_t)g.Mx * tile_stride(RX, TX, sizeof(C)), (size_t)RX * P.lsx);
-  // a tensor tile of the x passes (32 KB at a 1024-byte boundary) fits in front of the XI chunks
-  if (g.Mx == 256 || g.Mx == 512)
-    P.tlx = std::max(P.tlx, (int)(((size_t)(g.Mx / TMA_ROWS) * TMA_TILE_BYTES + 1024) / sizeof(C)));
+  // a tensor tile of the x passes (at a 1024-byte boundary) fits in front of the XI chunks
+  if (tma_length(g.Mx, sizeof(C))) P.tlx = std::max(P.tlx, (int)((tma_tile_bytes(g.Mx, RX) + 1024) / sizeof(C)));
   const size_t smx = (size_t)P.tlx * sizeof(C);
   // XI: the x and CXADIA chunks of RX rows, each sized as the kernel lays them
   // out (MAXC = RL * N/2 elements, which is RX * nx only when Mx = 2 nx)
   const size_t xi_maxc = (size_t)RX * (g.Mx / 2);
   const size_t smxi = smx + (xi_staged(g.Mx, TX, sizeof(C)) ? 2 * xi_maxc * sizeof(C) : 0);
   size_t smy = std::max((size_t)g.My * tile_stride(RY, TY, sizeof(C)), (size_t)RY * P.lsy) * sizeof(C);
-  // tensor tiles for the 256-point y passes (FP32, five-pass B layout): the
-  // slab as rows of n_z; the tile needs 32 KB at a 1024-byte boundary
+  // tensor tiles of the x and y passes (FP32, five-pass B layout): A as rows of
+  // n_y, the slab as rows of n_z
   P.tma = 0;
   P.tma_x = 0;
   if constexpr (sizeof(T) == 4) {
-    // the same for A (rows of n_y) in the 256-point x passes
-    if (E.use_tma && (g.Mx == 256 || g.Mx == 512) && RX == TMA_COLS && E.d_err &&
-        encode_b_map(&P.tmA, E.zhat, (size_t)E.zcap * 3 * g.nz * g.Mx, g.ny, P.lda))
+    if (E.use_tma && tma_length(g.Mx, sizeof(C)) && E.d_err &&
+        encode_b_map(&P.tmA, E.zhat, (size_t)E.zcap * 3 * g.nz * g.Mx, g.ny, P.lda, g.Mx))
       P.tma_x = 1;
-    if (E.use_tma && (g.My == 256 || g.My == 512) && RY == TMA_COLS && E.d_err &&
-        encode_b_map(&P.tmB, E.slab, (size_t)E.slab_nr * 3 * E.slab_B * g.My, g.nz, P.ldb)) {
+    if (E.use_tma && tma_length(g.My, sizeof(C)) && E.d_err &&
+        encode_b_map(&P.tmB, E.slab, (size_t)E.slab_nr * 3 * E.slab_B * g.My, g.nz, P.ldb, g.My)) {
       P.tma = 1;
-      smy = std::max(smy, (size_t)(g.My / TMA_ROWS) * TMA_TILE_BYTES + 1024);
+      smy = std::max(smy, tma_tile_bytes(g.My, RY) + 1024);
     }
   }
   // ZG3: FFT scratch
