@@ -218,9 +218,12 @@ template <typename C> __device__ __forceinline__ C cmulc(C a, C w) {
 // (the upper half of the line) are zero and are not read.  PAIR: transpose
 // rows of stride E + 2 written with 128-bit stores (complex-float lines; the
 // line stride must come from line_stride(..., pair = true)).
+// SWAP (E = 16, T = 8, PAIR): `swap` is 8 on odd lines and 0 on even ones; odd
+// lines exchange the halves of their scratch rows, which lets lines lie T * 18
+// elements apart without bank conflicts (152 otherwise).
 template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN = false, bool PAIR = false, bool CONJW = false,
-          typename C>
-__device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)[E]) {
+          bool SWAP = false, typename C>
+__device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)[E], int swap = 0) {
   constexpr int M = E / T;
   static_assert(M * T == E && M >= 1, "E must be a multiple of T");
   if constexpr (HALF_IN) dftr_h<E, DIR>(v); else dftr<E, DIR>(v);
@@ -228,10 +231,13 @@ __device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)
   for (int p = 1; p < E; ++p) v[p] = CONJW ? cmulc(v[p], w[p]) : cmul(v[p], w[p]);
   constexpr bool P2 = PAIR && sizeof(C) == 8;
   constexpr int RS = row_stride<E, P2>();
+  static_assert(!SWAP || (E == 16 && T == 8 && P2), "halves of 8 elements");
+  C* const lo = SWAP ? sl + swap : sl;  // elements p < 8 of a scratch row
+  C* const hi = SWAP ? sl - swap : sl;
   if constexpr (P2) {
 #pragma unroll
     for (int p = 0; p < E; p += 2)
-      *reinterpret_cast<float4*>(sl + t * RS + p) = make_float4(v[p].x, v[p].y, v[p + 1].x, v[p + 1].y);
+      *reinterpret_cast<float4*>((p < 8 ? lo : hi) + t * RS + p) = make_float4(v[p].x, v[p].y, v[p + 1].x, v[p + 1].y);
   } else {
 #pragma unroll
     for (int p = 0; p < E; ++p) sl[t * RS + p] = v[p];
@@ -241,7 +247,7 @@ __device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)
   for (int j = 0; j < M; ++j) {
     C u[T];
 #pragma unroll
-    for (int s = 0; s < T; ++s) u[s] = sl[s * RS + t + T * j];
+    for (int s = 0; s < T; ++s) u[s] = (j == 0 ? lo : hi)[s * RS + t + T * j];
     dftr<T, DIR>(u);
 #pragma unroll
     for (int q = 0; q < T; ++q) v[j + M * q] = u[q];

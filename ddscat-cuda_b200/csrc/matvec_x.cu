@@ -733,14 +733,17 @@ __device__ __forceinline__ void zg3_green_s(const C* rec, int t, C (&v)[3][E]) {
 
 // Row buffer of a line: N/2 elements.  The lines of a half-warp read different
 // banks: with TT = 8 the odd lines exchange neighbouring groups of 8 elements
-// (padding instead would leave 2 blocks per SM at N = 128: three need
-// (18.0 + 48.8 + 8 + 1) KB each of the SM's 228), with TT = 4 lines are 4
-// elements apart.
+// and the halves of their FFT scratch rows (padding either would leave 2
+// blocks per SM at N = 128: three need 18.0 + 48.8 + 8 + 1 KB each of the SM's
+// 228; 64^3, 8 RHS: 0.0426 against 0.0451 ms per RHS-MATVEC), with TT = 4 lines
+// are 4 elements apart.
 template <int N> struct ZRow {
   static constexpr int STRIDE = N / 2 + (XShape<N>::TT == 4 ? 4 : 0);
   static constexpr int PAIRS = (N / 4 + XShape<N>::TT - 1) / XShape<N>::TT;  // 16-byte copies per thread and row
   // exchanged groups of the odd lines (N/2 is a multiple of 16)
   static constexpr int SWAP = XShape<N>::TT == 8 && N % 32 == 0 ? 8 : 0;
+  // line stride of the FFT scratch where it is not the host's line_stride
+  static constexpr int SCRATCH = XShape<N>::TT == 8 && XShape<N>::E == 16 ? 8 * 18 : 0;
 };
 
 template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(XParams<T> P) {
@@ -752,8 +755,11 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
   static_assert(Z3Shape<N>::OK && RZ * TT == 128 && sizeof(C) == 8, "kx_zg3r: FP32, 128-thread blocks");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
-  C* my = reinterpret_cast<C*>(smem_raw) + (size_t)l * P.lsz;
-  C* gs = reinterpret_cast<C*>(smem_raw) + (size_t)RZ * P.lsz;  // [RZ][N/2+1][6]
+  // line scratch: at 16 elements x 8 threads lines lie T * 18 apart (ZRow::SCRATCH)
+  constexpr bool SW = ZRow<N>::SCRATCH != 0;
+  const int lss = SW ? ZRow<N>::SCRATCH : P.lsz, fswap = SW && (l & 1) ? 8 : 0;
+  C* my = reinterpret_cast<C*>(smem_raw) + (size_t)l * lss;
+  C* gs = reinterpret_cast<C*>(smem_raw) + (size_t)RZ * lss;  // [RZ][N/2+1][6]
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.x * RZ + l;
   const bool live = p < nlines;
@@ -822,7 +828,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
       __syncwarp();  // the buffer is read before the next row overwrites it
       if (c < 2) fetch(rb, c + 1);
       else if (nrb < rb1) fetch(nrb, 0);
-      line_fft_w<E, TT, +1, false, true, S_::PAIR>(v[c], my, t, w);
+      line_fft_w<E, TT, +1, false, true, S_::PAIR, false, SW>(v[c], my, t, w, fswap);
     }
     if (!staged) {
       __syncthreads();  // every thread's Green copies have landed (waited for at c = 1)
@@ -830,7 +836,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
     }
     if (live) zg3_green_s<N, TT, E>(gs + (size_t)l * LREC, t, v);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) line_fft_w<E, TT, -1, false, false, S_::PAIR, true>(v[c], my, t, w);
+    for (int c = 0; c < 3; ++c) line_fft_w<E, TT, -1, false, false, S_::PAIR, true, SW>(v[c], my, t, w, fswap);
     if (live) {
       C* row = P.B + (size_t)rb * 3 * cs + (size_t)p * P.ldb;
 #pragma unroll
@@ -1506,7 +1512,8 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   // ZG3R (Green lines staged once per block and reused for a chunk of RHS):
   // IPBC=0, batches of at least 4 RHS (DDSCAT_B200_NOZG3R=1 keeps ZG3)
   const void* fzg3r = fzg3 && g.ipbc == 0 && !env_flag("DDSCAT_B200_NOZG3R") ? xkernel<T>(XPass::ZG3R, g.Mz) : nullptr;
-  const size_t smzr = smz + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ == 4 ? 4 : 0)) * sizeof(C);
+  const int lszr = g.Mz == 128 ? 8 * 18 : P.lsz;  // ZRow::SCRATCH
+  const size_t smzr = ((size_t)RZ3 * lszr) * sizeof(C) + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ == 4 ? 4 : 0)) * sizeof(C);
   const void* fxf = xkernel<T>(XPass::XF, g.Mx);
   const void* fyf = xkernel<T>(XPass::YF, g.My);
   const void* fzg = xkernel<T>(XPass::ZG, g.Mz);
