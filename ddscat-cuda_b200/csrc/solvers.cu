@@ -236,6 +236,28 @@ __global__ void k_dq_vw(int n, C* vt, C* wt, const C* ap, const C* q, const DQSt
     wt[i] = dq_lin(wt[i], c5, q[i], one);
   }
 }
+// f(elements of the K vectors) over a grid-stride loop with two elements per
+// thread and round, all of a round's loads issued before its sums: on large
+// grids (128^3: 3.3 M elements) one in flight leaves the sums short of the copy
+// rate.
+template <int K, typename C, typename F> __device__ __forceinline__ void sum_loop(int n, const C* const (&v)[K], F f) {
+  const int st = gridDim.x * blockDim.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + st < n; i += 2 * st) {
+    C a[K], b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) { a[k] = v[k][i]; b[k] = v[k][i + st]; }
+    f(a);
+    f(b);
+  }
+  if (i < n) {
+    C a[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) a[k] = v[k][i];
+    f(a);
+  }
+}
+
 // the four inner products of an iteration, then the scalar recurrence
 template <typename C>
 __global__ void __launch_bounds__(RED_THREADS) k_dq_dots(int n, const C* vt, const C* wt, const C* atw, DQState* S,
@@ -243,15 +265,16 @@ __global__ void __launch_bounds__(RED_THREADS) k_dq_dots(int n, const C* vt, con
   double2 acc[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) acc[q] = make_double2(0.0, 0.0);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double2 v = to_d(vt[i]), w = to_d(wt[i]), a = to_d(atw[i]);
+  const C* const src[3] = {vt, wt, atw};
+  sum_loop<3>(n, src, [&](const C (&e)[3]) {
+    const double2 v = to_d(e[0]), w = to_d(e[1]), a = to_d(e[2]);
     acc[0].x += v.x * v.x + v.y * v.y;
     acc[1].x += w.x * w.x + w.y * w.y;
     acc[2].x += v.x * w.x - v.y * w.y;
     acc[2].y += v.x * w.y + v.y * w.x;
     acc[3].x += v.x * a.x - v.y * a.y;
     acc[3].y += v.x * a.y + v.y * a.x;
-  }
+  });
   reduce_tail<4>(acc, 4, part, out, cnt, [=](const double2* o) { dq_recur(S, o); });
 }
 // the d/s/x/r step with |r|^2 and the residual
@@ -262,12 +285,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_dq_dsxr(int n, C* d, C* s, C* x
   const double2 th = S->co[6], ka = S->co[7], one = make_double2(1.0, 0.0), mone = make_double2(-1.0, 0.0);
   double2 acc[1] = {make_double2(0.0, 0.0)};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const C dn = dq_lin(d[i], th, p[i], ka);
-    const C sn = dq_lin(s[i], th, ap[i], ka);
+    const C dv = d[i], pv = p[i], sv = s[i], av = ap[i], xv = x[i], rv = r[i];  // all loads before the stores
+    const C dn = dq_lin(dv, th, pv, ka);
+    const C sn = dq_lin(sv, th, av, ka);
     d[i] = dn;
     s[i] = sn;
-    x[i] = dq_lin(x[i], one, dn, one);
-    const C rn = dq_lin(r[i], one, sn, mone);
+    x[i] = dq_lin(xv, one, dn, one);
+    const C rn = dq_lin(rv, one, sn, mone);
     r[i] = rn;
     const double2 e = to_d(rn);
     acc[0].x += e.x * e.x + e.y * e.y;
@@ -276,7 +300,15 @@ __global__ void __launch_bounds__(RED_THREADS) k_dq_dsxr(int n, C* d, C* s, C* x
 }
 
 // blocks of a kernel with a sum: one resident wave, within the partials buffer
-template <typename T> static unsigned sum_grid(const VecOps<T>& o, int n, int per_sm) {
+// (a grid-stride loop over one and a half waves takes as long as over two:
+// PBCGS2 at 128^3 2.05 -> 1.74 ms per iteration with this and loads ahead of the
+// stores)
+template <typename T> static unsigned sum_grid(const VecOps<T>& o, int n, const void* kernel) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RED_THREADS, 0) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 2;
+  }
   return (unsigned)std::min<size_t>(ceil_div((size_t)std::max(n, 1), RED_THREADS),
                                     (size_t)std::min(o.nblocks, 148 * per_sm));
 }
@@ -438,11 +470,12 @@ template <typename C>
 __global__ void __launch_bounds__(RED_THREADS) k_dp_dot(int n, const C* rr, const C* v, int step, DPState* S,
                                                         double2* part, double2* out, unsigned* cnt) {
   double2 acc[1] = {make_double2(0.0, 0.0)};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double2 a = to_d(rr[i]), b = to_d(v[i]);
+  const C* const src[2] = {rr, v};
+  sum_loop<2>(n, src, [&](const C (&e)[2]) {
+    const double2 a = to_d(e[0]), b = to_d(e[1]);
     acc[0].x += a.x * b.x + a.y * b.y;
     acc[0].y += a.x * b.y - a.y * b.x;
-  }
+  });
   reduce_tail<1>(acc, 1, part, out, cnt, [=](const double2* o) {
     if (step == 2) dp_sigma(S, o);
     else dp_rho(S, o, step == 0);
@@ -454,8 +487,10 @@ __global__ void k_dp_u(int n, C* u0, const C* r0, C* u1, const C* r1, const DPSt
   if (S->status) return;
   const double2 mb = S->co[0], one = make_double2(1.0, 0.0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    u0[i] = dq_lin(u0[i], mb, r0[i], one);
-    if (K > 1) u1[i] = dq_lin(u1[i], mb, r1[i], one);
+    const C b0 = u0[i], a0 = r0[i];
+    const C b1 = K > 1 ? u1[i] : mk<C>(0, 0), a1 = K > 1 ? r1[i] : mk<C>(0, 0);
+    u0[i] = dq_lin(b0, mb, a0, one);
+    if (K > 1) u1[i] = dq_lin(b1, mb, a1, one);
   }
 }
 // X += alpha u0, r_j -= alpha u_{j+1} (j < K), and |r_0|
@@ -467,10 +502,12 @@ __global__ void __launch_bounds__(RED_THREADS) k_dp_xr(int n, C* X, const C* u0,
   const double2 al = S->co[1], mal = S->co[2], one = make_double2(1.0, 0.0);
   double2 acc[1] = {make_double2(0.0, 0.0)};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    X[i] = dq_lin(X[i], one, u0[i], al);
-    const C rn = dq_lin(r0[i], one, u1[i], mal);
+    const C xv = X[i], b0 = u0[i], a0 = r0[i], b1 = u1[i];  // all loads before the stores
+    const C a1 = K > 1 ? r1[i] : mk<C>(0, 0), b2 = K > 1 ? u2[i] : mk<C>(0, 0);
+    X[i] = dq_lin(xv, one, b0, al);
+    const C rn = dq_lin(a0, one, b1, mal);
     r0[i] = rn;
-    if (K > 1) r1[i] = dq_lin(r1[i], one, u2[i], mal);
+    if (K > 1) r1[i] = dq_lin(a1, one, b2, mal);
     const double2 e = to_d(rn);
     acc[0].x += e.x * e.x + e.y * e.y;
   }
@@ -484,8 +521,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_dp_gram(int n, const C* r0, con
   double2 acc[6];
 #pragma unroll
   for (int q = 0; q < 6; ++q) acc[q] = make_double2(0.0, 0.0);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double2 v[3] = {to_d(r0[i]), to_d(r1[i]), to_d(r2[i])};
+  const C* const src[3] = {r0, r1, r2};
+  sum_loop<3>(n, src, [&](const C (&e)[3]) {
+    const double2 v[3] = {to_d(e[0]), to_d(e[1]), to_d(e[2])};
     int q = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
@@ -494,7 +532,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_dp_gram(int n, const C* r0, con
         acc[q].x += v[a].x * v[b].x + v[a].y * v[b].y;
         acc[q].y += v[a].x * v[b].y - v[a].y * v[b].x;
       }
-  }
+  });
   reduce_tail<6>(acc, 6, part, out, cnt, [=](const double2* o) { dp_gram(S, o); });
 }
 // u0 -= Y1 u1 + Y2 u2 ; X += Y1 r0 + Y2 r1 ; r0 -= Y1 r1 + Y2 r2
@@ -502,13 +540,14 @@ template <typename C>
 __global__ void k_dp_poly(int n, C* u0, const C* u1, const C* u2, C* X, C* r0, const C* r1, const C* r2,
                           const DPState* S) {
   if (S->status) return;
-  const double2 one = make_double2(1.0, 0.0);
+  const double2 one = make_double2(1.0, 0.0), y1 = S->y1, y2 = S->y2, my1 = S->my1, my2 = S->my2;
   auto lin3 = [&](C d, C a, double2 za, C b, double2 zb) { return cadd(cadd(zmulv(one, d), zmulv(za, a)), zmulv(zb, b)); };
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const C a0 = r0[i], a1 = r1[i];
-    u0[i] = lin3(u0[i], u1[i], S->my1, u2[i], S->my2);
-    X[i] = lin3(X[i], a0, S->y1, a1, S->y2);
-    r0[i] = lin3(a0, a1, S->my1, r2[i], S->my2);
+    const C b0 = u0[i], b1 = u1[i], b2 = u2[i], xv = X[i], a2 = r2[i];
+    u0[i] = lin3(b0, b1, my1, b2, my2);
+    X[i] = lin3(xv, a0, y1, a1, y2);
+    r0[i] = lin3(a0, a1, my1, a2, my2);
   }
 }
 
@@ -556,7 +595,9 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
   double resid = S.resid;
   const int n = c.n;
   const VecOps<T>& vo = *io.ops;
-  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, 8), gr = sum_grid(vo, n, 6), gg = sum_grid(vo, n, 3);
+  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, (const void*)k_dp_dot<C>),
+                 gg = sum_grid(vo, n, (const void*)k_dp_gram<C>), gr1 = sum_grid(vo, n, (const void*)k_dp_xr<C, 1>),
+                 gr2 = sum_grid(vo, n, (const void*)k_dp_xr<C, 2>);
   auto dot = [&](const C* v, int step) {
     k_dp_dot<C><<<gd, RED_THREADS, 0, c.st()>>>(n, rr, v, step, dS, vo.d_red, vo.d_out, vo.d_count);
   };
@@ -569,14 +610,14 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
       k_dp_u<C, 1><<<gb, 256, 0, c.st()>>>(n, u[0], r[0], nullptr, nullptr, dS);
       MV(u[0], u[1], 96);
       dot(u[1], 2);
-      k_dp_xr<C, 1><<<gr, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], nullptr, nullptr, dS, vo.d_red, vo.d_out,
+      k_dp_xr<C, 1><<<gr1, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], nullptr, nullptr, dS, vo.d_red, vo.d_out,
                                                     vo.d_count);
       MV(r[0], r[1], 99);
       dot(r[1], 1);
       k_dp_u<C, 2><<<gb, 256, 0, c.st()>>>(n, u[0], r[0], u[1], r[1], dS);
       MV(u[1], u[2], 96);
       dot(u[2], 2);
-      k_dp_xr<C, 2><<<gr, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], r[1], u[2], dS, vo.d_red, vo.d_out,
+      k_dp_xr<C, 2><<<gr2, RED_THREADS, 0, c.st()>>>(n, X, u[0], r[0], u[1], r[1], u[2], dS, vo.d_red, vo.d_out,
                                                     vo.d_count);
       MV(r[1], r[2], 99);
       k_dp_gram<C><<<gg, RED_THREADS, 0, c.st()>>>(n, r[0], r[1], r[2], dS, vo.d_red, vo.d_out, vo.d_count);
@@ -718,7 +759,8 @@ template <typename T> int solve_qmrccg(SolveIO<T>& io) {
   CK(55);
   const int n = c.n;
   const VecOps<T>& vo = *io.ops;
-  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, 4), gr = sum_grid(vo, n, 6);
+  const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, (const void*)k_dq_dots<C>),
+                 gr = sum_grid(vo, n, (const void*)k_dq_dsxr<C>);
   IterGraph ig;
   int it = 0;
   while (it < io.maxit && resid > io.tol) {
