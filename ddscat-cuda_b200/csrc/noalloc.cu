@@ -16,13 +16,14 @@
 //    pipeline 3*nz*Mx*ny + 3*My*nz*Mx complex floats (ny and nz rounded up to
 //    even), with Mx, My the padded FFT lengths the prepare chose (2*nx, 2*ny,
 //    or the next register-FFT length for a padded axis), 3*Mz*ny*nx +
-//    3*ny*Mx*Mz on the z-first one.  With M = 2n that is 18*NAT, so targets
-//    with NAT = NX*NY*NZ <= 349,525 sites (e.g. 64^3) fit.  A finite target of
-//    even sides padded to at most 2.5 times the points of the 2n grid must fit
-//    whole (72x72x64, NAT = 331,776, pads 144 to 192 and needs 9.7 M); ragged
-//    and periodic targets within the NAT limit hold as many planes of the
-//    spectrum at a time as fit.  Targets beyond that are rejected with status
-//    601 before any launch.
+//    3*ny*Mx*Mz on the z-first one; where that is too much, as many planes of
+//    the spectrum at a time as fit.
+//  * Targets are taken up to NAT = NX*NY*NZ = 349,525 sites (18*NAT elements on
+//    the 2n grid; e.g. 64^3), with one exception (admission_elems): a finite
+//    target of even sides whose lengths would pad to 2^k or 3*2^k with at most
+//    2.5 times the points of the 2n grid counts with that padded grid (72x72x64,
+//    NAT = 331,776: 144 pads to 192, 9.7 M elements) unless its real grid fits
+//    whole.  Targets beyond that are rejected with status 601 before any launch.
 //  * The array is part of the library's device image: every GPU that loads
 //    the library holds these 48 MiB until the process exits.
 //  * Every call on a device uses the same array and it keeps the last call's
@@ -73,6 +74,26 @@ static int noalloc_scratch(int dev, float2** out) {
   return 0;
 }
 
+// Scratch elements that decide whether a target is taken when its grid does not
+// fit whole.  Callers go by the status (601: use ddscat_cuda_apply_f32), so the
+// set of targets does not follow the list of FFT lengths: it is the one of the
+// lengths 2^k and 3*2^k, whatever lengths were added since.  66^3, for one, ran on
+// its 132-point grid (5.2 M elements, taken) before 160 points were a length;
+// padded to 160 it needs 7.2 M and runs in two plane batches.
+static size_t admission_elems(const Geometry& g) {
+  size_t mx = 2 * (size_t)g.nx, my = 2 * (size_t)g.ny, mz = 2 * (size_t)g.nz;
+  if (g.ipbc == 0 && g.padded() && !((g.nx | g.ny | g.nz) & 1)) {
+    auto length = [](size_t m) -> size_t {
+      for (size_t l : {16, 32, 48, 64, 96, 128, 192, 256, 512})
+        if (l >= m) return l;
+      return 0;
+    };
+    const size_t lx = length(mx), ly = length(my), lz = length(mz);
+    if (lx && ly && lz && (double)(lx * ly * lz) <= 2.5 * (double)(mx * my * mz)) { mx = lx; my = ly; mz = lz; }
+  }
+  return 3 * (size_t)g.nz * mx * g.ny + 3 * my * (size_t)g.nz * mx;
+}
+
 }  // namespace ddb
 
 using namespace ddb;
@@ -108,12 +129,7 @@ extern "C" DDSCAT_CUDA_API int ddscat_b200_apply_noalloc_f32(int cwhat, const vo
   const int planes = e.xpipe ? g.Mx : g.Mz;
   const size_t room = (size_t)NOALLOC_SCRATCH_ELEMS - std::min(za, (size_t)NOALLOC_SCRATCH_ELEMS);
   const int fit = (int)std::min<size_t>((size_t)planes, room / plane);
-  // Finite targets of even sides padded to at most 2.5 times the points of the
-  // 2n grid hold every plane at once or are refused.  For the others the NAT
-  // limit alone decides: their middle stage runs in as many plane batches as
-  // it takes.
-  const bool whole = g.ipbc == 0 && !((g.nx | g.ny | g.nz) & 1) && (double)g.ngrid() <= 2.5 * 8.0 * (double)g.nat;
-  if (fit < (whole ? planes : 1)) {
+  if (fit < planes && (fit < 1 || admission_elems(g) > NOALLOC_SCRATCH_ELEMS)) {
     char msg[240];
     std::snprintf(msg, sizeof(msg),
                   "the padded FFT grid of this target needs %zu complex floats of scratch; the fixed scratch (48 MiB) "

@@ -107,10 +107,11 @@ DDSCAT_CUDA_API int ddscat_b200_residual_f64(int nrhs, const void *b, const void
  * scratch is a fixed 48 MiB array (6,291,456 complex floats) in the library's
  * device image; every GPU that loads the library holds it until exit.  It
  * holds 3*nz*Mx*ny + 3*My*nz*Mx complex floats for the padded FFT lengths Mx,
- * My of the prepared grid (18*NAT when M = 2n: targets up to NAT = 349,525
- * sites, e.g. 64^3; finite targets of even sides padded to at most 2.5 times
- * the points of the 2n grid must fit whole, others within the NAT limit run
- * their middle stage in plane batches), else the call
+ * My of the prepared grid (18*NAT when M = 2n), or as many planes of the middle
+ * stage at a time as fit.  Targets of up to NAT = 349,525 sites (e.g. 64^3) are
+ * taken; a finite target of even sides whose lengths pad to 2^k or 3*2^k with at
+ * most 2.5 times the points of the 2n grid counts with that padded grid (not
+ * 72x72x64) unless its real grid fits whole; else the call
  * returns 601.  All calls share the array and it keeps the last call's
  * contents (nothing needs to start at zero); calls that overlap on the GPU
  * race, so serialise them.  The first call on a device (and the first after

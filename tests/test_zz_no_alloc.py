@@ -103,12 +103,74 @@ def test_apply_noalloc_in_cuda_graph(dims):
     dda.release()
 
 
+def _taken(dims):
+    """Whether the entry point takes a finite target: up to 349,525 sites, but a
+    box of even sides counts at its next lengths 2^k (16..512) or 3 * 2^k
+    (48..192) where those have at most 2.5 times the points of the 2n grid."""
+    n = np.array(dims, dtype=np.int64)
+    if n.prod() > 6291456 // 18:
+        return False
+    m = 2 * n
+    if not (n % 2).any():
+        pad = [next((v for v in (16, 32, 48, 64, 96, 128, 192, 256, 512) if v >= a), 0) for a in m]
+        if min(pad) and np.prod(pad) <= 2.5 * m.prod():
+            m = np.array(pad)
+    return bool(3 * n[2] * m[0] * n[1] + 3 * m[1] * n[2] * m[0] <= 6291456)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(66, 66, 66), (70, 70, 70), (66, 66, 80), (74, 70, 66)])
+def test_apply_noalloc_even_boxes_in_plane_batches(dims):
+    """Boxes of even sides whose 2n grid fits the scratch and whose grid padded to
+    160 points does not: taken, the middle stage in plane batches."""
+    torch = pytest.importorskip("torch")
+    assert _taken(dims)
+    iocc, ak, x, _, adia, aoff = _inputs(dims, 5)
+    dda = D.DDA()
+    dda.prepare_green(*dims, iocc, ak)
+    t = [torch.from_numpy(a).cuda() for a in (x, adia, aoff)]
+    y = torch.zeros_like(t[0])
+    p = [ct.c_void_p(v.data_ptr()) for v in (t[0], y, t[1], t[2])]
+    for cw in "NC":
+        assert dda.lib.ddscat_b200_apply_noalloc_f32(ord(cw), *p, None) == 0
+        torch.cuda.synchronize()
+        ref = dda.apply(x, adia, aoff, cw)
+        assert np.linalg.norm(y.cpu().numpy() - ref) <= RTOL * np.linalg.norm(ref)
+    dda.release()
+
+
+@pytest.mark.gpu
+def test_apply_noalloc_takes_what_the_rule_says():
+    """Even boxes just below the NAT limit, on both sides of the rule of _taken;
+    a box it refuses may be taken where its real grid fits whole."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(12)
+    dda = D.DDA()
+    seen = {True: 0, False: 0}
+    while min(seen.values()) < 8:
+        dims = tuple(int(v) for v in 2 * rng.integers(16, 71, size=3))
+        nat = int(np.prod(dims))
+        if not 250_000 < nat <= 349_525 or seen[_taken(dims)] >= 12:
+            continue
+        seen[_taken(dims)] += 1
+        dda.prepare_green(*dims, np.ones(nat, dtype=np.int16), (0.3, 0.0, 0.0))
+        t = torch.zeros(3 * nat, dtype=torch.complex64, device="cuda")
+        y = torch.empty_like(t)
+        p = ct.c_void_p(t.data_ptr())
+        rc = dda.lib.ddscat_b200_apply_noalloc_f32(ord("N"), p, ct.c_void_p(y.data_ptr()), p, None, None)
+        torch.cuda.synchronize()
+        assert rc == 0 if _taken(dims) else rc in (0, 601), dims
+    dda.release()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(72, 72, 72), (72, 72, 64)])
 def test_apply_noalloc_rejects_large_target(dims):
     """72^3 has NAT = 373,248 > 349,525; 72x72x64 (NAT = 331,776) is under that
-    bound but its x and y axes are padded from 144 to 192, so its scratch
-    (9.7 M complex floats) exceeds the fixed 6.29 M as well."""
+    bound, but a box of even sides counts at its next 2^k or 3 * 2^k lengths: x
+    and y from 144 to 192, 9.7 M complex floats, more than the fixed 6.29 M, and
+    its real grid (160 points, 7.1 M) does not fit whole either."""
+    assert not _taken(dims)
     torch = pytest.importorskip("torch")
     nat = int(np.prod(dims))
     dda = D.DDA()
