@@ -103,7 +103,7 @@ struct F64State {
 };
 static F64State f64;
 static void release_f64() {
-  if (f64.ready) {
+  if (f64.eng.d_err) {  // init_geometry's first allocation: a set-up that failed later ends here too
     cudaStreamSynchronize(f64.eng.stream);
     dev_free(f64.x); dev_free(f64.y); dev_free(f64.b); dev_free(f64.ad); dev_free(f64.ao);
     f64.ops.release();
@@ -129,13 +129,14 @@ static void release_b64() {
 static void release_state() {
   // callers may still run the operator on streams of their own (the
   // allocation-free MATVEC): their work ends before its buffers are reused
-  if (s.ready || s.eng.green) cudaDeviceSynchronize();
+  const bool held = s.eng.d_err != nullptr;  // init_geometry's first allocation: also after a prepare that failed
+  if (held) cudaDeviceSynchronize();
   release_batch();
   release_b64();
   release_f64();
   delete[] s.h_iocc;
   s.h_iocc = nullptr;
-  if (s.ready || s.eng.green) {
+  if (held) {
     dev_free(s.d_xf); dev_free(s.d_yf); dev_free(s.d_adia); dev_free(s.d_aoff);
     dev_free(s.d_b); dev_free(s.d_sx); dev_free(s.d_sy); dev_free(s.d_work);
     dev_free(s.d_adia_c); dev_free(s.d_aoff_c);

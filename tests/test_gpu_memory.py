@@ -37,6 +37,27 @@ def test_reused_blocks_give_the_same_results():
 
 
 @pytest.mark.gpu
+def test_refused_prepares_keep_no_memory():
+    """A prepare whose NAT0 is not the occupied count (208) has built its index
+    maps, 10 bytes per site, when it finds out; 60 of them at 96^3 (530 MB) return
+    everything but the bounded reuse lists, and those with the release."""
+    torch = pytest.importorskip("torch")
+    n = 96
+    iocc = np.ones(n ** 3, dtype=np.int16)
+    dda = D.DDA()
+    dda.prepare_green(8, 8, 8, np.ones(512, dtype=np.int16), (0.3, 0.0, 0.0))  # one-time set-up
+    dda.release()
+    free0 = torch.cuda.mem_get_info()[0]
+    for _ in range(60):
+        with pytest.raises(D.DDSCATError) as err:
+            dda.prepare_green(n, n, n, iocc, (0.3, 0.0, 0.0), nat0=n ** 3 - 1)
+        assert err.value.code == 208
+    assert torch.cuda.mem_get_info()[0] >= free0 - (64 << 20)
+    dda.release()
+    assert torch.cuda.mem_get_info()[0] >= free0 - (4 << 20)
+
+
+@pytest.mark.gpu
 def test_concurrent_targets_do_not_share_blocks():
     probs = [targets.make_problem(n, m=1.4 + 0.03j, x=1.5) for n in (8, 10, 12, 14, 16, 9)]
 
