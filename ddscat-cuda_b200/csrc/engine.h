@@ -58,6 +58,25 @@ struct Geometry {
   int ldy() const { return (ny + 1) & ~1; }
   int ldz() const { return (nz + 1) & ~1; }
   bool padded() const { return Mx != 2 * nx || My != 2 * ny || Mz != 2 * nz; }
+  // The next lengths 2^k (16..512) or 3*2^k (48..192) of the target, where they
+  // are 2n already or, for finite targets of even sides, have at most 2.5 times
+  // the points of the 2n grid; false for every other target.  Two rules refer to
+  // these lengths and not to the list the pipeline runs (which has more): which
+  // targets plain FP32 line transforms serve (Engine::cx), and which the
+  // allocation-free MATVEC takes.
+  bool base_lengths(int m[3]) const {
+    const int n2[3] = {2 * nx, 2 * ny, 2 * nz};
+    bool exact = true;
+    for (int a = 0; a < 3; ++a) {
+      m[a] = 0;
+      for (int l : {512, 256, 192, 128, 96, 64, 48, 32, 16})
+        if (l >= n2[a]) m[a] = l;
+      exact = exact && m[a] == n2[a];
+    }
+    if (exact) return true;
+    if (ipbc || ((nx | ny | nz) & 1) || !m[0] || !m[1] || !m[2]) return false;
+    return (double)m[0] * m[1] * m[2] <= 2.5 * ((double)n2[0] * n2[1] * n2[2]);
+  }
   size_t green_count() const { return ipbc == 0 ? 6 * octant() : 6 * ngrid(); }
 };
 
@@ -98,6 +117,9 @@ template <typename T> struct Engine {
   Geometry g;
   FftPlan px, py, pz;
   C *twx = nullptr, *twy = nullptr, *twz = nullptr;
+  // twiddles as hi + lo in thread order (line_fft_acc), for targets that left the
+  // generic transforms for the register ones (set in init_geometry); else null
+  float4 *cx = nullptr, *cy = nullptr, *cz = nullptr;
   C* green = nullptr;
   int* occ = nullptr;      // [nat0]
   int* inv = nullptr;      // [nat], -1 for vacuum

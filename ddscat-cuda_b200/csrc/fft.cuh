@@ -43,6 +43,31 @@ inline FftPlan make_fft_plan(int n) {
 }
 
 // ---- butterflies: in-register R-point DFTs, W = exp(dir*2*pi*i/R) ---------
+// CC (FP32 only): constants are applied as hi + lo, so they are good to 48 bits
+// and only the roundings of the sums and products are left.
+// c * s
+template <bool CC, typename R> DDB_HD R kmul(double c, R s) {
+  if constexpr (CC && sizeof(R) == 4) {
+    const float hi = (float)c, lo = (float)(c - (double)hi);
+    return fmaf(s, hi, s * lo);
+  } else {
+    return (R)c * s;
+  }
+}
+// c * s + a
+template <bool CC, typename R> DDB_HD R kfma(double c, R s, R a) {
+  if constexpr (CC && sizeof(R) == 4) {
+    const float hi = (float)c, lo = (float)(c - (double)hi);
+    return fmaf(s, hi, fmaf(s, lo, a));
+  } else {
+    return a + (R)c * s;
+  }
+}
+// a * w, w = (hi.x + lo.x) + i (hi.y + lo.y)
+DDB_HD float2 cmul_hl(float2 a, float2 hi, float2 lo) {
+  return make_float2(fmaf(a.x, hi.x, fmaf(-a.y, hi.y, fmaf(-a.y, lo.y, a.x * lo.x))),
+                     fmaf(a.x, hi.y, fmaf(a.y, hi.x, fmaf(a.y, lo.x, a.x * lo.y))));
+}
 template <int DIR, typename C> __device__ __forceinline__ void bfly2(C* v) {
   C a = v[0], b = v[1];
   v[0] = vadd(a, b);
@@ -57,15 +82,17 @@ template <int DIR, typename C> __device__ __forceinline__ void bfly4(C* v) {
   v[3] = subrot<DIR>(d02, t13);
 }
 // W8^1 * o and W8^3 * o, W8 = exp(DIR*2*pi*i/8) = (1 + DIR*i)/sqrt2
-template <int DIR, typename C> __device__ __forceinline__ C w8_1(C o) {
+template <int DIR, bool CC = false, typename C> __device__ __forceinline__ C w8_1(C o) {
   using R = decltype(o.x);
-  const R h = (R)0.70710678118654752440;
-  return DIR > 0 ? mk2<C>(h * (o.x - o.y), h * (o.y + o.x)) : mk2<C>(h * (o.x + o.y), h * (o.y - o.x));
+  const double h = 0.70710678118654752440;
+  return DIR > 0 ? mk2<C>(kmul<CC, R>(h, o.x - o.y), kmul<CC, R>(h, o.y + o.x))
+                 : mk2<C>(kmul<CC, R>(h, o.x + o.y), kmul<CC, R>(h, o.y - o.x));
 }
-template <int DIR, typename C> __device__ __forceinline__ C w8_3(C o) {
+template <int DIR, bool CC = false, typename C> __device__ __forceinline__ C w8_3(C o) {
   using R = decltype(o.x);
-  const R h = (R)0.70710678118654752440, hn = (R)-0.70710678118654752440;
-  return DIR > 0 ? mk2<C>(hn * (o.x + o.y), h * (o.x - o.y)) : mk2<C>(h * (o.y - o.x), hn * (o.x + o.y));
+  const double h = 0.70710678118654752440, hn = -0.70710678118654752440;
+  return DIR > 0 ? mk2<C>(kmul<CC, R>(hn, o.x + o.y), kmul<CC, R>(h, o.x - o.y))
+                 : mk2<C>(kmul<CC, R>(h, o.y - o.x), kmul<CC, R>(hn, o.x + o.y));
 }
 // DIR*i*o
 template <int DIR, typename C> __device__ __forceinline__ C rot4(C o) {
@@ -73,12 +100,12 @@ template <int DIR, typename C> __device__ __forceinline__ C rot4(C o) {
   const R m1 = (R)-1.0;
   return DIR > 0 ? mk2<C>(m1 * o.y, o.x) : mk2<C>(o.y, m1 * o.x);
 }
-template <int DIR, typename C> __device__ __forceinline__ void bfly8(C* v) {
+template <int DIR, bool CC = false, typename C> __device__ __forceinline__ void bfly8(C* v) {
   C e[4] = {v[0], v[2], v[4], v[6]};
   C o[4] = {v[1], v[3], v[5], v[7]};
   bfly4<DIR>(e);
   bfly4<DIR>(o);
-  const C t1 = w8_1<DIR>(o[1]), t3 = w8_3<DIR>(o[3]);
+  const C t1 = w8_1<DIR, CC>(o[1]), t3 = w8_3<DIR, CC>(o[3]);
   v[0] = vadd(e[0], o[0]);
   v[4] = vsub(e[0], o[0]);
   v[1] = vadd(e[1], t1);
@@ -88,30 +115,41 @@ template <int DIR, typename C> __device__ __forceinline__ void bfly8(C* v) {
   v[3] = vadd(e[3], t3);
   v[7] = vsub(e[3], t3);
 }
-template <int DIR, typename C> __device__ __forceinline__ void bfly3(C* v) {
+template <int DIR, bool CC = false, typename C> __device__ __forceinline__ void bfly3(C* v) {
   using R = decltype(v[0].x);
-  const R c = (R)-0.5, s = (R)(DIR * 0.86602540378443864676), ms = (R)(-DIR * 0.86602540378443864676);
+  const double s = DIR * 0.86602540378443864676, ms = -DIR * 0.86602540378443864676;
+  const R c = (R)-0.5;
   const C t = vadd(v[1], v[2]);
   const C d = vsub(v[1], v[2]);
   const C a = v[0];
   const C m = mk2<C>(a.x + c * t.x, a.y + c * t.y);
-  const C u = mk2<C>(ms * d.y, s * d.x);
+  const C u = mk2<C>(kmul<CC, R>(ms, d.y), kmul<CC, R>(s, d.x));
   v[0] = vadd(a, t);
   v[1] = vadd(m, u);
   v[2] = vsub(m, u);
 }
-template <int DIR, typename C> __device__ __forceinline__ void bfly5(C* v) {
+template <int DIR, bool CC = false, typename C> __device__ __forceinline__ void bfly5(C* v) {
   using R = decltype(v[0].x);
-  const R c1 = (R)0.30901699437494742410, c2 = (R)-0.80901699437494742410;
-  const R s1 = (R)(DIR * 0.95105651629515357212), s2 = (R)(DIR * 0.58778525229247312917);
+  const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;
+  const double s1 = DIR * 0.95105651629515357212, s2 = DIR * 0.58778525229247312917;
   C a = v[0];
   C t1 = cadd(v[1], v[4]), d1 = csub(v[1], v[4]);
   C t2 = cadd(v[2], v[3]), d2 = csub(v[2], v[3]);
-  C m1 = mk<C>((double)(a.x + c1 * t1.x + c2 * t2.x), (double)(a.y + c1 * t1.y + c2 * t2.y));
-  C m2 = mk<C>((double)(a.x + c2 * t1.x + c1 * t2.x), (double)(a.y + c2 * t1.y + c1 * t2.y));
-  // i*(s1 d1 + s2 d2) and i*(s2 d1 - s1 d2)
-  C u1 = mk<C>((double)(-(s1 * d1.y + s2 * d2.y)), (double)(s1 * d1.x + s2 * d2.x));
-  C u2 = mk<C>((double)(-(s2 * d1.y - s1 * d2.y)), (double)(s2 * d1.x - s1 * d2.x));
+  C m1, m2, u1, u2;
+  if constexpr (CC && sizeof(R) == 4) {
+    auto two = [](double p, R x, double q, R y, R z) { return kfma<true, R>(p, x, kfma<true, R>(q, y, z)); };
+    m1 = mk2<C>(two(c1, t1.x, c2, t2.x, a.x), two(c1, t1.y, c2, t2.y, a.y));
+    m2 = mk2<C>(two(c2, t1.x, c1, t2.x, a.x), two(c2, t1.y, c1, t2.y, a.y));
+    u1 = mk2<C>(-two(s1, d1.y, s2, d2.y, (R)0), two(s1, d1.x, s2, d2.x, (R)0));
+    u2 = mk2<C>(-two(s2, d1.y, -s1, d2.y, (R)0), two(s2, d1.x, -s1, d2.x, (R)0));
+  } else {
+    const R C1 = (R)c1, C2 = (R)c2, S1 = (R)s1, S2 = (R)s2;
+    m1 = mk<C>((double)(a.x + C1 * t1.x + C2 * t2.x), (double)(a.y + C1 * t1.y + C2 * t2.y));
+    m2 = mk<C>((double)(a.x + C2 * t1.x + C1 * t2.x), (double)(a.y + C2 * t1.y + C1 * t2.y));
+    // i*(s1 d1 + s2 d2) and i*(s2 d1 - s1 d2)
+    u1 = mk<C>((double)(-(S1 * d1.y + S2 * d2.y)), (double)(S1 * d1.x + S2 * d2.x));
+    u2 = mk<C>((double)(-(S2 * d1.y - S1 * d2.y)), (double)(S2 * d1.x - S1 * d2.x));
+  }
   v[0] = cadd(a, cadd(t1, t2));
   v[1] = cadd(m1, u1);
   v[4] = csub(m1, u1);

@@ -32,7 +32,7 @@ template <int K, int DIR, typename C> DDB_HD C wk(int m) {
 
 // x * W_K^m: the multiples of pi/4 are a rotation, a negation or the radix-8
 // forms (m is a compile-time constant after unrolling, so the branches fold)
-template <int K, int DIR, typename C> __device__ __forceinline__ C cmul_wk(C x, int m) {
+template <int K, int DIR, bool CC = false, typename C> __device__ __forceinline__ C cmul_wk(C x, int m) {
   const int q = (8 * m) % (8 * K);  // in units of 1/(8 K) of a turn
   using R = decltype(x.x);
   const R m1 = (R)-1.0;
@@ -40,28 +40,34 @@ template <int K, int DIR, typename C> __device__ __forceinline__ C cmul_wk(C x, 
   if (q == 4 * K) return mk2<C>(m1 * x.x, m1 * x.y);
   if (q == 2 * K) return rot4<DIR>(x);
   if (q == 6 * K) return rot4<-DIR>(x);
-  if (q == K) return w8_1<DIR>(x);
-  if (q == 3 * K) return w8_3<DIR>(x);
-  if (q == 5 * K) return w8_3<-DIR>(x);  // exp(5 i pi/4) = exp(-3 i pi/4)
-  if (q == 7 * K) return w8_1<-DIR>(x);  // exp(7 i pi/4) = exp(-i pi/4)
-  return cmul(x, wk<K, DIR, C>(m));
+  if (q == K) return w8_1<DIR, CC>(x);
+  if (q == 3 * K) return w8_3<DIR, CC>(x);
+  if (q == 5 * K) return w8_3<-DIR, CC>(x);  // exp(5 i pi/4) = exp(-3 i pi/4)
+  if (q == 7 * K) return w8_1<-DIR, CC>(x);  // exp(7 i pi/4) = exp(-i pi/4)
+  if constexpr (CC && sizeof(R) == 4) {
+    const double2 w = wk<K, DIR, double2>(m);
+    const float2 hi = from_d<float2>(w);
+    return cmul_hl(x, hi, make_float2((float)(w.x - (double)hi.x), (float)(w.y - (double)hi.y)));
+  } else {
+    return cmul(x, wk<K, DIR, C>(m));
+  }
 }
 
 // first factor of the four-step split K = K1 * K2 of an in-register DFT
 template <int K> constexpr int dft_split() { return (K == 16 || K == 12 || K == 20) ? 4 : 8; }
 
-template <int K, int DIR, typename C> __device__ __forceinline__ void dftr(C* v) {
+template <int K, int DIR, bool CC = false, typename C> __device__ __forceinline__ void dftr(C* v) {
   if constexpr (K == 1) {
   } else if constexpr (K == 2) {
     bfly2<DIR>(v);
   } else if constexpr (K == 4) {
     bfly4<DIR>(v);
   } else if constexpr (K == 8) {
-    bfly8<DIR>(v);
+    bfly8<DIR, CC>(v);
   } else if constexpr (K == 3) {
-    bfly3<DIR>(v);
+    bfly3<DIR, CC>(v);
   } else if constexpr (K == 5) {
-    bfly5<DIR>(v);
+    bfly5<DIR, CC>(v);
   } else {
     // K = K1*K2 (16 = 4*4, 32 = 8*4, 12 = 4*3, 24 = 8*3, 20 = 4*5, 40 = 8*5): element K2*a + b ; output c + K1*d
     constexpr int K1 = dft_split<K>();
@@ -72,16 +78,16 @@ template <int K, int DIR, typename C> __device__ __forceinline__ void dftr(C* v)
       C t[K1];
 #pragma unroll
       for (int a = 0; a < K1; ++a) t[a] = v[K2 * a + b];
-      dftr<K1, DIR>(t);
+      dftr<K1, DIR, CC>(t);
 #pragma unroll
-      for (int c = 0; c < K1; ++c) Y[b][c] = cmul_wk<K, DIR>(t[c], b * c);
+      for (int c = 0; c < K1; ++c) Y[b][c] = cmul_wk<K, DIR, CC>(t[c], b * c);
     }
 #pragma unroll
     for (int c = 0; c < K1; ++c) {
       C t[K2];
 #pragma unroll
       for (int b = 0; b < K2; ++b) t[b] = Y[b][c];
-      dftr<K2, DIR>(t);
+      dftr<K2, DIR, CC>(t);
 #pragma unroll
       for (int d = 0; d < K2; ++d) v[c + K1 * d] = t[d];
     }
@@ -90,7 +96,7 @@ template <int K, int DIR, typename C> __device__ __forceinline__ void dftr(C* v)
 
 // DFT of K points whose upper half v[K/2..K-1] is zero (not read): the
 // zero-padded half of a forward DDA transform.  Same output as dftr<K>.
-template <int K, int DIR, typename C> __device__ __forceinline__ void dftr_h(C* v) {
+template <int K, int DIR, bool CC = false, typename C> __device__ __forceinline__ void dftr_h(C* v) {
   if constexpr (K == 2) {
     v[1] = v[0];
   } else if constexpr (K == 4) {
@@ -104,7 +110,7 @@ template <int K, int DIR, typename C> __device__ __forceinline__ void dftr_h(C* 
     C o[4] = {v[1], v[3], v[1], v[1]};
     dftr_h<4, DIR>(e);
     dftr_h<4, DIR>(o);
-    const C t1 = w8_1<DIR>(o[1]), t3 = w8_3<DIR>(o[3]);
+    const C t1 = w8_1<DIR, CC>(o[1]), t3 = w8_3<DIR, CC>(o[3]);
     v[0] = vadd(e[0], o[0]);
     v[4] = vsub(e[0], o[0]);
     v[1] = vadd(e[1], t1);
@@ -123,16 +129,16 @@ template <int K, int DIR, typename C> __device__ __forceinline__ void dftr_h(C* 
       C t[K1];
 #pragma unroll
       for (int a = 0; a < K1 / 2; ++a) t[a] = v[K2 * a + b];
-      dftr_h<K1, DIR>(t);
+      dftr_h<K1, DIR, CC>(t);
 #pragma unroll
-      for (int c = 0; c < K1; ++c) Y[b][c] = cmul_wk<K, DIR>(t[c], b * c);
+      for (int c = 0; c < K1; ++c) Y[b][c] = cmul_wk<K, DIR, CC>(t[c], b * c);
     }
 #pragma unroll
     for (int c = 0; c < K1; ++c) {
       C t[K2];
 #pragma unroll
       for (int b = 0; b < K2; ++b) t[b] = Y[b][c];
-      dftr<K2, DIR>(t);
+      dftr<K2, DIR, CC>(t);
 #pragma unroll
       for (int d = 0; d < K2; ++d) v[c + K1 * d] = t[d];
     }
@@ -192,15 +198,26 @@ inline int line_stride(int E, int T, int L, bool line_fastest, bool pair = false
 
 // Four-step twiddles W^(t p), p = 1..E-1, of thread t for DIR: the powers of
 // two come from the table tw[m] = exp(-2*pi*i*m/N), the others are products
-// of at most four of them (fewer shared-memory loads).  w[0] is not set.
+// of at most four of them (fewer shared-memory loads).  E = 20 (80 points) loads
+// 1..4, 5, 10 and 15 and multiplies once: with the powers of two 36^3 was 7.9e-8
+// against 64 bits, more than on 96 points (6.7e-8).  w[0] is not set.
 template <int E, int DIR, typename C>
 __device__ __forceinline__ void line_twiddles(C (&w)[E], int t, const C* __restrict__ tw) {
+  if constexpr (E == 20) {
 #pragma unroll
-  for (int b = 1; b < E; b <<= 1) w[b] = twid<DIR>(tw, t * b);
+    for (int p = 1; p < E; ++p)
+      if (p < 5 || p % 5 == 0) w[p] = twid<DIR>(tw, t * p);
 #pragma unroll
-  for (int p = 3; p < E; ++p) {
-    const int hb = 1 << (31 - __clz(p));  // highest set bit of p
-    if (p != hb) w[p] = cmul(w[hb], w[p - hb]);
+    for (int p = 6; p < E; ++p)
+      if (p % 5) w[p] = cmul(w[p - p % 5], w[p % 5]);
+  } else {
+#pragma unroll
+    for (int b = 1; b < E; b <<= 1) w[b] = twid<DIR>(tw, t * b);
+#pragma unroll
+    for (int p = 3; p < E; ++p) {
+      const int hb = 1 << (31 - __clz(p));  // highest set bit of p
+      if (p != hb) w[p] = cmul(w[hb], w[p - hb]);
+    }
   }
 }
 
@@ -209,26 +226,14 @@ template <typename C> __device__ __forceinline__ C cmulc(C a, C w) {
   return mk2<C>(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y);
 }
 
-// One length-E*T transform of the line held in v by thread t (0 <= t < T),
-// with the thread's twiddles w from line_twiddles: those of DIR, or with
-// CONJW those of -DIR, applied conjugated (so one set serves a forward and an
-// inverse transform; both give the same products as a set built for DIR).
-// `sl` is this line's shared scratch.  BLOCK_SYNC selects __syncthreads (line
-// spread over warps) or __syncwarp.  HALF_IN: elements t + T*i with i >= E/2
-// (the upper half of the line) are zero and are not read.  PAIR: transpose
-// rows of stride E + 2 written with 128-bit stores (complex-float lines; the
-// line stride must come from line_stride(..., pair = true)).
-// SWAP (E = 16, T = 8, PAIR): `swap` is 8 on odd lines and 0 on even ones; odd
-// lines exchange the halves of their scratch rows, which lets lines lie T * 18
-// elements apart without bank conflicts (152 otherwise).
-template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN = false, bool PAIR = false, bool CONJW = false,
-          bool SWAP = false, typename C>
-__device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)[E], int swap = 0) {
+// The two DFT steps of a line: tw(a, p) multiplies a by the twiddle of output p.
+template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN, bool PAIR, bool SWAP, bool CC, typename C, typename TW>
+__device__ __forceinline__ void line_fft_steps(C (&v)[E], C* sl, int t, TW tw, int swap) {
   constexpr int M = E / T;
   static_assert(M * T == E && M >= 1, "E must be a multiple of T");
-  if constexpr (HALF_IN) dftr_h<E, DIR>(v); else dftr<E, DIR>(v);
+  if constexpr (HALF_IN) dftr_h<E, DIR, CC>(v); else dftr<E, DIR, CC>(v);
 #pragma unroll
-  for (int p = 1; p < E; ++p) v[p] = CONJW ? cmulc(v[p], w[p]) : cmul(v[p], w[p]);
+  for (int p = 1; p < E; ++p) v[p] = tw(v[p], p);
   constexpr bool P2 = PAIR && sizeof(C) == 8;
   constexpr int RS = row_stride<E, P2>();
   static_assert(!SWAP || (E == 16 && T == 8 && P2), "halves of 8 elements");
@@ -248,11 +253,46 @@ __device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)
     C u[T];
 #pragma unroll
     for (int s = 0; s < T; ++s) u[s] = (j == 0 ? lo : hi)[s * RS + t + T * j];
-    dftr<T, DIR>(u);
+    dftr<T, DIR, CC>(u);
 #pragma unroll
     for (int q = 0; q < T; ++q) v[j + M * q] = u[q];
   }
   if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
+}
+
+// One length-E*T transform of the line held in v by thread t (0 <= t < T),
+// with the thread's twiddles w from line_twiddles: those of DIR, or with
+// CONJW those of -DIR, applied conjugated (so one set serves a forward and an
+// inverse transform; both give the same products as a set built for DIR).
+// `sl` is this line's shared scratch.  BLOCK_SYNC selects __syncthreads (line
+// spread over warps) or __syncwarp.  HALF_IN: elements t + T*i with i >= E/2
+// (the upper half of the line) are zero and are not read.  PAIR: transpose
+// rows of stride E + 2 written with 128-bit stores (complex-float lines; the
+// line stride must come from line_stride(..., pair = true)).
+// SWAP (E = 16, T = 8, PAIR): `swap` is 8 on odd lines and 0 on even ones; odd
+// lines exchange the halves of their scratch rows, which lets lines lie T * 18
+// elements apart without bank conflicts (152 otherwise).
+template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN = false, bool PAIR = false, bool CONJW = false,
+          bool SWAP = false, typename C>
+__device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)[E], int swap = 0) {
+  line_fft_steps<E, T, DIR, BLOCK_SYNC, HALF_IN, PAIR, SWAP, false>(
+      v, sl, t, [&](C a, int p) { return CONJW ? cmulc(a, w[p]) : cmul(a, w[p]); }, swap);
+}
+
+// The transform with constants good to 48 bits: twiddles from tab[p*T + t] =
+// (hi.x, hi.y, lo.x, lo.y) of exp(-2*pi*i*t*p/N), DFT constants as hi + lo (CC).
+// Lines within a warp.
+template <int E, int T, int DIR, bool HALF_IN = false, bool PAIR = false, bool SWAP = false>
+__device__ __forceinline__ void line_fft_acc(float2 (&v)[E], float2* sl, int t, const float4* __restrict__ tab,
+                                             int swap = 0) {
+  line_fft_steps<E, T, DIR, false, HALF_IN, PAIR, SWAP, true>(
+      v, sl, t,
+      [&](float2 a, int p) {
+        const float4 w = __ldg(tab + p * T + t);
+        const float s = DIR > 0 ? -1.f : 1.f;
+        return cmul_hl(a, make_float2(w.x, s * w.y), make_float2(w.z, s * w.w));
+      },
+      swap);
 }
 
 // One length-E*T transform with its own twiddles (`tw` as in line_twiddles).

@@ -660,6 +660,24 @@ static double pad_limit(const Geometry& g) {
   return smooth(g.Mx) && smooth(g.My) && smooth(g.Mz) ? 4.5 : 12.0;
 }
 
+// Twiddles of line_fft_acc: exp(-2*pi*i*t*p/n) as hi + lo at [p*T + t].
+static float4* upload_hl_twiddles(int n, size_t& bytes) {
+  const int T = reg_threads(n);
+  std::vector<float4> h(n);
+  const double pi = 3.14159265358979323846;
+  for (int p = 0; p < n / T; ++p)
+    for (int t = 0; t < T; ++t) {
+      const double a = -2.0 * pi * t * p / n, c = std::cos(a), s = std::sin(a);
+      const float ch = (float)c, sh = (float)s;
+      h[p * T + t] = make_float4(ch, sh, (float)(c - (double)ch), (float)(s - (double)sh));
+    }
+  float4* d = nullptr;
+  if (dev_alloc((void**)&d, n * sizeof(float4)) != cudaSuccess) return nullptr;
+  cudaMemcpy(d, h.data(), n * sizeof(float4), cudaMemcpyHostToDevice);
+  bytes += n * sizeof(float4);
+  return d;
+}
+
 template <typename T>
 int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0, const int16_t* iocc_host, bool pad) {
   g.nx = nx; g.ny = ny; g.nz = nz;
@@ -695,6 +713,26 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   twy = upload_twiddles<T>(g.My, bytes_allocated);
   twz = upload_twiddles<T>(g.Mz, bytes_allocated);
   if (!twx || !twy || !twz) { set_error("prepare", "twiddle allocation failed"); return 1; }
+  // The generic transforms that odd, periodic and widely padded targets would run
+  // on their 2n grid sum prime-length DFTs in FP64 and read each twiddle rounded
+  // once.  The plain register transforms multiply theirs up, and their constants
+  // round the same way forward and back, which adds up over the passes: 5.1-8.9e-8
+  // against 64 bits where the generic ones are 4.1-7.6e-8.  With constants as hi +
+  // lo and the finish in FP64 these targets are at 2.9-4.3e-8 (25x27x29 7.6 -> 3.4,
+  // generic 4.5; 63x61x59 8.9 -> 3.9, 4.5; 97^3 8.9 -> 3.7, 4.2; the transforms
+  // alone, CXADIA = 0: 63x61x59 26.7 -> 9.7, 9.7, and at worst, three prime sides,
+  // 47^3 19.7 -> 10.1, 8.0).  us per
+  // RHS-MATVEC, 8 RHS, plain / this / generic: 45x37x31 13.9 / 15.9 / 779,
+  // 51x75x39 47.9 / 60.4 / 361, 63x61x59 42.0 / 52.1 / 6397, 75^3 141 / 192 / 431,
+  // periodic 20x24x18 5.0 / 5.5 / 13.4.
+  int base[3];
+  if (sizeof(T) == 4 && xpipe && !(g.base_lengths(base) &&
+                                   (pad || (base[0] == g.Mx && base[1] == g.My && base[2] == g.Mz)))) {
+    cx = upload_hl_twiddles(g.Mx, bytes_allocated);
+    cy = upload_hl_twiddles(g.My, bytes_allocated);
+    cz = upload_hl_twiddles(g.Mz, bytes_allocated);
+    if (!cx || !cy || !cz) { set_error("prepare", "twiddle allocation failed"); return 1; }
+  }
   // index maps, built on the device from IOCC
   const int nrows = nat / nx;
   cudaError_t e;
@@ -909,7 +947,7 @@ template <typename T> int Engine<T>::upload_green(const void* host_green) {
 
 template <typename T> void Engine<T>::release() {
   cudaFree(d_err);  // waits for the device: nothing uses the engine's blocks any more
-  dev_free(twx); dev_free(twy); dev_free(twz);
+  dev_free(twx); dev_free(twy); dev_free(twz); dev_free(cx); dev_free(cy); dev_free(cz);
   dev_free(green); dev_free(occ); dev_free(inv); dev_free(iocc); dev_free(rowq);
   dev_free(zhat); dev_free(slab);
   *this = Engine<T>{};

@@ -29,6 +29,7 @@
 // for the FFT3D build, a few columns for the SLICES build).
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -73,6 +74,7 @@ template <typename T> struct XParams {
   const cplx<T>* twx;
   const cplx<T>* twy;
   const cplx<T>* twz;
+  const float4 *cx, *cy, *cz;  // hi + lo twiddles of the ACC passes (Engine::cx)
   int lsx, lsy, lsz;  // line strides of the x, y, z passes
   int tlx;            // tile / line scratch elements of the x passes
   T inv_ngrid;
@@ -269,9 +271,23 @@ template <int MAXC, typename C> __device__ __forceinline__ void stage_chunk_asyn
   }
 }
 
+// line transform of a pass (ACC: constants good to 48 bits)
+template <int E, int TT, int DIR, bool ACC, bool HALF_IN, bool PAIR, typename C>
+__device__ __forceinline__ void xline(C (&v)[E], C* sl, int t, const C* tw, const float4* tab) {
+  if constexpr (ACC) line_fft_acc<E, TT, DIR, HALF_IN, PAIR>(v, sl, t, tab);
+  else line_fft<E, TT, DIR, false, HALF_IN, PAIR>(v, sl, t, tw);
+}
+
+// line transform of a z pass whose thread keeps the twiddles w of DIR = +1
+template <int E, int TT, int DIR, bool ACC, bool HALF_IN, bool PAIR, bool SWAP = false, typename C>
+__device__ __forceinline__ void zline(C (&v)[E], C* sl, int t, const C (&w)[E], const float4* tab, int swap = 0) {
+  if constexpr (ACC) line_fft_acc<E, TT, DIR, HALF_IN, PAIR, SWAP>(v, sl, t, tab, swap);
+  else line_fft_w<E, TT, DIR, false, HALF_IN, PAIR, (DIR < 0), SWAP>(v, sl, t, w, swap);
+}
+
 // ------------------------------------------------------------- XF: x forward
 // block: RL rows (iy) x TT threads, thread-fastest; grid (ceil(ny/RL), nz, 3*nr)
-template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_xf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -312,7 +328,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
 #pragma unroll
     for (int i = 0; i < H; ++i) v[i].y = -v[i].y;
   }
-  line_fft<E, TT, +1, false, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx);
+  xline<E, TT, +1, ACC, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, P.cx);
   __syncthreads();  // all line scratch consumed before the tile reuses it
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma_x) {
@@ -336,7 +352,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xf(const 
 
 // ------------------------------------------------------------- YF: y forward
 // block: RL z-lines (iz) x TT; grid (ceil(nz/RL), nkx, 3*nrb)
-template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_yf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -354,7 +370,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yf(const 
   const bool zin = iz < P.nz;
 #pragma unroll
   for (int i = 0; i < H; ++i) v[i] = zin && t + TT * i < P.ny ? A[t + TT * i] : mk<C>(0, 0);  // iy < ny <= N/2
-  line_fft<E, TT, +1, false, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy);
+  xline<E, TT, +1, ACC, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, P.cy);
   __syncthreads();
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma) {
@@ -460,7 +476,7 @@ template <int BTY> constexpr int zline_stride() { return BTY > 0 ? BTY : 1; }
 // ------------------------------------------------------------- ZG: z * Green * z^-1
 // block: RZ lines x TT threads x 3 components, thread-fastest within a line;
 // lines are (kx, ky) pairs p = kxl*My + ky.  grid (nrb, ceil(nkx*My/RZ))
-template <typename T, int N, int BTY = 0>
+template <typename T, int N, int BTY = 0, bool ACC = false>
 __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) == 8 ? 1 : XShape<N>::ZG_MINB)
     kx_zg(XParams<T> P) {
   using C = cplx<T>;
@@ -512,7 +528,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
     for (int i = 0; i < H; ++i)
       v[i] = live && t + TT * i < P.nz ? row[(t + TT * i) * zs] : mk<C>(0, 0);  // iz < nz <= N/2
   }
-  line_fft<E, TT, +1, false, true, S_::PAIR>(v, my, t, P.twz);
+  xline<E, TT, +1, ACC, true, S_::PAIR>(v, my, t, P.twz, P.cz);
 #pragma unroll
   for (int i = 0; i < E; ++i) my[t + TT * i] = v[i];
   __syncthreads();
@@ -563,7 +579,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
 #pragma unroll
   for (int i = 0; i < E; ++i) v[i] = my[t + TT * i];
   __syncwarp();
-  line_fft<E, TT, -1, false, false, S_::PAIR>(v, my, t, P.twz);
+  xline<E, TT, -1, ACC, false, S_::PAIR>(v, my, t, P.twz, P.cz);
   if constexpr (BULK) {
 #pragma unroll
     for (int i = 0; i < H; ++i)
@@ -628,7 +644,7 @@ __device__ __forceinline__ void zg3_green(const C* rec0, int t, C (&v)[3][E]) {
   }
 }
 
-template <typename T, int N, int BTY = 0> __global__ void __launch_bounds__(128, 3) kx_zg3(XParams<T> P) {
+template <typename T, int N, int BTY = 0, bool ACC = false> __global__ void __launch_bounds__(128, 3) kx_zg3(XParams<T> P) {
   using C = cplx<T>;
   using R = T;
   using S_ = XShape<N>;
@@ -662,9 +678,9 @@ template <typename T, int N, int BTY = 0> __global__ void __launch_bounds__(128,
   }
   // one twiddle set for the six transforms: forward, and conjugated for the inverse
   C w[E];
-  line_twiddles<E, +1>(w, t, P.twz);
+  if constexpr (!ACC) line_twiddles<E, +1>(w, t, P.twz);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) line_fft_w<E, TT, +1, false, true, S_::PAIR>(v[c], my, t, w);
+  for (int c = 0; c < 3; ++c) zline<E, TT, +1, ACC, true, S_::PAIR>(v[c], my, t, w, P.cz);
   if (live) {
     if (P.ipbc == 0) {
       R sxy, sxz, syz;
@@ -680,7 +696,7 @@ template <typename T, int N, int BTY = 0> __global__ void __launch_bounds__(128,
     }
   }
 #pragma unroll
-  for (int c = 0; c < 3; ++c) line_fft_w<E, TT, -1, false, false, S_::PAIR, true>(v[c], my, t, w);
+  for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, false, S_::PAIR>(v[c], my, t, w, P.cz);
   if (live) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -746,7 +762,7 @@ template <int N> struct ZRow {
   static constexpr int SCRATCH = XShape<N>::TT == 8 && XShape<N>::E == 16 ? 8 * 18 : 0;
 };
 
-template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(XParams<T> P) {
+template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(128, 3) kx_zg3r(XParams<T> P) {
   using C = cplx<T>;
   using R = T;
   using S_ = XShape<N>;
@@ -810,7 +826,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
   cp_async_commit();
   const R sx = 2 * kx > P.Mx ? (R)-1 : (R)1, sy = 2 * ky > P.My ? (R)-1 : (R)1;
   C w[E];
-  line_twiddles<E, +1>(w, t, P.twz);
+  if constexpr (!ACC) line_twiddles<E, +1>(w, t, P.twz);
   bool staged = false;
   while (rb < rb1) {
     const int nrb = next_rb(rb + 1);
@@ -828,7 +844,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
       __syncwarp();  // the buffer is read before the next row overwrites it
       if (c < 2) fetch(rb, c + 1);
       else if (nrb < rb1) fetch(nrb, 0);
-      line_fft_w<E, TT, +1, false, true, S_::PAIR, false, SW>(v[c], my, t, w, fswap);
+      zline<E, TT, +1, ACC, true, S_::PAIR, SW>(v[c], my, t, w, P.cz, fswap);
     }
     if (!staged) {
       __syncthreads();  // every thread's Green copies have landed (waited for at c = 1)
@@ -836,7 +852,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
     }
     if (live) zg3_green_s<N, TT, E>(gs + (size_t)l * LREC, t, v);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) line_fft_w<E, TT, -1, false, false, S_::PAIR, true, SW>(v[c], my, t, w, fswap);
+    for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, false, S_::PAIR, SW>(v[c], my, t, w, P.cz, fswap);
     if (live) {
       C* row = P.B + (size_t)rb * 3 * cs + (size_t)p * P.ldb;
 #pragma unroll
@@ -853,7 +869,7 @@ template <typename T, int N> __global__ void __launch_bounds__(128, 3) kx_zg3r(X
 
 // ------------------------------------------------------------- YI: y inverse
 // block: RL z-lines x TT; grid (ceil(nz/RL), nkx, 3*nrb)
-template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_yi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -900,7 +916,7 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_yi(const 
     for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();  // the tile is consumed before the line scratch reuses it
   }
-  line_fft<E, TT, -1, false, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy);
+  xline<E, TT, -1, ACC, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, P.cy);
   if (iz < nz) {
     C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * nz + iz) * P.Mx + kx) * P.lda;
 #pragma unroll
@@ -969,7 +985,7 @@ constexpr bool xi_staged(int n, int TT, size_t elem) {
 
 // block: RL rows (iy) x TT; grid (ceil(ny/RL), nz, 3*nr)
 // shared memory: tile / line scratch [tlx] | x chunk | CXADIA chunk
-template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_xi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -1050,11 +1066,16 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
     for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();
   }
-  line_fft<E, TT, -1, false, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx);
+  xline<E, TT, -1, ACC, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, P.cx);
   // finish (cu:116-118): y = CXADIA x - w/ngrid [+ CXAOFF terms], conj for 'C'
   C* y = P.y + (size_t)rl * P.y_rs + (size_t)c * S;
   const C* ao = P.aoff ? P.aoff + (size_t)rl * P.a_rs : nullptr;
   double2 dacc = make_double2(0.0, 0.0);  // x*y of this thread's sites (dot_out)
+  // ACC: in FP64, rounded once
+  using TF = typename std::conditional<ACC, double, T>::type;
+  using F = cplx<TF>;
+  auto up = [](C a) { return mk2<F>((TF)a.x, (TF)a.y); };
+  const TF inv_ngrid = ACC ? (TF)(1.0 / ((double)P.Mx * P.My * P.Mz)) : (TF)P.inv_ngrid;
 #pragma unroll
   for (int i = 0; i < H; ++i) {
     if (iy >= ny) break;
@@ -1070,15 +1091,16 @@ template <typename T, int N> __global__ void __launch_bounds__(256) kx_xi(const 
     C xc = chunked ? xs[q - q0] : x[(size_t)c * S + q];
     const C av = chunked ? as[q - q0] : ad[qa];
     if (P.conj) xc.y = -xc.y;
-    C yv = csub(cmul(av, xc), cscale(v[i], P.inv_ngrid));
+    F yf = csub(cmul(up(av), up(xc)), cscale(up(v[i]), inv_ngrid));
     if (ao) {
       C x1 = x[q], x2 = x[S + q], x3 = x[2 * (size_t)S + q];
       if (P.conj) { x1.y = -x1.y; x2.y = -x2.y; x3.y = -x3.y; }
-      const C a23 = ao[qa], a31 = ao[SA + qa], a12 = ao[2 * (size_t)SA + qa];
-      if (c == 0) yv = cadd(yv, cadd(cmul(a31, x3), cmul(a12, x2)));
-      else if (c == 1) yv = cadd(yv, cadd(cmul(a12, x1), cmul(a23, x3)));
-      else yv = cadd(yv, cadd(cmul(a23, x2), cmul(a31, x1)));
+      const F a23 = up(ao[qa]), a31 = up(ao[SA + qa]), a12 = up(ao[2 * (size_t)SA + qa]);
+      if (c == 0) yf = cadd(yf, cadd(cmul(a31, up(x3)), cmul(a12, up(x2))));
+      else if (c == 1) yf = cadd(yf, cadd(cmul(a12, up(x1)), cmul(a23, up(x3))));
+      else yf = cadd(yf, cadd(cmul(a23, up(x2)), cmul(a31, up(x1))));
     }
+    C yv = mk2<C>((T)yf.x, (T)yf.y);
     if (P.conj) yv.y = -yv.y;
     y[q] = yv;
     if (P.dot_out) {  // conj = 0 here: xc is x
@@ -1302,7 +1324,22 @@ template <typename T, int N, int BTY> static const void* xkt(XPass p) {
   return nullptr;
 }
 
-template <typename T, int N> static const void* xk(XPass p, int my = 0) {
+template <typename T, int N> static const void* xk(XPass p, int my = 0, bool acc = false) {
+  if constexpr (sizeof(T) == 4)
+    if (acc) switch (p) {
+      case XPass::XF: return (const void*)kx_xf<T, N, true>;
+      case XPass::YF: return (const void*)kx_yf<T, N, true>;
+      case XPass::ZG: return (const void*)kx_zg<T, N, 0, true>;
+      case XPass::ZG3:
+        if constexpr (Z3Shape<N>::OK) return (const void*)kx_zg3<T, N, 0, true>;
+        return nullptr;
+      case XPass::ZG3R:
+        if constexpr (Z3Shape<N>::OK) return (const void*)kx_zg3r<T, N, true>;
+        return nullptr;
+      case XPass::YI: return (const void*)kx_yi<T, N, true>;
+      case XPass::XI: return (const void*)kx_xi<T, N, true>;
+      default: return nullptr;
+    }
   if (p == XPass::ZGT || p == XPass::ZG3T) {
     switch (my) {
       case 64: return xkt<T, N, 64>(p);
@@ -1329,26 +1366,26 @@ template <typename T, int N> static const void* xk(XPass p, int my = 0) {
 }
 
 // my: M_y, for the z passes on the fused layout (ZGT, ZG3T)
-template <typename T> static const void* xkernel(XPass p, int n, int my = 0) {
+template <typename T> static const void* xkernel(XPass p, int n, int my = 0, bool acc = false) {
   switch (n) {
-    case 16: return xk<T, 16>(p, my);
-    case 32: return xk<T, 32>(p, my);
-    case 48: return xk<T, 48>(p, my);
-    case 64: return xk<T, 64>(p, my);
-    case 80: return xk<T, 80>(p, my);
-    case 96: return xk<T, 96>(p, my);
-    case 128: return xk<T, 128>(p, my);
-    case 192: return xk<T, 192>(p, my);
-    case 256: return xk<T, 256>(p, my);
+    case 16: return xk<T, 16>(p, my, acc);
+    case 32: return xk<T, 32>(p, my, acc);
+    case 48: return xk<T, 48>(p, my, acc);
+    case 64: return xk<T, 64>(p, my, acc);
+    case 80: return xk<T, 80>(p, my, acc);
+    case 96: return xk<T, 96>(p, my, acc);
+    case 128: return xk<T, 128>(p, my, acc);
+    case 192: return xk<T, 192>(p, my, acc);
+    case 256: return xk<T, 256>(p, my, acc);
     // FP64: the shared memory of the 160-, 320- and 512-point passes is too large
     case 160:
-      if constexpr (sizeof(T) == 4) return xk<T, 160>(p, my);
+      if constexpr (sizeof(T) == 4) return xk<T, 160>(p, my, acc);
       return nullptr;
     case 320:
-      if constexpr (sizeof(T) == 4) return xk<T, 320>(p, my);
+      if constexpr (sizeof(T) == 4) return xk<T, 320>(p, my, acc);
       return nullptr;
     case 512:
-      if constexpr (sizeof(T) == 4) return xk<T, 512>(p, my);
+      if constexpr (sizeof(T) == 4) return xk<T, 512>(p, my, acc);
       return nullptr;
     default: return nullptr;
   }
@@ -1468,6 +1505,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   P.B = E.slab;
   P.green = E.green; P.ipbc = g.ipbc;
   P.twx = E.twx; P.twy = E.twy; P.twz = E.twz;
+  P.cx = E.cx; P.cy = E.cy; P.cz = E.cz;
   P.inv_ngrid = (T)(1.0 / (double)g.ngrid());
   P.dot_out = a.dot_out; P.dot_part = a.dot_part; P.dot_cnt = a.dot_cnt; P.dot_k = a.dot_k;
   if (a.dot_out && (a.conj || !a.dot_part || !a.dot_cnt)) { set_error("MATVEC", "fused x*y sum needs conj = 0"); return 25; }
@@ -1476,7 +1514,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   const int RZ = std::max(1, 128 / TZ);  // ZG: 3*TZ*RZ threads
   // ZG3 (components in registers, E <= 16) unless the engine's tunable (autotuner
   // or DDSCAT_B200_ZG=1) selects ZG
-  const void* fzg3 = E.tune_zg ? nullptr : xkernel<T>(XPass::ZG3, g.Mz);
+  const void* fzg3 = E.tune_zg ? nullptr : xkernel<T>(XPass::ZG3, g.Mz, 0, E.cz != nullptr);
   const int RZ3 = 128 / TZ;  // ZG3: RZ3 lines of TZ threads
   // must match XShape<N>::PAIR
   P.lsx = line_stride(g.Mx / TX, TX, RX, false, TX >= 8);
@@ -1511,14 +1549,14 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   const size_t smz = fzg3 ? (size_t)RZ3 * P.lsz * sizeof(C) : (size_t)3 * RZ * P.lsz * sizeof(C);
   // ZG3R (Green lines staged once per block and reused for a chunk of RHS):
   // IPBC=0, batches of at least 4 RHS (DDSCAT_B200_NOZG3R=1 keeps ZG3)
-  const void* fzg3r = fzg3 && g.ipbc == 0 && !env_flag("DDSCAT_B200_NOZG3R") ? xkernel<T>(XPass::ZG3R, g.Mz) : nullptr;
+  const void* fzg3r = fzg3 && g.ipbc == 0 && !env_flag("DDSCAT_B200_NOZG3R") ? xkernel<T>(XPass::ZG3R, g.Mz, 0, E.cz != nullptr) : nullptr;
   const int lszr = g.Mz == 128 ? 8 * 18 : P.lsz;  // ZRow::SCRATCH
   const size_t smzr = ((size_t)RZ3 * lszr) * sizeof(C) + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ == 4 ? 4 : 0)) * sizeof(C);
-  const void* fxf = xkernel<T>(XPass::XF, g.Mx);
-  const void* fyf = xkernel<T>(XPass::YF, g.My);
-  const void* fzg = xkernel<T>(XPass::ZG, g.Mz);
-  const void* fyi = xkernel<T>(XPass::YI, g.My);
-  const void* fxi = xkernel<T>(XPass::XI, g.Mx);
+  const void* fxf = xkernel<T>(XPass::XF, g.Mx, 0, E.cx != nullptr);
+  const void* fyf = xkernel<T>(XPass::YF, g.My, 0, E.cy != nullptr);
+  const void* fzg = xkernel<T>(XPass::ZG, g.Mz, 0, E.cz != nullptr);
+  const void* fyi = xkernel<T>(XPass::YI, g.My, 0, E.cy != nullptr);
+  const void* fxi = xkernel<T>(XPass::XI, g.Mx, 0, E.cx != nullptr);
   // DDSCAT_B200_FUSEXY=1, FP32 with all kx planes of a slab batch resident
   // (FFT3D): the x and y passes fused per z plane (kxy_f / kxy_i), three
   // launches per slab batch.  Opt-in: at 128^3 it moves 41 % fewer DRAM bytes
@@ -1528,7 +1566,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   const void* fxyf = nullptr;
   const void* fxyi = nullptr;
   if constexpr (sizeof(T) == 4) {
-    if (E.slab_B == g.Mx && env_flag("DDSCAT_B200_FUSEXY")) {
+    if (E.slab_B == g.Mx && !E.cx && env_flag("DDSCAT_B200_FUSEXY")) {
       fxyf = xykernel(true, g.Mx, g.My);
       fxyi = xykernel(false, g.Mx, g.My);
     }

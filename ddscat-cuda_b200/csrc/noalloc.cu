@@ -81,16 +81,9 @@ static int noalloc_scratch(int dev, float2** out) {
 // its 132-point grid (5.2 M elements, taken) before 160 points were a length;
 // padded to 160 it needs 7.2 M and runs in two plane batches.
 static size_t admission_elems(const Geometry& g) {
-  size_t mx = 2 * (size_t)g.nx, my = 2 * (size_t)g.ny, mz = 2 * (size_t)g.nz;
-  if (g.ipbc == 0 && g.padded() && !((g.nx | g.ny | g.nz) & 1)) {
-    auto length = [](size_t m) -> size_t {
-      for (size_t l : {16, 32, 48, 64, 96, 128, 192, 256, 512})
-        if (l >= m) return l;
-      return 0;
-    };
-    const size_t lx = length(mx), ly = length(my), lz = length(mz);
-    if (lx && ly && lz && (double)(lx * ly * lz) <= 2.5 * (double)(mx * my * mz)) { mx = lx; my = ly; mz = lz; }
-  }
+  int m[3];
+  const bool base = g.padded() && g.base_lengths(m);
+  const size_t mx = base ? m[0] : 2 * g.nx, my = base ? m[1] : 2 * g.ny;
   return 3 * (size_t)g.nz * mx * g.ny + 3 * my * (size_t)g.nz * mx;
 }
 

@@ -102,6 +102,44 @@ def test_ragged_fp64_and_batch_equal_unpadded(monkeypatch, dims):
         assert np.linalg.norm(sol[k] - sol[2 + k]) <= 40e-5 * np.linalg.norm(sol[k])
 
 
+def _rel_errors(monkeypatch, dims, periodic=False):
+    """Norm errors against the FP64 oracle on the default grid and on the 2n grid,
+    with CXADIA of the size of an inverse polarisability (14 at m = 1.5)."""
+    iocc, ak, x, _, aoff = _case(dims, seed=17)
+    adia = np.full_like(x, 12.0 - 3.0j)
+    per = dict(ipbc=1, gamma=0.1, pyd=float(dims[1]), pzd=float(dims[2])) if periodic else {}
+    gp = O.GreenParams(*dims, ak=tuple(float(np.float32(a)) for a in ak),
+                       **{k: float(np.float32(v)) if k == "gamma" else v for k, v in per.items()})
+    ref = O.Operator.from_params(gp, iocc).apply_full(x, adia, aoff)
+    out = []
+    for nopad in ("0", "1"):
+        monkeypatch.setenv("DDSCAT_B200_NOPAD", nopad)
+        dda = D.DDA()
+        dda.prepare_green(*dims, iocc, ak, **per)
+        out.append(np.linalg.norm(dda.apply(x, adia, aoff) - ref) / np.linalg.norm(ref))
+        dda.release()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,periodic", [((13, 17, 11), False), ((25, 27, 29), False), ((35, 35, 35), False),
+                                           ((47, 47, 47), False), ((66, 12, 10), False), ((45, 37, 31), False),
+                                           ((8, 9, 65), False), ((7, 131, 6), False), ((13, 13, 13), True),
+                                           ((15, 15, 15), True), ((20, 24, 18), True)])
+def test_register_grid_is_no_less_precise_than_2n(monkeypatch, dims, periodic):
+    """Targets that would run the generic transforms on their 2n grid, which sum
+    prime-length DFTs in FP64, lose no precision on register lengths."""
+    padded, generic = _rel_errors(monkeypatch, dims, periodic)
+    assert padded <= generic
+
+
+@pytest.mark.gpu
+def test_80_points_are_no_less_precise_than_96(monkeypatch):
+    """36^3 runs on 80 points per axis, 48^3 on 96: the shorter transform has no
+    more roundings, so its twiddles must not make it less precise."""
+    assert _rel_errors(monkeypatch, (36, 36, 36))[0] <= _rel_errors(monkeypatch, (48, 48, 48))[0]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims,planes", [((69, 69, 73), "some"), ((45, 37, 31), "all"), ((5, 255, 251), "some")])
 def test_ragged_noalloc_equals_apply(dims, planes):
