@@ -313,29 +313,37 @@ template <typename T> static unsigned sum_grid(const VecOps<T>& o, int n, const 
                                     (size_t)std::min(o.nblocks, 148 * per_sm));
 }
 
-// The iterations of a solver as one CUDA graph.  An iteration is 14 to 30
+// The iterations of a solver as one CUDA graph.  An iteration is 6 to 30
 // launches, most of them shorter than the 3 us the host takes for a launch on
-// small grids (32^3: 175 us of kernels in 280 us per iteration).  The first
-// iteration runs launch by launch (one-time kernel set-up), the second is
-// captured and every later one is a single launch.  Not with per-MATVEC output
-// (its events are read between the MATVECs).  If the capture is not possible
-// the iterations keep running launch by launch.
+// small grids.  Recording and instantiating the graph costs 350-450 us; it gains
+// 22-25 us per PBCGS2 iteration up to 45x37x31 and 7-16 us per QMRCCG iteration
+// (us by launches / by graph: 16^3 132 / 103 and 68 / 61; 32^3 150 / 122 and 80 / 64;
+// 45x37x31 189 / 160 and 98 / 88; 64^3 307 / 260 and 155 / 145).  So it starts at
+// iteration `from`, where a solve that ends there is not longer than the one with
+// a launch per scalar step was (230 and 95 us per iteration at 16^3): 4 for PBCGS2,
+// 16 for QMRCCG.  Shorter solves pay nothing: QMRCCG at 16^3, us per call by launches
+// / with a graph from the second iteration: 2 iterations 477 / 785, 5 689 / 968, 12
+// 1169 / 1392.
+// Not with per-MATVEC output (its events are read between the MATVECs).  If the
+// capture is not possible the iterations keep running launch by launch.
 struct IterGraph {
+  const int from;  // first iteration of the graph
   cudaStream_t cap = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned long long kernels = 0;
   int products = 0;
   bool off = false;
+  explicit IterGraph(int from_) : from(from_) {}
   ~IterGraph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (cap) cudaStreamDestroy(cap);
   }
-  // Runs body (one iteration on io.stream / eng.stream / ops.stream), as a graph
-  // from its second call on; nc counts the iteration's products.
+  // Runs body (iteration it = 1, 2, ... on io.stream / eng.stream / ops.stream), as
+  // a graph from iteration `from` on; nc counts the iteration's products.
   template <typename T, typename F> int run(SolveIO<T>& io, int& nc, int it, F body) {
-    if (off || io.verbose || it < 2) return body();
+    if (off || io.verbose || it < from) return body();
     if (!exec && !capture(io, nc, body)) {
       off = true;
       cudaGetLastError();
@@ -378,7 +386,7 @@ static inline unsigned dq_grid(int n) { return (unsigned)std::min<size_t>(ceil_d
 // host waits once per iteration (for the residual, the breakdown status and the
 // reliable-update tests); the reference waits for every inner product
 // (cu:1190-1255).  32^3 sphere, PBCGS2 + EVALQ + SCAT through the drop-in entry
-// points: 4.54 -> 3.23 ms with the iterations as a graph (IterGraph).
+// points: 4.54 -> 3.23 ms (16 iterations).
 struct DPState {
   double2 alpha, omega, sigma, rho0, rho1, beta;
   double2 one, mone;
@@ -601,7 +609,7 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
   auto dot = [&](const C* v, int step) {
     k_dp_dot<C><<<gd, RED_THREADS, 0, c.st()>>>(n, rr, v, step, dS, vo.d_red, vo.d_out, vo.d_count);
   };
-  IterGraph ig;
+  IterGraph ig(4);
   int it = 0;
   while (resid > io.tol && it < io.maxit) {
     ++it;
@@ -761,7 +769,7 @@ template <typename T> int solve_qmrccg(SolveIO<T>& io) {
   const VecOps<T>& vo = *io.ops;
   const unsigned gb = dq_grid(n), gd = sum_grid(vo, n, (const void*)k_dq_dots<C>),
                  gr = sum_grid(vo, n, (const void*)k_dq_dsxr<C>);
-  IterGraph ig;
+  IterGraph ig(16);
   int it = 0;
   while (it < io.maxit && resid > io.tol) {
     ++it;
