@@ -799,7 +799,15 @@ template <typename T> int Engine<T>::ensure_workspace(int nrhs) {
     else { slab_nr = 1; slab_B = (int)std::max<size_t>(1, slab_budget_elems / per_plane); }
   }
   e = dev_alloc((void**)&slab, (size_t)slab_nr * slab_B * per_plane * sizeof(C));
-  if (e != cudaSuccess) { set_cuda_error("malloc xy-slab workspace", e); return 1; }
+  if (e != cudaSuccess) {
+    // no half a workspace: the next call would take it for complete
+    dev_free(zhat);
+    bytes_allocated -= (size_t)zcap * per_rhs_z * sizeof(C);
+    zhat = nullptr;
+    zcap = 0;
+    set_cuda_error("malloc xy-slab workspace", e);
+    return 1;
+  }
   bytes_allocated += (size_t)slab_nr * slab_B * per_plane * sizeof(C);
   return 0;
 }
