@@ -169,6 +169,13 @@ static int slices_build() {
 #endif
 }
 
+// The SLICES build is taken for its bounded memory: it keeps less for reuse, what
+// a target of 96^3 gives back and takes again.
+[[maybe_unused]] static const bool g_keep_set = [] {
+  if (slices_build()) mem_keep((size_t)512 << 20);
+  return true;
+}();
+
 static int allocate_runtime() {
   const size_t n = (size_t)3 * s.eng.g.nat, cn = (size_t)3 * s.eng.g.nat0;
   if (cn > (size_t)0x7fffffff) { set_error("allocate runtime", "3*NAT0 exceeds solver int range"); return 204; }

@@ -35,6 +35,7 @@ void dev_free(void* p);
 cudaError_t host_alloc(void** p, size_t bytes);
 void host_free(void* p);
 void mem_trim();  // give every idle block back to the driver
+void mem_keep(size_t device_bytes);  // limit of the idle device blocks
 void raise_smem_limit(const void* f);  // thread-safe, once per kernel
 // an on/off environment switch: on when set to a non-empty value other than "0"
 bool env_flag(const char* name);

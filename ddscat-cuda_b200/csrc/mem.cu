@@ -10,10 +10,12 @@
 // Rules: a block is handed back only when no work that uses it is in flight
 // (the callers wait for their stream first; Engine::release and release_state
 // for the device, as cudaFree did), so any thread or stream may take it next.
-// The lists hold at most DEV_KEEP and HOST_KEEP bytes; what does not fit goes
-// straight back to the driver, mem_trim (ddscat_cuda_release) returns
-// everything, and an allocation that fails trims first and tries again.
+// The lists hold at most mem_keep's limit and HOST_KEEP bytes; what does not fit
+// goes straight back to the driver, mem_trim (ddscat_cuda_release) returns
+// everything, and an allocation that fails trims first and tries again.  A block
+// serves requests down to half its size, and at most SLACK bytes smaller.
 // Contents of a block are undefined.
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -23,8 +25,12 @@ namespace ddb {
 
 namespace {
 
-constexpr size_t DEV_KEEP = (size_t)2 << 30;    // the temporaries of a 128^3 Green build are 1.2 GB
+// Limit of the idle device bytes (mem_keep).  The default holds what a prepare at
+// 128^3 gives back and takes again, 1.5 GB: Green tensor 0.1, its temporaries 0.4,
+// vectors 0.7, MATVEC workspace 0.3.
+size_t g_dev_keep = (size_t)2 << 30;
 constexpr size_t HOST_KEEP = (size_t)64 << 20;
+constexpr size_t SLACK = (size_t)64 << 20;
 
 struct Block {
   size_t bytes;
@@ -68,9 +74,9 @@ cudaError_t get(void** p, size_t bytes, bool host) {
   Cache& c = cache();
   {
     std::lock_guard<std::mutex> lock(c.mu);
-    // the smallest idle block that holds the request without wasting as much again
+    // the smallest idle block that holds the request
     auto it = c.idle.lower_bound({dev, want});
-    if (it != c.idle.end() && it->first.first == dev && it->first.second <= 2 * want) {
+    if (it != c.idle.end() && it->first.first == dev && it->first.second <= want + std::min(want, SLACK)) {
       *p = it->second;
       c.live[*p] = Block{it->first.second, dev};
       c.held[host] -= it->first.second;
@@ -99,7 +105,7 @@ void put(void* p, bool host) {
     if (it != c.live.end()) {
       const Block b = it->second;
       c.live.erase(it);
-      if (c.held[host] + b.bytes <= (host ? HOST_KEEP : DEV_KEEP)) {
+      if (c.held[host] + b.bytes <= (host ? HOST_KEEP : g_dev_keep)) {
         c.held[host] += b.bytes;
         c.idle.emplace(std::make_pair(b.dev, b.bytes), p);
         return;
@@ -115,6 +121,11 @@ cudaError_t dev_alloc(void** p, size_t bytes) { return get(p, bytes, false); }
 void dev_free(void* p) { put(p, false); }
 cudaError_t host_alloc(void** p, size_t bytes) { return get(p, bytes, true); }
 void host_free(void* p) { put(p, true); }
+
+void mem_keep(size_t device_bytes) {
+  std::lock_guard<std::mutex> lock(cache().mu);
+  g_dev_keep = device_bytes;
+}
 
 void mem_trim() {
   Cache& c = cache();

@@ -58,6 +58,29 @@ def test_refused_prepares_keep_no_memory():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("layout,keep_mib", [("slices", 512), ("fft3d", 2048)])
+def test_idle_blocks_stay_within_the_limit(layout, keep_mib):
+    """A 160^3 target (3.4 GB) followed by a small one leaves at most the limit of
+    the reuse lists; the SLICES build's is small."""
+    torch = pytest.importorskip("torch")
+    dda = D.DDA(layout)
+
+    def prepare(n):
+        dda.prepare_green(n, n, n, np.ones(n ** 3, dtype=np.int16), (0.3, 0.0, 0.0))
+
+    prepare(16)
+    dda.release()
+    free0 = torch.cuda.mem_get_info()[0]
+    prepare(160)
+    big = free0 - torch.cuda.mem_get_info()[0]
+    prepare(16)
+    idle = free0 - torch.cuda.mem_get_info()[0]
+    assert big > (2 << 30) and idle <= (keep_mib + 64) << 20
+    dda.release()
+    assert torch.cuda.mem_get_info()[0] >= free0 - (4 << 20)
+
+
+@pytest.mark.gpu
 def test_concurrent_targets_do_not_share_blocks():
     probs = [targets.make_problem(n, m=1.4 + 0.03j, x=1.5) for n in (8, 10, 12, 14, 16, 9)]
 
