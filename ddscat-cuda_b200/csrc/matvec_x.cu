@@ -1359,7 +1359,6 @@ template <typename T, int N> static const void* xk(XPass p, int my = 0, bool acc
       if constexpr (Z3Shape<N>::OK && sizeof(T) == 4 && 128 / RegShape<N>::T * RegShape<N>::T == 128)
         return (const void*)kx_zg3r<T, N>;
       return nullptr;
-
     case XPass::YI: return (const void*)kx_yi<T, N>;
     default: return (const void*)kx_xi<T, N>;
   }

@@ -389,7 +389,6 @@ static inline unsigned dq_grid(int n) { return (unsigned)std::min<size_t>(ceil_d
 // points: 4.54 -> 3.23 ms (16 iterations).
 struct DPState {
   double2 alpha, omega, sigma, rho0, rho1, beta;
-  double2 one, mone;
   double2 co[3];           // -beta, alpha, -alpha
   double2 y1, y2, my1, my2;  // Y1, Y2 of the minimal-residual step and their negatives
   double rnrm0, rnrm, mxnrmx, mxnrmr, resid;
@@ -587,7 +586,6 @@ template <typename T> int solve_pbcgs2(SolveIO<T>& io) {
   DPState S{};
   S.alpha = make_double2(0.0, 0.0); S.omega = make_double2(1.0, 0.0); S.sigma = make_double2(1.0, 0.0);
   S.rho0 = make_double2(1.0, 0.0); S.rho1 = make_double2(0.0, 0.0);
-  S.one = make_double2(1.0, 0.0); S.mone = make_double2(-1.0, 0.0);
   S.rnrm0 = rnrm0; S.rnrm = S.mxnrmx = S.mxnrmr = rnrm0;
   S.resid = rnrm0 > 0.0 ? 1.0 : 0.0;
   auto upload = [&]() -> int {
