@@ -1,7 +1,7 @@
 """FFT launch-shape autotuner (ddscat_b200_autotune_f32): on grids that run the
-z-first pipeline (non-power-of-two and mixed axes) it picks launch shapes, on
-grids of the x-first pipeline (24^3: 48-point axes; 32x24x16) it picks between
-the two z passes; the choice is never slower than the default (the default is
+z-first pipeline (here by DDSCAT_B200_ZFIRST=1: generic and mixed axes) it picks
+launch shapes, on grids of the x-first pipeline (24^3: 48-point axes; 15x27x20,
+padded; 32x24x16) it picks between the two z passes; the choice is never slower than the default (the default is
 a candidate) and the MATVEC still matches the FP64 oracle (relative L2 <= 2e-5)."""
 import numpy as np
 import pytest
@@ -11,8 +11,10 @@ from oracle import ddscat_oracle as O
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(24, 24, 24), (15, 27, 20), (32, 24, 16)])
-def test_autotune_keeps_parity(dims):
+@pytest.mark.parametrize("dims,zfirst", [((24, 24, 24), 0), ((15, 27, 20), 0), ((32, 24, 16), 0), ((15, 27, 20), 1),
+                                         ((32, 24, 16), 1), ((16, 32, 64), 1)])
+def test_autotune_keeps_parity(dims, zfirst, monkeypatch):
+    monkeypatch.setenv("DDSCAT_B200_ZFIRST", str(zfirst))
     nx, ny, nz = dims
     rng = np.random.default_rng(8)
     nat = nx * ny * nz

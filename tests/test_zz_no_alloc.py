@@ -28,10 +28,14 @@ def _inputs(dims, seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(16, 16, 16), (12, 10, 9), (18, 18, 18)])
-def test_apply_noalloc_matches_apply(dims):
-    """16^3: x-first pipeline with M = 2n; 12x10x9: z-first pipeline; 18^3: x-first
-    on padded FFT lengths (36 -> 48)."""
+@pytest.mark.parametrize("dims,zfirst", [((16, 16, 16), 0), ((12, 10, 9), 0), ((18, 18, 18), 0), ((12, 10, 9), 1),
+                                         ((16, 32, 8), 1), ((70, 69, 72), 1)])
+def test_apply_noalloc_matches_apply(dims, zfirst, monkeypatch):
+    """16^3: x-first pipeline with M = 2n; 18^3: x-first on padded FFT lengths (36
+    -> 48), 12x10x9 on 32, 32 and 32; the z-first pipeline (generic and power-of-two
+    axes, and near the site limit) by DDSCAT_B200_ZFIRST=1.  There M = 2n, so every
+    target within the limit fits whole."""
+    monkeypatch.setenv("DDSCAT_B200_ZFIRST", str(zfirst))
     torch = pytest.importorskip("torch")
     iocc, ak, x1, x2, adia, aoff = _inputs(dims, 7)
     dda = D.DDA()
