@@ -644,13 +644,14 @@ __global__ void k_row_maps(const int16_t* iocc, int nx, int nrows, const int* ro
 // Largest ratio of padded to 2n grid points at which the register pipeline is
 // the faster one.  The generic passes cost 0.10-0.13 ns per point when 2n has
 // the factors 2, 3, 5 only and 0.27 ns and more with larger ones (their
-// butterflies grow with the factor), the register passes 0.02-0.03 ns.
-// Measured at 8 RHS per call, ms per RHS padded / on 2n: factors 2, 3, 5:
-// 135x135x40 (4.3 times the points) 0.52 / 0.84, 12x10x9 (3.8) 0.0038 / 0.0053,
-// 72^3 (2.4) 0.156 / 0.383; larger ones: 34^3 (2.8) 0.027 / 0.274, 65^3 (3.2)
-// 0.154 / 1.11, 131x131x33 (5.6) 0.50 / 77.  4.5 and 12 keep a margin for
-// single-RHS calls on small grids, where launches decide (5^3, 4.1 times the
-// points: 0.028 / 0.031 ms).
+// butterflies grow with the factor), the register passes 0.02-0.04 ns.
+// Measured, us per RHS padded / on 2n with 1 RHS per call and with 8: factors 2, 3,
+// 5: 5^3 (4.1 times the points) 12 / 32 and 1.6 / 4.3, 10^3 (4.1) 19 / 36 and 3.0 /
+// 5.2, 162x10x162 (4.0) 229 / 287 and 198 / 260, 135x135x40 (1.6) 325 / 888 and 277
+// / 837; larger ones: 2x7x7 (5.2) 12 / 84 and 1.6 / 11, 161x9x161 (4.5) 230 / 1252
+// and 200 / 1083, 34^3 (1.6) 44 / 463 and 17 / 274.  FP64 (axes up to 256 but 160; a
+// residual): 10^3 88 / 104, 5x5x72 (3.4) 93 / 117, 72x72x10 (2.8) 163 / 169, 72^3
+// (2.4) 513 / 625, 100^3 (2.1) 932 / 1229, 65^3 (3.2) 497 / 1771.
 static double pad_limit(const Geometry& g) {
   auto smooth = [](int m) {
     for (int f : {2, 3, 5})

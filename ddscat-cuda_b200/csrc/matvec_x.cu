@@ -16,6 +16,9 @@
 // the x and y passes of a z plane run fused in one cluster of four CTAs (XYF,
 // XYI below): the plane meets in distributed shared memory instead of an HBM
 // round trip of A, and B is laid out [c][kx][iz][ky] for them.
+// Targets that left the generic transforms for these lengths (Engine::cx) run
+// the ACC forms of the passes: every constant applied as hi + lo, the finish in
+// FP64.
 // The Green octant is stored z-fastest, [irx][iry][irz][6], so a z-line reads
 // contiguous 48-byte records.  kx_zg3 (the ZG pass for E <= 16, FP32) keeps
 // the three components of a z position in one thread and reads its records
@@ -1482,7 +1485,7 @@ template <typename T> int matvec_check(Engine<T>& E) {
   if (e != cudaSuccess) { set_cuda_error("MATVEC status", e); return 26; }
   if (h == 0) return 0;
   cudaMemsetAsync(E.d_err, 0, sizeof(int), E.stream);
-  set_error("MATVEC", "a tile copy of the y passes did not complete in the allowed time");
+  set_error("MATVEC", "a tile or row copy of the passes did not complete in the allowed time");
   return 26;
 }
 template int matvec_check<float>(Engine<float>&);

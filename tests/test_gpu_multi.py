@@ -3,8 +3,8 @@ the C4 configuration, 40 seeded random ellipsoids with lattice sides drawn
 uniformly from 24 to 96 per axis, semi-axes filling 0.6-1.0 of the box,
 Re m ~ U[1.2, 1.8], Im m ~ U[0.001, 0.1], x = 0.15 * (largest side), two
 polarisations each (80 RHS), PBCGS2.  Each target is solved on its drawn
-lattice sides (even sides run on padded register-FFT lengths, odd ones on
-the generic z-first pipeline).  Every RHS converges; for three targets the
+lattice sides (an odd side is extended by a vacuum plane; all run on padded
+register-FFT lengths).  Every RHS converges; for three targets the
 FP64 true residual is <= 1.2*TOL, the solutions match the single-target
 batched solve to 20*TOL, and Cext, Cabs (EVALQ) and Csca (SCAT) of the FP32
 solutions are within 1e-4 of those of the all-FP64 batched solve."""
