@@ -280,15 +280,14 @@ __device__ __forceinline__ void line_fft_w(C (&v)[E], C* sl, int t, const C (&w)
 }
 
 // The transform with constants good to 48 bits: twiddles from tab[p*T + t] =
-// (hi.x, hi.y, lo.x, lo.y) of exp(-2*pi*i*t*p/N), DFT constants as hi + lo (CC).
-// Lines within a warp.
-template <int E, int T, int DIR, bool HALF_IN = false, bool PAIR = false, bool SWAP = false>
-__device__ __forceinline__ void line_fft_acc(float2 (&v)[E], float2* sl, int t, const float4* __restrict__ tab,
-                                             int swap = 0) {
+// (hi.x, hi.y, lo.x, lo.y) of exp(-2*pi*i*t*p/N) in shared (SHARED) or global
+// memory, DFT constants as hi + lo (CC).  Lines within a warp.
+template <int E, int T, int DIR, bool SHARED, bool HALF_IN = false, bool PAIR = false, bool SWAP = false>
+__device__ __forceinline__ void line_fft_acc(float2 (&v)[E], float2* sl, int t, const float4* tab, int swap = 0) {
   line_fft_steps<E, T, DIR, false, HALF_IN, PAIR, SWAP, true>(
       v, sl, t,
       [&](float2 a, int p) {
-        const float4 w = __ldg(tab + p * T + t);
+        const float4 w = SHARED ? tab[p * T + t] : __ldg(tab + p * T + t);
         const float s = DIR > 0 ? -1.f : 1.f;
         return cmul_hl(a, make_float2(w.x, s * w.y), make_float2(w.z, s * w.w));
       },

@@ -723,8 +723,8 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   // generic 4.5; 63x61x59 8.9 -> 3.9, 4.5; 97^3 8.9 -> 3.7, 4.2; the transforms
   // alone, CXADIA = 0: 63x61x59 26.7 -> 9.7, 9.7, and at worst, three prime sides,
   // 47^3 19.7 -> 10.1, 8.0).  us per
-  // RHS-MATVEC, 8 RHS, plain / this / generic: 45x37x31 13.9 / 15.9 / 779,
-  // 51x75x39 47.9 / 60.4 / 361, 63x61x59 42.0 / 52.1 / 6397, 75^3 141 / 192 / 431,
+  // RHS-MATVEC, 8 RHS, plain / this / generic: 45x37x31 13.9 / 15.7 / 779,
+  // 51x75x39 47.9 / 54.8 / 361, 63x61x59 42.0 / 50.4 / 6397, 75^3 141 / 177 / 431,
   // periodic 20x24x18 5.0 / 5.5 / 13.4.
   int base[3];
   if (sizeof(T) == 4 && xpipe && !(g.base_lengths(base) &&

@@ -274,17 +274,39 @@ template <int MAXC, typename C> __device__ __forceinline__ void stage_chunk_asyn
   }
 }
 
-// line transform of a pass (ACC: constants good to 48 bits)
-template <int E, int TT, int DIR, bool ACC, bool HALF_IN, bool PAIR, typename C>
+// Where an ACC pass of n points reads its twiddle table: from the start of shared
+// memory, copied there before pdl_wait (the table is constant), or from global
+// memory through L1.  us per RHS-MATVEC shared / global, 1 and 8 RHS: 66^3 (160
+// points) 194 / 220 and 164 / 176, 51x75x39 (128, 160, 80) 69 / 82 and 55 / 60, 63x61x59
+// (128) 64 / 65 and 50.5 / 52.1, 25x27x29 (64) 23.7 / 24.6 and 6.6 / 6.5; but 47^3 (96)
+// 47 / 48 and 29.5 / 28.7, 21^3 (48) 28.4 / 26.4 and 5.6 / 5.5, 165x13x15 (512, 32, 32)
+// 40 / 43 and 22.4 / 21.7.
+constexpr bool acc_staged(int n) { return n != 48 && n != 96 && n != 512; }
+template <bool STAGED, int N> __device__ __forceinline__ void table_stage(unsigned char* dst, const float4* src) {
+  if constexpr (STAGED) {
+    for (int u = threadIdx.x; u < N; u += blockDim.x) cp_async16(reinterpret_cast<float4*>(dst) + u, src + u);
+    cp_async_commit();
+  }
+}
+template <bool STAGED> __device__ __forceinline__ void table_wait() {
+  if constexpr (STAGED) {
+    cp_async_wait_all();
+    __syncthreads();
+  }
+}
+
+// line transform of a pass (ACC: constants good to 48 bits, their table in shared
+// memory with TB)
+template <int E, int TT, int DIR, bool ACC, bool TB, bool HALF_IN, bool PAIR, typename C>
 __device__ __forceinline__ void xline(C (&v)[E], C* sl, int t, const C* tw, const float4* tab) {
-  if constexpr (ACC) line_fft_acc<E, TT, DIR, HALF_IN, PAIR>(v, sl, t, tab);
+  if constexpr (ACC) line_fft_acc<E, TT, DIR, TB, HALF_IN, PAIR>(v, sl, t, tab);
   else line_fft<E, TT, DIR, false, HALF_IN, PAIR>(v, sl, t, tw);
 }
 
 // line transform of a z pass whose thread keeps the twiddles w of DIR = +1
-template <int E, int TT, int DIR, bool ACC, bool HALF_IN, bool PAIR, bool SWAP = false, typename C>
+template <int E, int TT, int DIR, bool ACC, bool TB, bool HALF_IN, bool PAIR, bool SWAP = false, typename C>
 __device__ __forceinline__ void zline(C (&v)[E], C* sl, int t, const C (&w)[E], const float4* tab, int swap = 0) {
-  if constexpr (ACC) line_fft_acc<E, TT, DIR, HALF_IN, PAIR, SWAP>(v, sl, t, tab, swap);
+  if constexpr (ACC) line_fft_acc<E, TT, DIR, TB, HALF_IN, PAIR, SWAP>(v, sl, t, tab, swap);
   else line_fft_w<E, TT, DIR, false, HALF_IN, PAIR, (DIR < 0), SWAP>(v, sl, t, w, swap);
 }
 
@@ -294,15 +316,22 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cx;
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);   // [kx][TS], aliases the line scratch
   C* lines = reinterpret_cast<C*>(smem_raw);  // RL * lsx
   const int iy0 = blockIdx.x * RL, iy = iy0 + l, iz = blockIdx.y;
   const int rl = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
+  table_stage<TB, N>(smem_all, P.cx);
   pdl_launch();
   pdl_wait();
-  if (xoff(P, rl)) return;
+  if (xoff(P, rl)) {
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
   const int S = P.io_full ? P.nat : P.nat0;
   const C* x = P.x + (size_t)rl * P.x_rs + (size_t)c * S;
   const int jrow = P.nx * (iy + P.ny * iz);
@@ -331,7 +360,8 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
 #pragma unroll
     for (int i = 0; i < H; ++i) v[i].y = -v[i].y;
   }
-  xline<E, TT, +1, ACC, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, P.cx);
+  table_wait<TB>();
+  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
   __syncthreads();  // all line scratch consumed before the tile reuses it
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma_x) {
@@ -359,21 +389,29 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cy;
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
   C* lines = reinterpret_cast<C*>(smem_raw);
   const int iz0 = blockIdx.x * RL, iz = iz0 + l, kxl = blockIdx.y, kx = P.kx0 + kxl;
   const int rb = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3), rl = P.b_rhs0 + rb;
+  table_stage<TB, N>(smem_all, P.cy);
   pdl_launch();
   pdl_wait();
-  if (xoff(P, rl)) return;
+  if (xoff(P, rl)) {
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
   const C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * P.nz + iz) * P.Mx + kx) * P.lda;
   C v[E];
   const bool zin = iz < P.nz;
 #pragma unroll
   for (int i = 0; i < H; ++i) v[i] = zin && t + TT * i < P.ny ? A[t + TT * i] : mk<C>(0, 0);  // iy < ny <= N/2
-  xline<E, TT, +1, ACC, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, P.cy);
+  table_wait<TB>();
+  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
   __syncthreads();
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma) {
@@ -493,14 +531,21 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
   // are short or one block per SM waits for its copies (36^3 0.0151 -> 0.0153,
   // 72^3 0.136 -> 0.140), nor at 512 (128-byte loads).
   constexpr bool BULK = sizeof(C) == 8 && BTY == 0 && E == 24;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cz;
   const int t = threadIdx.x % TT, l = (threadIdx.x / TT) % RL, c = threadIdx.x / (TT * RL);
   C* lines = reinterpret_cast<C*>(smem_raw);  // [3][RL][lsz]
   C* my = lines + (size_t)(c * RL + l) * P.lsz;
   const int rb = blockIdx.x, rl = P.b_rhs0 + rb;
+  table_stage<TB, N>(smem_all, P.cz);
   pdl_launch();
   pdl_wait();
-  if (xoff(P, rl)) return;
+  if (xoff(P, rl)) {
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
   const int nlines = P.nkx * P.My;
   const int p = blockIdx.y * RL + l;
   const bool live = p < nlines;
@@ -521,6 +566,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
     if (!__syncthreads_and(mbar_wait(&bar, 0, TMA_WAIT_POLLS))) {
       if (threadIdx.x == 0) atomicOr(P.err, 1);
       mbar_wait(&bar, 0, TMA_WAIT_POLLS);
+      table_wait<TB>();
       return;
     }
 #pragma unroll
@@ -531,7 +577,8 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
     for (int i = 0; i < H; ++i)
       v[i] = live && t + TT * i < P.nz ? row[(t + TT * i) * zs] : mk<C>(0, 0);  // iz < nz <= N/2
   }
-  xline<E, TT, +1, ACC, true, S_::PAIR>(v, my, t, P.twz, P.cz);
+  table_wait<TB>();
+  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, my, t, P.twz, tab);
 #pragma unroll
   for (int i = 0; i < E; ++i) my[t + TT * i] = v[i];
   __syncthreads();
@@ -582,7 +629,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
 #pragma unroll
   for (int i = 0; i < E; ++i) v[i] = my[t + TT * i];
   __syncwarp();
-  xline<E, TT, -1, ACC, false, S_::PAIR>(v, my, t, P.twz, P.cz);
+  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, my, t, P.twz, tab);
   if constexpr (BULK) {
 #pragma unroll
     for (int i = 0; i < H; ++i)
@@ -683,7 +730,7 @@ template <typename T, int N, int BTY = 0, bool ACC = false> __global__ void __la
   C w[E];
   if constexpr (!ACC) line_twiddles<E, +1>(w, t, P.twz);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) zline<E, TT, +1, ACC, true, S_::PAIR>(v[c], my, t, w, P.cz);
+  for (int c = 0; c < 3; ++c) zline<E, TT, +1, ACC, false, true, S_::PAIR>(v[c], my, t, w, P.cz);
   if (live) {
     if (P.ipbc == 0) {
       R sxy, sxz, syz;
@@ -699,7 +746,7 @@ template <typename T, int N, int BTY = 0, bool ACC = false> __global__ void __la
     }
   }
 #pragma unroll
-  for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, false, S_::PAIR>(v[c], my, t, w, P.cz);
+  for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, false, false, S_::PAIR>(v[c], my, t, w, P.cz);
   if (live) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -772,7 +819,10 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RZ = Z3Shape<N>::RZ;
   constexpr int LREC = 6 * (N / 2 + 1);  // complex elements of a line's records
   static_assert(Z3Shape<N>::OK && RZ * TT == 128 && sizeof(C) == 8, "kx_zg3r: FP32, 128-thread blocks");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cz;
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   // line scratch: at 16 elements x 8 threads lines lie T * 18 apart (ZRow::SCRATCH)
   constexpr bool SW = ZRow<N>::SCRATCH != 0;
@@ -809,10 +859,15 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     }
     cp_async_commit();
   };
+  table_stage<TB, N>(smem_all, P.cz);
   pdl_launch();
   pdl_wait();
   int rb = next_rb((int)blockIdx.y * P.zg_rch);
-  if (rb >= rb1) return;  // every RHS of the chunk masked
+  if (rb >= rb1) {  // every RHS of the chunk masked
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
+  table_wait<TB>();
   fetch(rb, 0);
   // the block's octant lines: line ll is the contiguous record run of
   // (irx, iry) = (min(kx, Mx - kx), min(ky, My - ky)), kz = 0..N/2
@@ -847,7 +902,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
       __syncwarp();  // the buffer is read before the next row overwrites it
       if (c < 2) fetch(rb, c + 1);
       else if (nrb < rb1) fetch(nrb, 0);
-      zline<E, TT, +1, ACC, true, S_::PAIR, SW>(v[c], my, t, w, P.cz, fswap);
+      zline<E, TT, +1, ACC, TB, true, S_::PAIR, SW>(v[c], my, t, w, tab, fswap);
     }
     if (!staged) {
       __syncthreads();  // every thread's Green copies have landed (waited for at c = 1)
@@ -855,7 +910,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     }
     if (live) zg3_green_s<N, TT, E>(gs + (size_t)l * LREC, t, v);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, false, S_::PAIR, SW>(v[c], my, t, w, P.cz, fswap);
+    for (int c = 0; c < 3; ++c) zline<E, TT, -1, ACC, TB, false, S_::PAIR, SW>(v[c], my, t, w, tab, fswap);
     if (live) {
       C* row = P.B + (size_t)rb * 3 * cs + (size_t)p * P.ldb;
 #pragma unroll
@@ -876,15 +931,22 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cy;
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
   C* lines = reinterpret_cast<C*>(smem_raw);
   const int iz0 = blockIdx.x * RL, iz = iz0 + l, kxl = blockIdx.y, kx = P.kx0 + kxl;
   const int rb = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3), rl = P.b_rhs0 + rb;
+  table_stage<TB, N>(smem_all, P.cy);
   pdl_launch();
   pdl_wait();
-  if (xoff(P, rl)) return;
+  if (xoff(P, rl)) {
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
   const int nz = P.nz;
   C v[E];
   bool loaded = false;
@@ -903,6 +965,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
         // more (bounded) for the copy in flight, and leave this block's lines
         if (threadIdx.x == 0) atomicOr(P.err, 1);
         mbar_wait(&bar, 0, TMA_WAIT_POLLS);
+        table_wait<TB>();
         return;
       }
 #pragma unroll
@@ -919,7 +982,8 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();  // the tile is consumed before the line scratch reuses it
   }
-  xline<E, TT, -1, ACC, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, P.cy);
+  table_wait<TB>();
+  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
   if (iz < nz) {
     C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * nz + iz) * P.Mx + kx) * P.lda;
 #pragma unroll
@@ -994,7 +1058,10 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
   constexpr int MAXC = RL * (N / 2);
   constexpr bool STAGE = xi_staged(N, TT, sizeof(C));  // the other rows keep direct loads (shared memory)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool TB = ACC && acc_staged(N);  // twiddle table in shared memory
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  unsigned char* const smem_raw = smem_all + (TB ? N * sizeof(float4) : 0);
+  const float4* const tab = TB ? reinterpret_cast<const float4*>(smem_all) : P.cx;
   const int t = threadIdx.x % TT, l = threadIdx.x / TT;
   C* tile = reinterpret_cast<C*>(smem_raw);
   C* lines = reinterpret_cast<C*>(smem_raw);
@@ -1002,9 +1069,13 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
   C* as = xs + MAXC;
   const int iy0 = blockIdx.x * RL, iy = iy0 + l, iz = blockIdx.y;
   const int rl = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
+  table_stage<TB, N>(smem_all, P.cx);
   pdl_launch();
   pdl_wait();
-  if (xoff(P, rl)) return;
+  if (xoff(P, rl)) {
+    table_wait<TB>();  // no copy in flight at exit
+    return;
+  }
   const int ny = P.ny;
   const int S = P.io_full ? P.nat : P.nat0;
   const int SA = P.a_full ? P.nat : P.nat0;
@@ -1052,6 +1123,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
         // more (bounded) for the copy in flight, and leave this block's rows
         if (threadIdx.x == 0) atomicOr(P.err, 1);
         mbar_wait(&bar, 0, TMA_WAIT_POLLS);
+        table_wait<TB>();
         return;
       }
 #pragma unroll
@@ -1069,7 +1141,8 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     for (int i = 0; i < E; ++i) v[i] = tile[(t + TT * i) * TS + l];
     __syncthreads();
   }
-  xline<E, TT, -1, ACC, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, P.cx);
+  table_wait<TB>();
+  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
   // finish (cu:116-118): y = CXADIA x - w/ngrid [+ CXAOFF terms], conj for 'C'
   C* y = P.y + (size_t)rl * P.y_rs + (size_t)c * S;
   const C* ao = P.aoff ? P.aoff + (size_t)rl * P.a_rs : nullptr;
@@ -1554,6 +1627,9 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   const void* fzg3r = fzg3 && g.ipbc == 0 && !env_flag("DDSCAT_B200_NOZG3R") ? xkernel<T>(XPass::ZG3R, g.Mz, 0, E.cz != nullptr) : nullptr;
   const int lszr = g.Mz == 128 ? 8 * 18 : P.lsz;  // ZRow::SCRATCH
   const size_t smzr = ((size_t)RZ3 * lszr) * sizeof(C) + (size_t)RZ3 * (6 * (g.Mz / 2 + 1) + g.Mz / 2 + (TZ == 4 ? 4 : 0)) * sizeof(C);
+  // shared memory of the ACC passes' tables, in front of the rest (kx_zg3 has none)
+  const auto table = [](const float4* t, int n) { return t && acc_staged(n) ? (size_t)n * sizeof(float4) : 0; };
+  const size_t tabx = table(E.cx, g.Mx), taby = table(E.cy, g.My), tabz = table(E.cz, g.Mz);
   const void* fxf = xkernel<T>(XPass::XF, g.Mx, 0, E.cx != nullptr);
   const void* fyf = xkernel<T>(XPass::YF, g.My, 0, E.cy != nullptr);
   const void* fzg = xkernel<T>(XPass::ZG, g.Mz, 0, E.cz != nullptr);
@@ -1611,7 +1687,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
     P.y = a.y + (size_t)r0 * a.y_rs;
     P.adia = a.adia + (size_t)r0 * a.a_rs;
     P.aoff = a.aoff ? a.aoff + (size_t)r0 * a.a_rs : nullptr;
-    if (xlaunch<T>(fxf, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smx, E.stream, P, pdl))
+    if (xlaunch<T>(fxf, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smx + tabx, E.stream, P, pdl))
       return 21;
     for (int rb0 = 0; rb0 < nr; rb0 += E.slab_nr) {
       const int nrb = std::min(E.slab_nr, nr - rb0);
@@ -1620,7 +1696,7 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
       for (int kx0 = 0; kx0 < g.Mx; kx0 += E.slab_B) {
         P.kx0 = kx0;
         P.nkx = std::min(E.slab_B, g.Mx - kx0);
-        if (xlaunch<T>(fyf, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy,
+        if (xlaunch<T>(fyf, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy + taby,
                        E.stream, P, pdl))
           return 22;
         // ZG3R: RHS chunks so that the grid has at least 4 waves of 3 blocks per SM
@@ -1628,19 +1704,19 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
         const int nchunk = (int)std::min<size_t>((size_t)nrb, std::max<size_t>(1, ceil_div(4 * 3 * 148, nlb)));
         P.zg_rch = (int)ceil_div((size_t)nrb, (size_t)nchunk);
         const bool use_r = fzg3r && P.zg_rch >= E.zg3r_min;
-        if (use_r ? xlaunch<T>(fzg3r, dim3((unsigned)nlb, (unsigned)ceil_div((size_t)nrb, (size_t)P.zg_rch)), 128, smzr,
+        if (use_r ? xlaunch<T>(fzg3r, dim3((unsigned)nlb, (unsigned)ceil_div((size_t)nrb, (size_t)P.zg_rch)), 128, smzr + tabz,
                                E.stream, P, pdl)
             : fzg3 ? xlaunch<T>(fzg3, dim3((unsigned)nrb, (unsigned)ceil_div((size_t)P.nkx * g.My, RZ3)), 128, smz,
                               E.stream, P, pdl)
                  : xlaunch<T>(fzg, dim3((unsigned)nrb, (unsigned)ceil_div((size_t)P.nkx * g.My, RZ)), 3 * TZ * RZ,
-                              smz, E.stream, P, pdl))
+                              smz + tabz, E.stream, P, pdl))
           return 23;
-        if (xlaunch<T>(fyi, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy,
+        if (xlaunch<T>(fyi, dim3((unsigned)ceil_div(g.nz, RY), (unsigned)P.nkx, (unsigned)(3 * nrb)), 256, smy + taby,
                        E.stream, P, pdl))
           return 24;
       }
     }
-    if (xlaunch<T>(fxi, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smxi, E.stream, P, pdl))
+    if (xlaunch<T>(fxi, dim3((unsigned)ceil_div(g.ny, RX), (unsigned)g.nz, (unsigned)(3 * nr)), 256, smxi + tabx, E.stream, P, pdl))
       return 25;
   }
   return 0;
