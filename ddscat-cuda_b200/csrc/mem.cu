@@ -30,7 +30,7 @@ namespace {
 // vectors 0.7, MATVEC workspace 0.3.
 size_t g_dev_keep = (size_t)2 << 30;
 constexpr size_t HOST_KEEP = (size_t)64 << 20;
-constexpr size_t SLACK = (size_t)64 << 20;
+constexpr size_t SLACK = (size_t)256 << 20;
 
 struct Block {
   size_t bytes;
