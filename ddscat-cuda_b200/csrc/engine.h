@@ -117,6 +117,7 @@ template <typename T> struct Engine {
   using C = cplx<T>;
   Geometry g;
   FftPlan px, py, pz;
+  unsigned char* tables = nullptr;  // the twiddle tables below
   C *twx = nullptr, *twy = nullptr, *twz = nullptr;
   // twiddles as hi + lo in thread order (line_fft_acc), for targets that left the
   // generic transforms for the register ones (set in init_geometry); else null

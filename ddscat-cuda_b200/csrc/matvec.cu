@@ -563,18 +563,45 @@ static int env_int(const char* name, int dflt) {
   return std::atoi(v);
 }
 
-template <typename T> static cplx<T>* upload_twiddles(int n, size_t& bytes) {
-  std::vector<cplx<T>> h(n);
+// The twiddle tables of the three axes, in one allocation and one copy:
+// twx, twy, twz: exp(-2*pi*i*m/n); with hi_lo also cx, cy, cz (line_fft_acc): the
+// same roots as hi + lo, exp(-2*pi*i*t*p/n) at [p*T + t].
+template <typename T> static bool upload_twiddles(Engine<T>& e, bool hi_lo) {
+  using C = cplx<T>;
+  const int n[3] = {e.g.Mx, e.g.My, e.g.Mz};
+  const size_t sum = (size_t)n[0] + n[1] + n[2], head = hi_lo ? sum * sizeof(float4) : 0;
+  std::vector<unsigned char> h(head + sum * sizeof(C));
+  float4* c = reinterpret_cast<float4*>(h.data());
+  C* w = reinterpret_cast<C*>(h.data() + head);
   const double pi = 3.14159265358979323846;
-  for (int m = 0; m < n; ++m) {
-    const double a = -2.0 * pi * (double)m / (double)n;
-    h[m] = mk<cplx<T>>(std::cos(a), std::sin(a));
+  for (int k = 0; k < 3; ++k) {
+    std::vector<double2> r(n[k]);
+    for (int m = 0; m < n[k]; ++m) {
+      const double a = -2.0 * pi * (double)m / (double)n[k];
+      r[m] = make_double2(std::cos(a), std::sin(a));
+      *w++ = mk<C>(r[m].x, r[m].y);
+    }
+    if (!hi_lo) continue;
+    const int T_ = reg_threads(n[k]);
+    for (int p = 0; p < n[k] / T_; ++p)
+      for (int t = 0; t < T_; ++t) {
+        const double2 v = r[t * p];  // t p < n
+        const float x = (float)v.x, y = (float)v.y;
+        *c++ = make_float4(x, y, (float)(v.x - (double)x), (float)(v.y - (double)y));
+      }
   }
-  cplx<T>* d = nullptr;
-  if (dev_alloc((void**)&d, n * sizeof(cplx<T>)) != cudaSuccess) return nullptr;
-  cudaMemcpy(d, h.data(), n * sizeof(cplx<T>), cudaMemcpyHostToDevice);
-  bytes += n * sizeof(cplx<T>);
-  return d;
+  if (dev_alloc((void**)&e.tables, h.size()) != cudaSuccess) return false;
+  if (cudaMemcpy(e.tables, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+  e.bytes_allocated += h.size();
+  e.twx = reinterpret_cast<C*>(e.tables + head);
+  e.twy = e.twx + n[0];
+  e.twz = e.twy + n[1];
+  if (hi_lo) {
+    e.cx = reinterpret_cast<float4*>(e.tables);
+    e.cy = e.cx + n[0];
+    e.cz = e.cy + n[1];
+  }
+  return true;
 }
 
 // ---------------------------------------------------------------- index maps
@@ -647,9 +674,9 @@ __global__ void k_row_maps(const int16_t* iocc, int nx, int nrows, const int* ro
 // butterflies grow with the factor), the register passes 0.02-0.04 ns.
 // Measured, us per RHS padded / on 2n with 1 RHS per call and with 8: factors 2, 3,
 // 5: 5^3 (4.1 times the points) 12 / 32 and 1.6 / 4.3, 10^3 (4.1) 19 / 36 and 3.0 /
-// 5.2, 162x10x162 (4.0) 229 / 287 and 198 / 260, 135x135x40 (1.6) 325 / 888 and 277
+// 5.2, 162x10x162 (4.0) 228 / 287 and 200 / 260, 135x135x40 (1.6) 312 / 889 and 268
 // / 837; larger ones: 2x7x7 (5.2) 12 / 84 and 1.6 / 11, 161x9x161 (4.5) 230 / 1252
-// and 200 / 1083, 34^3 (1.6) 44 / 463 and 17 / 274.  FP64 (axes up to 256 but 160; a
+// and 202 / 1083, 34^3 (1.6) 40 / 463 and 17 / 274.  FP64 (axes up to 256 but 160; a
 // residual): 10^3 88 / 104, 5x5x72 (3.4) 93 / 117, 72x72x10 (2.8) 163 / 169, 72^3
 // (2.4) 513 / 625, 100^3 (2.1) 932 / 1229, 65^3 (3.2) 497 / 1771.
 static double pad_limit(const Geometry& g) {
@@ -659,24 +686,6 @@ static double pad_limit(const Geometry& g) {
     return m == 1;
   };
   return smooth(g.Mx) && smooth(g.My) && smooth(g.Mz) ? 4.5 : 12.0;
-}
-
-// Twiddles of line_fft_acc: exp(-2*pi*i*t*p/n) as hi + lo at [p*T + t].
-static float4* upload_hl_twiddles(int n, size_t& bytes) {
-  const int T = reg_threads(n);
-  std::vector<float4> h(n);
-  const double pi = 3.14159265358979323846;
-  for (int p = 0; p < n / T; ++p)
-    for (int t = 0; t < T; ++t) {
-      const double a = -2.0 * pi * t * p / n, c = std::cos(a), s = std::sin(a);
-      const float ch = (float)c, sh = (float)s;
-      h[p * T + t] = make_float4(ch, sh, (float)(c - (double)ch), (float)(s - (double)sh));
-    }
-  float4* d = nullptr;
-  if (dev_alloc((void**)&d, n * sizeof(float4)) != cudaSuccess) return nullptr;
-  cudaMemcpy(d, h.data(), n * sizeof(float4), cudaMemcpyHostToDevice);
-  bytes += n * sizeof(float4);
-  return d;
 }
 
 template <typename T>
@@ -710,10 +719,6 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
     set_error("prepare", "FFT length has too many prime factors");
     return 1;
   }
-  twx = upload_twiddles<T>(g.Mx, bytes_allocated);
-  twy = upload_twiddles<T>(g.My, bytes_allocated);
-  twz = upload_twiddles<T>(g.Mz, bytes_allocated);
-  if (!twx || !twy || !twz) { set_error("prepare", "twiddle allocation failed"); return 1; }
   // The generic transforms that odd, periodic and widely padded targets would run
   // on their 2n grid sum prime-length DFTs in FP64 and read each twiddle rounded
   // once.  The plain register transforms multiply theirs up, and their constants
@@ -722,17 +727,14 @@ int Engine<T>::init_geometry(int nx, int ny, int nz, int ipbc, int nat, int nat0
   // lo and the finish in FP64 these targets are at 2.9-4.3e-8 (25x27x29 7.6 -> 3.4,
   // generic 4.5; 63x61x59 8.9 -> 3.9, 4.5; 97^3 8.9 -> 3.7, 4.2; the transforms
   // alone, CXADIA = 0: 63x61x59 26.7 -> 9.7, 9.7, and at worst, three prime sides,
-  // 47^3 19.7 -> 10.1, 8.0).  us per
-  // RHS-MATVEC, 8 RHS, plain / this / generic: 45x37x31 13.9 / 15.7 / 779,
-  // 51x75x39 47.9 / 54.8 / 361, 63x61x59 42.0 / 50.4 / 6397, 75^3 141 / 177 / 431,
-  // periodic 20x24x18 5.0 / 5.5 / 13.4.
+  // 47^3 19.7 -> 10.1, 8.0).  us per RHS-MATVEC, 8 RHS, plain / this / generic:
+  // 45x37x31 13.9 / 15.7 / 779, 51x75x39 47.9 / 54.8 / 361, 63x61x59 42.0 / 50.4 /
+  // 6397, 75^3 141 / 177 / 431, periodic 20x24x18 5.0 / 5.5 / 13.4.
   int base[3];
-  if (sizeof(T) == 4 && xpipe && !(g.base_lengths(base) &&
-                                   (pad || (base[0] == g.Mx && base[1] == g.My && base[2] == g.Mz)))) {
-    cx = upload_hl_twiddles(g.Mx, bytes_allocated);
-    cy = upload_hl_twiddles(g.My, bytes_allocated);
-    cz = upload_hl_twiddles(g.Mz, bytes_allocated);
-    if (!cx || !cy || !cz) { set_error("prepare", "twiddle allocation failed"); return 1; }
+  const bool plain = g.base_lengths(base) && (pad || (base[0] == g.Mx && base[1] == g.My && base[2] == g.Mz));
+  if (!upload_twiddles<T>(*this, sizeof(T) == 4 && xpipe && !plain)) {
+    set_error("prepare", "twiddle allocation failed");
+    return 1;
   }
   // index maps, built on the device from IOCC
   const int nrows = nat / nx;
@@ -956,7 +958,7 @@ template <typename T> int Engine<T>::upload_green(const void* host_green) {
 
 template <typename T> void Engine<T>::release() {
   cudaFree(d_err);  // waits for the device: nothing uses the engine's blocks any more
-  dev_free(twx); dev_free(twy); dev_free(twz); dev_free(cx); dev_free(cy); dev_free(cz);
+  dev_free(tables);
   dev_free(green); dev_free(occ); dev_free(inv); dev_free(iocc); dev_free(rowq);
   dev_free(zhat); dev_free(slab);
   *this = Engine<T>{};

@@ -82,8 +82,8 @@ int multi_solve(int nt, const int* dims, const int16_t* const* iocc, const float
     // The engine's grid: each odd side extended by one vacuum plane (every
     // length that holds 2n holds 2n + 2 as well), because targets of even sides
     // run on the plain line transforms and odd ones on the slower ones with hi +
-    // lo constants (Engine::cx): 8 targets of sides 29 to 47 32.0 against 34.1 ms,
-    // 7 to 21 10.6 against 10.9, 4 of 57 to 65 80 against 85.  The occupied sites,
+    // lo constants (Engine::cx): 8 targets of sides 29 to 47 31.2 against 32.5 ms,
+    // 7 to 21 10.1 against 10.9, 4 of 57 to 65 75 against 78.  The occupied sites,
     // their order (z, then y, then x) and so the compact vectors are those of the
     // caller's grid; the Green tensor depends on the lags only, so the operator
     // on them is unchanged.
