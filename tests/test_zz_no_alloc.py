@@ -63,7 +63,7 @@ def test_apply_noalloc_matches_apply(dims, zfirst, monkeypatch):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(16, 16, 16), (18, 18, 18)])
+@pytest.mark.parametrize("dims", [(16, 16, 16), (18, 18, 18), (17, 13, 33)])
 def test_apply_noalloc_in_cuda_graph(dims):
     """The call captured into a CUDA graph on a caller's stream: every replay
     reads the current contents of x and writes y, equal to ddscat_cuda_apply_f32
