@@ -67,26 +67,23 @@ def test_graph_on_a_caller_supplied_odd_grid(solver, maxit):
 @pytest.mark.gpu
 @pytest.mark.parametrize("solver", ["pbcgs2", "qmrccg"])
 def test_short_solves_pay_for_no_graph(solver):
-    """The 2nd and 3rd iteration take no longer than the 7th and 8th (recording a
-    graph in one of them costs three to six iterations on a 16^3 grid)."""
+    """The 2nd and 3rd iteration take at most 150 us more than the 7th and 8th:
+    recording a graph in one of them costs 350.  The fastest of calls taken in
+    turn, so that a change of the host's clock meets all of them."""
     prob = targets.make_problem(16, 16, 16, m=2.5 + 0.02j, x=3.0)
     b, adia, aoff = prob.rhs(0), prob.adia(0), prob.aoff()
     dda = D.DDA()
     dda.prepare_green(16, 16, 16, prob.iocc, prob.incid[0].k)
-
-    def seconds(maxit):
-        ts = []
-        for _ in range(60):
-            t = time.perf_counter()
-            o = dda.solve(solver, b, adia, aoff, maxit=maxit, tol=1e-7, check=False)
-            ts.append(time.perf_counter() - t)
-            assert o.itno == maxit
-        return float(np.median(ts))
-
+    best = {1: 1.0, 3: 1.0, 6: 1.0, 8: 1.0}
     try:
         dda.lib.ddscat_b200_set_verbose(0)
-        seconds(8)
-        assert seconds(3) - seconds(1) <= 1.6 * (seconds(8) - seconds(6))
+        for _ in range(100):
+            for maxit in best:
+                t = time.perf_counter()
+                o = dda.solve(solver, b, adia, aoff, maxit=maxit, tol=1e-7, check=False)
+                best[maxit] = min(best[maxit], time.perf_counter() - t)
+                assert o.itno == maxit
+        assert best[3] - best[1] <= best[8] - best[6] + 150e-6
     finally:
         dda.lib.ddscat_b200_set_verbose(-1)
     dda.release()
