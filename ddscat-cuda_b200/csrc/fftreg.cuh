@@ -198,12 +198,15 @@ inline int line_stride(int E, int T, int L, bool line_fastest, bool pair = false
 
 // Four-step twiddles W^(t p), p = 1..E-1, of thread t for DIR: the powers of
 // two come from the table tw[m] = exp(-2*pi*i*m/N), the others are products
-// of at most four of them (fewer shared-memory loads).  E = 20 (80 points) loads
-// 1..4, 5, 10 and 15 and multiplies once: with the powers of two 36^3 was 7.9e-8
-// against 64 bits, more than on 96 points (6.7e-8).  w[0] is not set.
-template <int E, int DIR, typename C>
+// of at most four of them (fewer shared-memory loads).  w[0] is not set.
+// BY5 (E = 20): 1..4, 5, 10 and 15 from the table and one product, for grids of 80
+// points on all axes.  There the rounding errors of the products act in the same
+// direction in all passes, 7.9e-8 against 64 bits at 36^3 (6.7e-8 on 96 points),
+// and 5.5e-8 this way; next to other lengths they partly cancel, and the powers of
+// two are better (50x40x44 5.2 against 5.4e-8, 7.4e-8 on 96 points).
+template <int E, int DIR, bool BY5 = false, typename C>
 __device__ __forceinline__ void line_twiddles(C (&w)[E], int t, const C* __restrict__ tw) {
-  if constexpr (E == 20) {
+  if constexpr (BY5) {
 #pragma unroll
     for (int p = 1; p < E; ++p)
       if (p < 5 || p % 5 == 0) w[p] = twid<DIR>(tw, t * p);
@@ -295,10 +298,11 @@ __device__ __forceinline__ void line_fft_acc(float2 (&v)[E], float2* sl, int t, 
 }
 
 // One length-E*T transform with its own twiddles (`tw` as in line_twiddles).
-template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN = false, bool PAIR = false, typename C>
+template <int E, int T, int DIR, bool BLOCK_SYNC, bool HALF_IN = false, bool PAIR = false, bool BY5 = false,
+          typename C>
 __device__ __forceinline__ void line_fft(C (&v)[E], C* sl, int t, const C* __restrict__ tw) {
   C w[E];
-  line_twiddles<E, DIR>(w, t, tw);
+  line_twiddles<E, DIR, BY5>(w, t, tw);
   line_fft_w<E, T, DIR, BLOCK_SYNC, HALF_IN, PAIR>(v, sl, t, w);
 }
 

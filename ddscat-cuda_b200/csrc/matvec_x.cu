@@ -296,11 +296,11 @@ template <bool STAGED> __device__ __forceinline__ void table_wait() {
 }
 
 // line transform of a pass (ACC: constants good to 48 bits, their table in shared
-// memory with TB)
-template <int E, int TT, int DIR, bool ACC, bool TB, bool HALF_IN, bool PAIR, typename C>
+// memory with TB; BY5: line_twiddles)
+template <int E, int TT, int DIR, bool ACC, bool TB, bool BY5, bool HALF_IN, bool PAIR, typename C>
 __device__ __forceinline__ void xline(C (&v)[E], C* sl, int t, const C* tw, const float4* tab) {
   if constexpr (ACC) line_fft_acc<E, TT, DIR, TB, HALF_IN, PAIR>(v, sl, t, tab);
-  else line_fft<E, TT, DIR, false, HALF_IN, PAIR>(v, sl, t, tw);
+  else line_fft<E, TT, DIR, false, HALF_IN, PAIR, BY5>(v, sl, t, tw);
 }
 
 // line transform of a z pass whose thread keeps the twiddles w of DIR = +1
@@ -312,7 +312,8 @@ __device__ __forceinline__ void zline(C (&v)[E], C* sl, int t, const C (&w)[E], 
 
 // ------------------------------------------------------------- XF: x forward
 // block: RL rows (iy) x TT threads, thread-fastest; grid (ceil(ny/RL), nz, 3*nr)
-template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_xf(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false, bool BY5 = false>
+__global__ void __launch_bounds__(256) kx_xf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -361,7 +362,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     for (int i = 0; i < H; ++i) v[i].y = -v[i].y;
   }
   table_wait<TB>();
-  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
+  xline<E, TT, +1, ACC, TB, BY5, true, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
   __syncthreads();  // all line scratch consumed before the tile reuses it
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma_x) {
@@ -385,7 +386,8 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
 
 // ------------------------------------------------------------- YF: y forward
 // block: RL z-lines (iz) x TT; grid (ceil(nz/RL), nkx, 3*nrb)
-template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_yf(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false, bool BY5 = false>
+__global__ void __launch_bounds__(256) kx_yf(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -411,7 +413,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
 #pragma unroll
   for (int i = 0; i < H; ++i) v[i] = zin && t + TT * i < P.ny ? A[t + TT * i] : mk<C>(0, 0);  // iy < ny <= N/2
   table_wait<TB>();
-  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
+  xline<E, TT, +1, ACC, TB, BY5, true, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
   __syncthreads();
   if constexpr (tma_length(N, sizeof(C))) {
     if (P.tma) {
@@ -517,7 +519,7 @@ template <int BTY> constexpr int zline_stride() { return BTY > 0 ? BTY : 1; }
 // ------------------------------------------------------------- ZG: z * Green * z^-1
 // block: RZ lines x TT threads x 3 components, thread-fastest within a line;
 // lines are (kx, ky) pairs p = kxl*My + ky.  grid (nrb, ceil(nkx*My/RZ))
-template <typename T, int N, int BTY = 0, bool ACC = false>
+template <typename T, int N, int BTY = 0, bool ACC = false, bool BY5 = false>
 __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) == 8 ? 1 : XShape<N>::ZG_MINB)
     kx_zg(XParams<T> P) {
   using C = cplx<T>;
@@ -578,7 +580,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
       v[i] = live && t + TT * i < P.nz ? row[(t + TT * i) * zs] : mk<C>(0, 0);  // iz < nz <= N/2
   }
   table_wait<TB>();
-  xline<E, TT, +1, ACC, TB, true, S_::PAIR>(v, my, t, P.twz, tab);
+  xline<E, TT, +1, ACC, TB, BY5, true, S_::PAIR>(v, my, t, P.twz, tab);
 #pragma unroll
   for (int i = 0; i < E; ++i) my[t + TT * i] = v[i];
   __syncthreads();
@@ -629,7 +631,7 @@ __global__ void __launch_bounds__(3 * XShape<N>::TT * XShape<N>::RZ, sizeof(T) =
 #pragma unroll
   for (int i = 0; i < E; ++i) v[i] = my[t + TT * i];
   __syncwarp();
-  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, my, t, P.twz, tab);
+  xline<E, TT, -1, ACC, TB, BY5, false, S_::PAIR>(v, my, t, P.twz, tab);
   if constexpr (BULK) {
 #pragma unroll
     for (int i = 0; i < H; ++i)
@@ -927,7 +929,8 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
 
 // ------------------------------------------------------------- YI: y inverse
 // block: RL z-lines x TT; grid (ceil(nz/RL), nkx, 3*nrb)
-template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_yi(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false, bool BY5 = false>
+__global__ void __launch_bounds__(256) kx_yi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -983,7 +986,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     __syncthreads();  // the tile is consumed before the line scratch reuses it
   }
   table_wait<TB>();
-  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
+  xline<E, TT, -1, ACC, TB, BY5, false, S_::PAIR>(v, lines + (size_t)l * P.lsy, t, P.twy, tab);
   if (iz < nz) {
     C* A = P.A + (size_t)rl * P.A_rs + ((size_t)(c * nz + iz) * P.Mx + kx) * P.lda;
 #pragma unroll
@@ -1052,7 +1055,8 @@ constexpr bool xi_staged(int n, int TT, size_t elem) {
 
 // block: RL rows (iy) x TT; grid (ceil(ny/RL), nz, 3*nr)
 // shared memory: tile / line scratch [tlx] | x chunk | CXADIA chunk
-template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__(256) kx_xi(const __grid_constant__ XParams<T> P) {
+template <typename T, int N, bool ACC = false, bool BY5 = false>
+__global__ void __launch_bounds__(256) kx_xi(const __grid_constant__ XParams<T> P) {
   using C = cplx<T>;
   using S_ = XShape<N>;
   constexpr int E = S_::E, TT = S_::TT, H = S_::H, RL = S_::RL, TS = tile_stride(RL, TT, sizeof(C));
@@ -1142,7 +1146,7 @@ template <typename T, int N, bool ACC = false> __global__ void __launch_bounds__
     __syncthreads();
   }
   table_wait<TB>();
-  xline<E, TT, -1, ACC, TB, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
+  xline<E, TT, -1, ACC, TB, BY5, false, S_::PAIR>(v, lines + (size_t)l * P.lsx, t, P.twx, tab);
   // finish (cu:116-118): y = CXADIA x - w/ngrid [+ CXAOFF terms], conj for 'C'
   C* y = P.y + (size_t)rl * P.y_rs + (size_t)c * S;
   const C* ao = P.aoff ? P.aoff + (size_t)rl * P.a_rs : nullptr;
@@ -1400,7 +1404,16 @@ template <typename T, int N, int BTY> static const void* xkt(XPass p) {
   return nullptr;
 }
 
-template <typename T, int N> static const void* xk(XPass p, int my = 0, bool acc = false) {
+template <typename T, int N> static const void* xk(XPass p, int my = 0, bool acc = false, bool by5 = false) {
+  if constexpr (N == 80)
+    if (by5 && !acc) switch (p) {
+      case XPass::XF: return (const void*)kx_xf<T, N, false, true>;
+      case XPass::YF: return (const void*)kx_yf<T, N, false, true>;
+      case XPass::ZG: return (const void*)kx_zg<T, N, 0, false, true>;
+      case XPass::YI: return (const void*)kx_yi<T, N, false, true>;
+      case XPass::XI: return (const void*)kx_xi<T, N, false, true>;
+      default: return nullptr;
+    }
   if constexpr (sizeof(T) == 4)
     if (acc) switch (p) {
       case XPass::XF: return (const void*)kx_xf<T, N, true>;
@@ -1441,13 +1454,13 @@ template <typename T, int N> static const void* xk(XPass p, int my = 0, bool acc
 }
 
 // my: M_y, for the z passes on the fused layout (ZGT, ZG3T)
-template <typename T> static const void* xkernel(XPass p, int n, int my = 0, bool acc = false) {
+template <typename T> static const void* xkernel(XPass p, int n, int my = 0, bool acc = false, bool by5 = false) {
   switch (n) {
     case 16: return xk<T, 16>(p, my, acc);
     case 32: return xk<T, 32>(p, my, acc);
     case 48: return xk<T, 48>(p, my, acc);
     case 64: return xk<T, 64>(p, my, acc);
-    case 80: return xk<T, 80>(p, my, acc);
+    case 80: return xk<T, 80>(p, my, acc, by5);
     case 96: return xk<T, 96>(p, my, acc);
     case 128: return xk<T, 128>(p, my, acc);
     case 192: return xk<T, 192>(p, my, acc);
@@ -1630,11 +1643,12 @@ int matvec_xpipe(Engine<T>& E, const MvArgs<T>& a) {
   // shared memory of the ACC passes' tables, in front of the rest (kx_zg3 has none)
   const auto table = [](const float4* t, int n) { return t && acc_staged(n) ? (size_t)n * sizeof(float4) : 0; };
   const size_t tabx = table(E.cx, g.Mx), taby = table(E.cy, g.My), tabz = table(E.cz, g.Mz);
-  const void* fxf = xkernel<T>(XPass::XF, g.Mx, 0, E.cx != nullptr);
-  const void* fyf = xkernel<T>(XPass::YF, g.My, 0, E.cy != nullptr);
-  const void* fzg = xkernel<T>(XPass::ZG, g.Mz, 0, E.cz != nullptr);
-  const void* fyi = xkernel<T>(XPass::YI, g.My, 0, E.cy != nullptr);
-  const void* fxi = xkernel<T>(XPass::XI, g.Mx, 0, E.cx != nullptr);
+  const bool by5 = g.Mx == 80 && g.My == 80 && g.Mz == 80;  // line_twiddles
+  const void* fxf = xkernel<T>(XPass::XF, g.Mx, 0, E.cx != nullptr, by5);
+  const void* fyf = xkernel<T>(XPass::YF, g.My, 0, E.cy != nullptr, by5);
+  const void* fzg = xkernel<T>(XPass::ZG, g.Mz, 0, E.cz != nullptr, by5);
+  const void* fyi = xkernel<T>(XPass::YI, g.My, 0, E.cy != nullptr, by5);
+  const void* fxi = xkernel<T>(XPass::XI, g.Mx, 0, E.cx != nullptr, by5);
   // DDSCAT_B200_FUSEXY=1, FP32 with all kx planes of a slab batch resident
   // (FFT3D): the x and y passes fused per z plane (kxy_f / kxy_i), three
   // launches per slab batch.  Opt-in: at 128^3 it moves 41 % fewer DRAM bytes
